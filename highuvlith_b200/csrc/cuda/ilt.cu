@@ -705,6 +705,7 @@ cudaError_t socs_cols_split(const float2* T, int K, int hb, int L, int clips, fl
                             const float* mean, void* split, const float2* tw, cudaStream_t st);
 
 bool xt_ok(int L, int hb);
+bool interp_fused_ok(int M, int n);
 
 cudaError_t ilt_set_smem() {
   const int big = 200 * 1024;
@@ -803,7 +804,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   // N-point row and column syntheses
   const bool xt_fwd = M <= 1024 && xt_ok(M, hb) && ilt_adj_xt_smem(M, hb) <= static_cast<size_t>(kXtSmemMax);
   const bool sep = coarse && xt_fwd && separable_ok(ds, M);
-  const size_t s_bi = sep ? a256(sizeof(uint16_t) * 2 * static_cast<size_t>(n) * M) : 0;
+  const size_t s_bi = sep && !interp_fused_ok(M, n) ? a256(sizeof(uint16_t) * 2 * static_cast<size_t>(n) * M) : 0;
   const size_t s_img = a256(sizeof(float) * npix);         // image on N, then G
   const size_t s_V = grad ? a256(sizeof(float2) * static_cast<size_t>(K) * B * M) : 0;
   const size_t s_q = grad ? a256(sizeof(float2) * B * B) : 0;

@@ -817,6 +817,9 @@ cudaError_t socs_field_fused(const float2* kband, const float2* Mband, int K, in
                              float flare, const float* mean, float* out, void* split, float* part, const float2* tw,
                              cudaStream_t st);
 unsigned long long probe_wait_ns() { return g_probe_wait_ns.load(std::memory_order_relaxed); }
+bool interp_fused_ok(int M, int n);
+cudaError_t interp_fused(const CUtensorMap& map_p, const void* im_split, int M, int n, int nc, const float* mean,
+                         float* out, int* err, cudaStream_t st);
 bool xt_ok(int L, int hb);
 cudaError_t socs_rows_x(const float2* kband, float scale, const float2* Mband, int K, int hb, int L, int clips,
                         float2* T, const float2* tw, cudaStream_t st);
@@ -964,6 +967,13 @@ void launch_rows(const float2* kband, float scale, const float2* Mband, int K, i
 bool tc_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows) {
   return make_map(map, ptr, rows, kp, box_rows);
 }
+
+// FP16 map of 32-wide boxes (64B swizzle) and the f32 output map (32 x 32
+// boxes, 128B swizzle) for other files' kernels.
+bool tc_map_sw64_f16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows, int cols) {
+  return make_map_sw64(map, ptr, rows, kp, box_rows, cols, true);
+}
+bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) { return make_out_map(map, ptr, rows, cols); }
 
 cudaError_t tc_set_smem() {
   const int bytes = static_cast<int>(tc_smem_bytes(3));
@@ -1125,7 +1135,8 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
   const size_t per_i = align256(sizeof(float) * M * M);
   const size_t per_x2 = sep ? 0 : align256(sizeof(float2) * M * B2);  // band of I_M (band-transform path)
   const size_t per_c = sep ? 0 : align256(sizeof(float2) * B2 * B2);
-  const size_t per_bi = align256(static_cast<size_t>(2) * n * std::max(kbI, M) * 2);
+  // Z^T of the two-kernel separable interpolation, or the Hermitian half band
+  const size_t per_bi = sep && interp_fused_ok(M, n) ? 0 : align256(static_cast<size_t>(2) * n * std::max(kbI, M) * 2);
   const size_t per_mean = align256(sizeof(float) * (1 + (B + 3) / 4));
   const size_t per_clip = per_x + per_m + per_be + per_p + per_i + per_x2 + per_c + per_bi + per_mean;
   // a C2 step (256 clips) runs as one chunk of the engine's own workspace, so
@@ -1164,8 +1175,8 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
                  "band_forward");
     prof.end(st);
     CUtensorMap mbE, mbI, mbP;
-    if (!make_map(&mbE, BE, static_cast<uint64_t>(nc) * K * 2 * M, kbE, kTcBN, kcE) ||
-        !make_map(&mbI, BI, static_cast<uint64_t>(nc) * 2 * n, kbI, kTcBN, kcI) ||
+    if ((!fft_field && !make_map(&mbE, BE, static_cast<uint64_t>(nc) * K * 2 * M, kbE, kTcBN, kcE)) ||
+        (!sep && !make_map(&mbI, BI, static_cast<uint64_t>(nc) * 2 * n, kbI, kTcBN, kcI)) ||
         (gemm_rows && !make_map(&mbP, P, static_cast<uint64_t>(nc) * K * 2 * rbn, kpE, rbn)))
       throw Error(HUV_ERR_CUDA, "cuTensorMapEncodeTiled failed for the band operands");
     if (fft_field) {
@@ -1307,9 +1318,9 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
       prof.end(st);
       check_cuda(cudaGetLastError(), "tc_dft_gemm<1>");
     }
-    // mask band (rows, columns, mean), 2 field launches (3 with the row GEMM), 2 (separable) or 4 interpolation launches
+    // mask band (rows, columns, mean), 2 field launches (3 with the row GEMM), 1 or 2 (separable) or 4 interpolation launches
     // (the fused field pass is one launch, two when kernel groups are reduced)
-    prof.launches += (sep ? 7 : (gemm_rows ? 10 : 9)) - (fused && field_fused_part_bytes(M, K) == 0 ? 1 : 0);
+    prof.launches += (sep ? (interp_fused_ok(M, n) ? 6 : 7) : (gemm_rows ? 10 : 9)) - (fused && field_fused_part_bytes(M, K) == 0 ? 1 : 0);
   }
 }
 
@@ -1352,6 +1363,12 @@ void Engine::interp_separable(DeviceSet& ds, int M, int nc, const void* im_split
   once_per_device(smem_set, [] { check_cuda(tc_set_smem(), "cudaFuncSetAttribute(tc)"); });
   interp_matrix(ds, M);
   TcState& tc = ds.tc[M];
+  if (interp_fused_ok(M, n)) {
+    if (profile) prof.begin("tc_interp_fused", st);
+    check_cuda(interp_fused(tc.map_pi32, im_split, M, n, nc, mean, o, dev_err, st), "tc_interp_fused");
+    if (profile) prof.end(st);
+    return;
+  }
   const void* IM = im_split;
   __nv_bfloat16* BI = static_cast<__nv_bfloat16*>(BIv);
   struct Region {  // the profiler's regions only when the caller is not inside one of its own
