@@ -1,6 +1,6 @@
 // Register-radix Stockham FFT over S interleaved sequences (FP32 complex).
 //
-// Each pass of radix R (16, 12, 10, 8, 4) loads R points of one butterfly
+// Each pass of radix R (16, 12, 10, 8, 6 .. 2) loads R points of one butterfly
 // into registers, applies the Stockham twiddles w^{r k}, does the R-point DFT
 // in registers (16 = 4 x 4, 8 = 4 x 2, 12 = 3 x 4, 10 = 5 x 2 with their
 // internal twiddles as constants) and stores R points; a length L of
@@ -138,8 +138,28 @@ __host__ __device__ __forceinline__ void fr_dft(float2 (&v)[R]) {
     const float2 a = v[0];
     v[0] = fr_add(a, v[1]);
     v[1] = fr_sub(a, v[1]);
+  } else if constexpr (R == 3) {
+    fr_dft3<DIR>(v);
   } else if constexpr (R == 4) {
     fr_dft4<DIR>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 5) {
+    fr_dft5<DIR>(v);
+  } else if constexpr (R == 6) {
+    // n = q + 2 m, k = p + 3 q': X = sum_q W2^{q q'} W6^{q p} [sum_m v W3^{m p}]
+    float2 u[2][3];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) u[q][m] = v[q + 2 * m];
+      fr_dft3<DIR>(u[q]);
+    }
+#pragma unroll
+    for (int p = 1; p < 3; ++p) u[1][p] = fr_mul(u[1][p], fr_w<12, DIR>(2 * p));
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      v[p] = fr_add(u[0][p], u[1][p]);
+      v[p + 3] = fr_sub(u[0][p], u[1][p]);
+    }
   } else if constexpr (R == 8) {
     // n = q + 2 m, k = p + 4 q': X = sum_q W2^{q q'} W8^{q p} [sum_m v W4^{m p}]
     float2 u[2][4];

@@ -319,6 +319,30 @@ void Engine::prebuild_planes(const double* z, int planes) {
   }
 }
 
+// A sweep of a narrow band in one field launch and one interpolation: the
+// mask band is the same on every plane.  Only when the engine holds every
+// plane and they share the band (true of every plane of one source and pupil).
+bool Engine::sweep_small(const huv_batch& b, const double* z, int planes, float* out, cudaStream_t st) {
+  if (planes < 2 || (b.form != HUV_FORM_AUTO && b.form != HUV_FORM_HYBRID)) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  check_batch(b, out);
+  for (int p = 0; p < planes; ++p)
+    if (!held_set(z[p])) return false;
+  ensure_device();
+  std::vector<DeviceSet*> sets(planes);
+  int M = 0;
+  for (int p = 0; p < planes; ++p) {
+    sets[p] = &device_set(z[p]);
+    choose_eval_grid(*sets[p], b.eval_grid, true);  // refuses what a single call refuses
+    const int m = small_grid(*sets[p], b.eval_grid);
+    if (!m || (p > 0 && (m != M || sets[p]->hb != sets[0]->hb))) return false;
+    M = m;
+  }
+  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b);
+  run_small_form(b, sets.data(), nullptr, nullptr, planes, M, out, st);
+  return true;
+}
+
 void Engine::image_focus_sweep(const huv_batch& b, const double* z, int planes, float* out, cudaStream_t st) {
   if (planes < 0) throw Error(HUV_ERR_INVALID_PARAMETER, "n_planes: must be >= 0");
   if (planes == 0 || b.n_clips == 0) return;
@@ -326,6 +350,7 @@ void Engine::image_focus_sweep(const huv_batch& b, const double* z, int planes, 
   for (int p = 0; p < planes; ++p)
     if (!std::isfinite(z[p])) throw Error(HUV_ERR_INVALID_PARAMETER, "focus_nm: must be finite");
   prebuild_planes(z, planes);
+  if (sweep_small(b, z, planes, out, st)) return;
   const size_t plane = static_cast<size_t>(b.n_clips) * n * n;
   for (int p = 0; p < planes; ++p) {
     huv_batch bp = b;
@@ -612,8 +637,17 @@ void Engine::run_fft_form(const huv_batch& b, const DeviceSet& ds, int M, float*
   }
 }
 
-void Engine::image_batch(const huv_batch& b, float* out, cudaStream_t st) {
-  std::lock_guard<std::mutex> lock(mu);
+void Engine::run_hybrid_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use,
+                             const float* W_use) {
+  if (small_grid(ds, M)) {
+    DeviceSet* set = &ds;
+    run_small_form(b, &set, &K_use, &W_use, 1, M, out, st);
+  } else {
+    run_tc_form(b, ds, M, out, st, K_use, W_use, kTcCoreFftField);
+  }
+}
+
+void Engine::check_batch(const huv_batch& b, const float* out) const {
   if (b.n_clips < 0) throw Error(HUV_ERR_INVALID_PARAMETER, "n_clips: must be >= 0");
   if (b.n_clips == 0) return;
   if (!b.input || !out) throw Error(HUV_ERR_INVALID_PARAMETER, "input/out: null pointer");
@@ -623,6 +657,12 @@ void Engine::image_batch(const huv_batch& b, float* out, cudaStream_t st) {
   if ((reinterpret_cast<uintptr_t>(out) & 15u) != 0 ||
       (b.input_kind != HUV_INPUT_RECTS && (reinterpret_cast<uintptr_t>(b.input) & 15u) != 0))
     throw Error(HUV_ERR_INVALID_PARAMETER, "input/out: device buffers must be 16-byte aligned");
+}
+
+void Engine::image_batch(const huv_batch& b, float* out, cudaStream_t st) {
+  std::lock_guard<std::mutex> lock(mu);
+  check_batch(b, out);
+  if (b.n_clips == 0) return;
   ensure_device();
   if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b);
   DeviceSet& ds = device_set(b.defocus_nm == 0.0 ? 0.0 : b.defocus_nm);
@@ -637,7 +677,8 @@ void Engine::image_batch(const huv_batch& b, float* out, cudaStream_t st) {
   if (form == HUV_FORM_AUTO) form = hybrid_supported(ds, M) ? HUV_FORM_HYBRID : HUV_FORM_FFT;
   if (form == HUV_FORM_HYBRID) {
     if (!hybrid_supported(ds, M)) throw Error(HUV_ERR_UNSUPPORTED, "hybrid form: band or grid outside what its kernels support");
-    run_tc_form(b, ds, M, out, st, 0, nullptr, kTcCoreFftField);
+    const int ms = small_grid(ds, b.eval_grid);
+    run_hybrid_form(b, ds, ms ? ms : M, out, st);
   } else if (form == HUV_FORM_TC || form == HUV_FORM_TC_ROWS) {
     if (!tc_supported(ds, Mtc)) throw Error(HUV_ERR_UNSUPPORTED, "TC form: band or grid outside what its kernels support");
     run_tc_form(b, ds, Mtc, out, st, 0, nullptr, form == HUV_FORM_TC_ROWS ? kTcCoreGemmRows : kTcCoreFftRows);

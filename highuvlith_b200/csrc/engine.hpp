@@ -179,6 +179,14 @@ struct SurrogateReport {
   std::vector<double> judge_errors;  // max relative image error at each judge
 };
 
+// One focus plane of a narrow-band field pass (csrc/cuda/field_small.cu).
+struct SmallPlane {
+  const float2* kband;
+  const float* W;
+  int K;
+  float keep, flare;
+};
+
 struct CacheEntry {
   double z = 0;
   std::shared_ptr<KernelSet> ks;
@@ -254,6 +262,20 @@ struct Engine {
                     const float* W_use = nullptr);
   void run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use = 0,
                    const float* W_use = nullptr, int core = kTcCoreFftRows);
+  // The hybrid form of narrow bands: `requested` (0 = automatic) as an
+  // evaluation grid of the narrow-band field kernel, or 0 where it does not
+  // apply; the automatic grid is the smallest multiple of 16 above 4h.
+  int small_grid(const DeviceSet& ds, int requested) const;
+  // The batch on every plane of `sets` (kernel sets of equal band); out is
+  // [plane][clip][y][x].  K_use / W_use: per plane, as in run_fft_form (may be
+  // null).
+  void run_small_form(const huv_batch& b, DeviceSet* const* sets, const int* K_use, const float* const* W_use,
+                      int planes, int M, float* out, cudaStream_t st);
+  // The hybrid form on M: the narrow-band kernel where it serves M, else run_tc_form.
+  void run_hybrid_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use = 0,
+                       const float* W_use = nullptr);
+  void check_batch(const huv_batch& b, const float* out) const;
+  bool sweep_small(const huv_batch& b, const double* z, int planes, float* out, cudaStream_t st);
   // Separable band interpolation of nc coarse images to the N grid on
   // tcgen05: im_split holds I_M / interp_scale(mean) as FP16 hi/lo planes
   // [clip][2][M][M] (socs_cols_split), BI is 2 N M halves of workspace per

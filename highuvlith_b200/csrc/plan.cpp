@@ -128,7 +128,7 @@ struct Plan {
     if (c.form == HUV_FORM_TC)
       g.e->run_tc_form(b, ds, c.M, out, st, g.K, g.W);
     else if (c.form == HUV_FORM_HYBRID)
-      g.e->run_tc_form(b, ds, c.M, out, st, g.K, g.W, kTcCoreFftField);
+      g.e->run_hybrid_form(b, ds, c.M, out, st, g.K, g.W);
     else
       g.e->run_fft_form(b, ds, c.M, out, st, g.K, g.W);
     if (!g.contiguous) {
@@ -156,7 +156,8 @@ std::vector<Choice> candidates(Engine* e, DeviceSet& ds) {
   // between 4h and the next power of two
   const int mx = e->choose_eval_grid(ds, 0, true);
   if (mtc <= n && e->tc_supported(ds, mtc)) out.push_back(Choice{HUV_FORM_TC, mtc, 0});
-  if (e->hybrid_supported(ds, mx)) out.push_back(Choice{HUV_FORM_HYBRID, mx, 0});
+  const int ms = e->small_grid(ds, 0);  // narrow bands: the field kernel's own grid
+  if (e->hybrid_supported(ds, mx)) out.push_back(Choice{HUV_FORM_HYBRID, ms ? ms : mx, 0});
   if (mx != m) out.push_back(Choice{HUV_FORM_FFT, mx, 0});
   out.push_back(Choice{HUV_FORM_FFT, m, 0});
   if (2 * m <= n && m < n) out.push_back(Choice{HUV_FORM_FFT, 2 * m, 0});
