@@ -38,8 +38,18 @@ bool fno_tc_layer(int B, int S, int m, const __nv_bfloat16* v, const __nv_bfloat
 bool fno_tc_proj(int B, int S, const __nv_bfloat16* v, const __nv_bfloat16* Q1b, const float* b1, const float* q2,
                  const float* b2, float* out, int* err, cudaStream_t st);
 void fno_tc_to_bf16(const float* a, int n, __nv_bfloat16* b, cudaStream_t st);
-void fno_tc_pack_zs(const float2* Z, int rows, int m, int S, __nv_bfloat16* Zs, cudaStream_t st);
 void fno_tc_tw_table(const float2* twx, int S, int m, __nv_bfloat16* Tw, cudaStream_t st);
+// DFTs over the retained modes and the lift (csrc/cuda/fno_dft.cu)
+cudaError_t fno_dft_x_bf16(const __nv_bfloat16* in, int S, int m, const float2* twt, float2* out, int rows,
+                           cudaStream_t st);
+cudaError_t fno_dft_x_f32(const float* in, int S, int m, const float2* twt, float2* out, int rows, cudaStream_t st);
+cudaError_t fno_dft_y(const float2* in, int B, int S, int m, const float2* tyt, float2* out, cudaStream_t st);
+cudaError_t fno_idft_y(const float2* in, int B, int S, int m, const float2* tyt, float2* Z, __nv_bfloat16* Zs,
+                       cudaStream_t st);
+cudaError_t fno_lift_fwd(const float* a, int B, int S, const float* Wl, const float* bl, __nv_bfloat16* v,
+                         cudaStream_t st);
+cudaError_t fno_lift_back(const float* a, const float* dv0, int B, int S, const float* Wl, float* dWl, float* dbl,
+                          float* da, cudaStream_t st);
 }  // namespace huv_launch
 
 namespace huv_dev {
@@ -52,20 +62,6 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }
 __device__ __forceinline__ float ld(const __nv_bfloat16* p, size_t i) { return __bfloat162float(p[i]); }
 __device__ __forceinline__ float ld(const float* p, size_t i) { return p[i]; }
-
-// ------------------------------------------------------------ lift
-// v0[b][p][c] = Wl[c][0] a + Wl[c][1] x/S + Wl[c][2] y/S + bl[c]
-__global__ void fno_lift(const float* __restrict__ a, int S, int C, const float* __restrict__ Wl,
-                         const float* __restrict__ bl, __nv_bfloat16* __restrict__ v, size_t total) {
-  for (size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(t % C);
-    const size_t bp = t / C;
-    const int p = static_cast<int>(bp % (static_cast<size_t>(S) * S));
-    const float gx = static_cast<float>(p % S) / S, gy = static_cast<float>(p / S) / S;
-    v[t] = __float2bfloat16_rn(Wl[c * 3] * a[bp] + Wl[c * 3 + 1] * gx + Wl[c * 3 + 2] * gy + bl[c]);
-  }
-}
 
 // ------------------------------------------------------------ register tiles
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -83,123 +79,6 @@ __device__ __forceinline__ void st_bf16x4(__nv_bfloat16* p, float a, float b, fl
   u.x = *reinterpret_cast<uint32_t*>(&lo);
   u.y = *reinterpret_cast<uint32_t*>(&hi);
   *reinterpret_cast<uint2*>(p) = u;
-}
-
-// ------------------------------------------------------------ DFT along x
-// out[r][kx][c] (complex) = sum_x in[r][x][c] e^{-2 pi i kx x / S} for rows r
-// (= (b, y)), kx < m <= 16, C = 64.  Rows are grid-strided; x runs in chunks
-// of up to 128 split over four thread groups; thread (kg, cg) of a group owns
-// kx 4kg..4kg+3 x c 4cg..4cg+3 (complex), the groups are summed at the end.
-// Dynamic shared memory: 48 KiB.
-template <typename T>
-__global__ void __launch_bounds__(256) fno_dft_x(const T* __restrict__ in, int S, int m,
-                                                  const float2* __restrict__ twx, float2* __restrict__ out,
-                                                  int rows) {
-  constexpr int C = 64, XC = 128;
-  extern __shared__ __align__(16) float dsm[];
-  float* sIn = dsm;                                        // [XC][C]
-  float2* sTw = reinterpret_cast<float2*>(sIn + XC * C);   // [16][XC]
-  float2* red = reinterpret_cast<float2*>(sIn);            // [4][16][C], aliases sIn
-  const int t = threadIdx.x;
-  const int grp = t >> 6, kg = t & 3, cg = (t >> 2) & 15;
-  const int xc = min(XC, S), xs = xc >> 2;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    float acc[4][4][2];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[q][c][0] = acc[q][c][1] = 0.f;
-    const size_t row = static_cast<size_t>(r) * S * C;
-    for (int x0 = 0; x0 < S; x0 += xc) {
-      __syncthreads();
-      for (int e = t; e < xc * C; e += 256) sIn[e] = ld(in, row + static_cast<size_t>(x0) * C + e);
-      for (int e = t; e < 16 * xc; e += 256) {
-        const int kx = e / xc, x = e - kx * xc;
-        sTw[e] = kx < m ? __ldg(twx + static_cast<size_t>(kx) * S + x0 + x) : make_float2(0.f, 0.f);
-      }
-      __syncthreads();
-      for (int xx = 0; xx < xs; ++xx) {
-        const int x = grp * xs + xx;
-        const float4 a = ld4(sIn + x * C + cg * 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 w = sTw[(kg * 4 + q) * xc + x];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            acc[q][c][0] = fmaf(av[c], w.x, acc[q][c][0]);
-            acc[q][c][1] = fmaf(av[c], w.y, acc[q][c][1]);
-          }
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        red[(grp * 16 + kg * 4 + q) * C + cg * 4 + c] = make_float2(acc[q][c][0], acc[q][c][1]);
-    __syncthreads();
-    for (int e = t; e < m * C; e += 256) {
-      float2 sum = red[e];
-#pragma unroll
-      for (int g = 1; g < 4; ++g) {
-        const float2 v = red[g * 16 * C + e];
-        sum.x += v.x;
-        sum.y += v.y;
-      }
-      out[static_cast<size_t>(r) * m * C + e] = sum;
-    }
-  }
-}
-
-// ------------------------------------------------------------ DFT along y
-// Forward (to modes): out[b][j][col] = sum_y in[b][y][col] twy[j][y], col =
-// (kx, c) over m * C columns; grid (ceil(mC / 64), B), thread (col, j group
-// of 8), J = 2m <= 32.
-// Inverse (from modes): out[b][y][col] = sum_j in[b][j][col] conj(twy[j][y]);
-// grid (S, B).  twy[j][y] = e^{-2 pi i ky_j y / S}.
-template <bool INVERSE>
-__global__ void __launch_bounds__(256) fno_dft_y(const float2* __restrict__ in, int S, int C, int m,
-                                                  const float2* __restrict__ twy, float2* __restrict__ out) {
-  const int J = 2 * m, mC = m * C;
-  if (!INVERSE) {
-    const int b = blockIdx.y;
-    const int col = blockIdx.x * 64 + (threadIdx.x & 63);
-    const int j0 = (threadIdx.x >> 6) * 8;
-    if (col >= mC || j0 >= J) return;
-    float2 acc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = make_float2(0.f, 0.f);
-    const float2* src = in + static_cast<size_t>(b) * S * mC + col;
-    for (int y = 0; y < S; ++y) {
-      const float2 v = src[static_cast<size_t>(y) * mC];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        if (j0 + q < J) {
-          const float2 w = __ldg(twy + static_cast<size_t>(j0 + q) * S + y);
-          acc[q].x = fmaf(v.x, w.x, fmaf(-v.y, w.y, acc[q].x));
-          acc[q].y = fmaf(v.x, w.y, fmaf(v.y, w.x, acc[q].y));
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (j0 + q < J) out[(static_cast<size_t>(b) * J + j0 + q) * mC + col] = acc[q];
-  } else {
-    const int r = blockIdx.x, b = blockIdx.y;
-    for (int t = threadIdx.x; t < mC; t += blockDim.x) {
-      float re = 0.f, im = 0.f;
-      for (int q = 0; q < J; ++q) {
-        const float2 v = in[(static_cast<size_t>(b) * J + q) * mC + t];
-        float2 w = __ldg(twy + static_cast<size_t>(q) * S + r);
-        w.y = -w.y;
-        re += v.x * w.x - v.y * w.y;
-        im += v.x * w.y + v.y * w.x;
-      }
-      out[(static_cast<size_t>(b) * S + r) * mC + t] = make_float2(re, im);
-    }
-  }
 }
 
 // ------------------------------------------------------------ mode mixing
@@ -655,53 +534,6 @@ __global__ void __launch_bounds__(256) fno_proj_bwd(const __nv_bfloat16* __restr
   }
 }
 
-// Lift backward: dWl, dbl and the input gradient da = sum_c Wl[c][0] dv0[c].
-// Thread (c, lane group) accumulates over pixels in registers; block 256, C = 64.
-__global__ void __launch_bounds__(256) fno_lift_bwd(const float* __restrict__ a, const float* __restrict__ dv0,
-                                                     int S, const float* __restrict__ Wl, size_t npix,
-                                                     float* __restrict__ dWl, float* __restrict__ dbl,
-                                                     float* __restrict__ da) {
-  constexpr int C = 64;
-  __shared__ float red[4][C][4];
-  const int c = threadIdx.x % C, grp = threadIdx.x / C;  // 4 groups of 64
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  const size_t SS = static_cast<size_t>(S) * S;
-  for (size_t p = blockIdx.x * 4 + grp; p < npix; p += static_cast<size_t>(gridDim.x) * 4) {
-    const int pp = static_cast<int>(p % SS);
-    const float gx = static_cast<float>(pp % S) / S, gy = static_cast<float>(pp / S) / S;
-    const float d = dv0[p * C + c];
-    s0 += d * a[p];
-    s1 += d * gx;
-    s2 += d * gy;
-    s3 += d;
-  }
-  red[grp][c][0] = s0;
-  red[grp][c][1] = s1;
-  red[grp][c][2] = s2;
-  red[grp][c][3] = s3;
-  __syncthreads();
-  if (threadIdx.x < C) {
-    float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
-    for (int g = 0; g < 4; ++g) {
-      t0 += red[g][threadIdx.x][0];
-      t1 += red[g][threadIdx.x][1];
-      t2 += red[g][threadIdx.x][2];
-      t3 += red[g][threadIdx.x][3];
-    }
-    atomicAdd(dWl + threadIdx.x * 3, t0);
-    atomicAdd(dWl + threadIdx.x * 3 + 1, t1);
-    atomicAdd(dWl + threadIdx.x * 3 + 2, t2);
-    atomicAdd(dbl + threadIdx.x, t3);
-  }
-  if (da)
-    for (size_t p = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; p < npix;
-         p += static_cast<size_t>(gridDim.x) * blockDim.x) {
-      float acc = 0.f;
-      for (int k = 0; k < C; ++k) acc += Wl[k * 3] * dv0[p * C + k];
-      da[p] = acc;
-    }
-}
-
 // MSE loss on [B][S][S]: dout = 2 (out - tgt) / n (and loss parts).
 __global__ void fno_mse(const float* __restrict__ out, const float* __restrict__ tgt, size_t n,
                         float* __restrict__ dout, float* __restrict__ loss) {
@@ -749,7 +581,8 @@ struct Fno {
   size_t oWl, obl, oQ1, ob1, oQ2, ob2;
   std::vector<size_t> oR, oW, ob;
   float *par = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
-  float2 *twx = nullptr, *twy = nullptr;
+  float2 *twx = nullptr;                   // [kx][x]
+  float2 *twt = nullptr, *tyt = nullptr;   // [x][16] and [y][32], zero past the retained modes
   int64_t adam_t = 0;
   // tensor-core forward (grids of at least 128): bf16 weights, twiddle table,
   // packed spectral operand, device error flag
@@ -804,28 +637,26 @@ struct Fno {
     check_cuda(cudaMemcpy(par, h.data(), npar * 4, cudaMemcpyHostToDevice), "upload fno params");
     check_cuda(cudaMemset(m1, 0, npar * 4), "memset");
     check_cuda(cudaMemset(m2, 0, npar * 4), "memset");
-    std::vector<float2> tx(static_cast<size_t>(m) * S), ty(static_cast<size_t>(J) * S);
+    std::vector<float2> tx(static_cast<size_t>(m) * S), txt(static_cast<size_t>(S) * 16, make_float2(0.f, 0.f)),
+        tyt_h(static_cast<size_t>(S) * 32, make_float2(0.f, 0.f));
+    auto w = [&](int k, int x) {
+      const double a = -2.0 * 3.14159265358979323846 * k * static_cast<double>(x) / S;
+      return make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
+    };
     for (int k = 0; k < m; ++k)
-      for (int x = 0; x < S; ++x) {
-        const double a = -2.0 * 3.14159265358979323846 * k * static_cast<double>(x) / S;
-        tx[static_cast<size_t>(k) * S + x] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
-      }
-    for (int j = 0; j < J; ++j) {
-      const int ky = j < m ? j : j - J;
-      for (int y = 0; y < S; ++y) {
-        const double a = -2.0 * 3.14159265358979323846 * ky * static_cast<double>(y) / S;
-        ty[static_cast<size_t>(j) * S + y] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
-      }
-    }
-    check_cuda(cudaMalloc(&twx, tx.size() * 8), "cudaMalloc(twx)");
-    check_cuda(cudaMalloc(&twy, ty.size() * 8), "cudaMalloc(twy)");
-    check_cuda(cudaMemcpy(twx, tx.data(), tx.size() * 8, cudaMemcpyHostToDevice), "upload twx");
-    check_cuda(cudaMemcpy(twy, ty.data(), ty.size() * 8, cudaMemcpyHostToDevice), "upload twy");
+      for (int x = 0; x < S; ++x) tx[static_cast<size_t>(k) * S + x] = txt[static_cast<size_t>(x) * 16 + k] = w(k, x);
+    for (int j = 0; j < J; ++j)
+      for (int y = 0; y < S; ++y) tyt_h[static_cast<size_t>(y) * 32 + j] = w(j < m ? j : j - J, y);
+    auto table = [&](float2** d, const std::vector<float2>& h2) {
+      check_cuda(cudaMalloc(d, h2.size() * 8), "cudaMalloc(fno twiddles)");
+      check_cuda(cudaMemcpy(*d, h2.data(), h2.size() * 8, cudaMemcpyHostToDevice), "upload fno twiddles");
+    };
+    table(&twx, tx);
+    table(&twt, txt);
+    table(&tyt, tyt_h);
     static std::atomic<uint64_t> attr{0};
     huv::once_per_device(attr, [] {
       const int big = 200 * 1024;
-      check_cuda(cudaFuncSetAttribute(huv_dev::fno_dft_x<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
-      check_cuda(cudaFuncSetAttribute(huv_dev::fno_dft_x<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
       check_cuda(cudaFuncSetAttribute(huv_dev::fno_proj, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
       check_cuda(cudaFuncSetAttribute(huv_dev::fno_proj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
       check_cuda(cudaFuncSetAttribute(huv_dev::fno_layer_out, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
@@ -880,7 +711,8 @@ struct Fno {
     cudaFree(m1);
     cudaFree(m2);
     cudaFree(twx);
-    cudaFree(twy);
+    cudaFree(twt);
+    cudaFree(tyt);
   }
 
   void ensure(int B) {
@@ -916,7 +748,6 @@ struct Fno {
   }
 
   // Launch shapes and dynamic shared memory of the tiled kernels.
-  static constexpr size_t kDftXSmem = (128 * 64 + 16 * 128 * 2) * 4;
   static constexpr size_t kProjSmem = (64 * 128 + 64 * 68) * 4;
   static constexpr size_t kProjBwdSmem = (2 * 64 * 128 + 2 * 64 * 68 + 64 * 132 + 128 * 68 + 64) * 4;
   static constexpr size_t kLayerBwdSmem = (64 * 64 + 3 * 64 * 68) * 4;
@@ -931,18 +762,17 @@ struct Fno {
     const size_t pix = static_cast<size_t>(B) * S * S;
     const int rows = B * S;
     const dim3 rgrid(std::min(rows, 4096));
-    const dim3 ygrid((m * C + 63) / 64, B);
-    fno_lift<<<2048, 256, 0, st>>>(masks, S, C, par + oWl, par + obl, v[0], pix * C);
+    using namespace huv_launch;
+    check_cuda(fno_lift_fwd(masks, B, S, par + oWl, par + obl, v[0], st), "fno lift");
     for (int l = 0; l < L; ++l) {
-      fno_dft_x<__nv_bfloat16><<<rgrid, 256, kDftXSmem, st>>>(v[l], S, m, twx, Xa, rows);
-      fno_dft_y<false><<<ygrid, 256, 0, st>>>(Xa, S, C, m, twy, Xl[l]);
+      check_cuda(fno_dft_x_bf16(v[l], S, m, twt, Xa, rows, st), "fno dft x");
+      check_cuda(fno_dft_y(Xa, B, S, m, tyt, Xl[l], st), "fno dft y");
       fno_mix<<<dim3(modes, B), C, C * 8, st>>>(Xl[l], reinterpret_cast<const float2*>(par + oR[l]), C, modes, Y);
-      fno_dft_y<true><<<dim3(S, B), 256, 0, st>>>(Y, S, C, m, twy, Za);
+      check_cuda(fno_idft_y(Y, B, S, m, tyt, Za, tc ? zs : nullptr, st), "fno inverse dft y");
       if (tc) {
-        huv_launch::fno_tc_to_bf16(par + oW[l], C * C, wb + static_cast<size_t>(l) * C * C, st);
-        huv_launch::fno_tc_pack_zs(Za, rows, m, S, zs, st);
-        if (!huv_launch::fno_tc_layer(B, S, m, v[l], wb + static_cast<size_t>(l) * C * C, tw_tab, zs, par + ob[l],
-                                      l < L - 1 ? 1 : 0, z[l], v[l + 1], tc_err, st))
+        fno_tc_to_bf16(par + oW[l], C * C, wb + static_cast<size_t>(l) * C * C, st);
+        if (!fno_tc_layer(B, S, m, v[l], wb + static_cast<size_t>(l) * C * C, tw_tab, zs, par + ob[l],
+                          l < L - 1 ? 1 : 0, z[l], v[l + 1], tc_err, st))
           throw Error(HUV_ERR_CUDA, "fno: tensor-core layer launch failed");
       } else {
         fno_layer_out<<<rgrid, 256, layer_out_smem(), st>>>(
@@ -967,7 +797,6 @@ struct Fno {
     const size_t pix = static_cast<size_t>(B) * S * S;
     const int rows = B * S;
     const dim3 rgrid(std::min(rows, 4096));
-    const dim3 ygrid((m * C + 63) / 64, B);
     check_cuda(cudaMemsetAsync(grad, 0, npar * 4, st), "memset grad");
     if (tc) {
       if (!huv_launch::fno_tc_proj_bwd(pix, v[L], par + oQ1, par + ob1, par + oQ2, dOut, dvA, grad + oQ1, grad + ob1,
@@ -988,17 +817,18 @@ struct Fno {
         fno_layer_bwd<<<std::min(rows, 296), 256, kLayerBwdSmem, st>>>(
             dnext, z[l], v[l], par + oW[l], S, l < L - 1 ? 1 : 0, dz, dcur, grad + oW[l], grad + ob[l], rows);
       }
-      fno_dft_x<float><<<rgrid, 256, kDftXSmem, st>>>(dz, S, m, twx, Xa, rows);
-      fno_dft_y<false><<<ygrid, 256, 0, st>>>(Xa, S, C, m, twy, Y);
+      check_cuda(huv_launch::fno_dft_x_f32(dz, S, m, twt, Xa, rows, st), "fno dft x");
+      check_cuda(huv_launch::fno_dft_y(Xa, B, S, m, tyt, Y, st), "fno dft y");
       fno_scale_modes<<<256, 256, 0, st>>>(Y, B, J, m, C, 1.f / (static_cast<float>(S) * S));
       fno_mix_bwd<<<modes, 256, static_cast<size_t>(2) * B * C * 8, st>>>(
           Xl[l], Y, reinterpret_cast<const float2*>(par + oR[l]), C, modes, B, dX,
           reinterpret_cast<float2*>(grad + oR[l]));
-      fno_dft_y<true><<<dim3(S, B), 256, 0, st>>>(dX, S, C, m, twy, Za);
+      check_cuda(huv_launch::fno_idft_y(dX, B, S, m, tyt, Za, nullptr, st), "fno inverse dft y");
       fno_spec_to_dv<<<rgrid, 256, spec_smem(), st>>>(Za, S, m, twx, dcur, rows);
       std::swap(dnext, dcur);
     }
-    fno_lift_bwd<<<1184, 256, 0, st>>>(masks, dnext, S, par + oWl, pix, grad + oWl, grad + obl, dmask);
+    check_cuda(huv_launch::fno_lift_back(masks, dnext, B, S, par + oWl, grad + oWl, grad + obl, dmask, st),
+               "fno lift backward");
     check_cuda(cudaGetLastError(), "fno backward");
   }
 

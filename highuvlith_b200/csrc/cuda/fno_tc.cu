@@ -748,26 +748,6 @@ __global__ void fno_to_bf16(const float* __restrict__ a, int n, __nv_bfloat16* _
     b[i] = __float2bfloat16_rn(a[i]);
 }
 
-// Zs[r][o][kk] (bf16, kk < 64): kk = 2 kx -> w Re Z, 2 kx + 1 -> -w Im Z,
-// w = (kx ? 2 : 1) / S^2, zero for kk >= 2m; Z: [r][kx][o] float2 (r = b S + y).
-__global__ void fno_zs_pack(const float2* __restrict__ Z, int rows, int m, int S, __nv_bfloat16* __restrict__ Zs) {
-  const float inv = 1.f / (static_cast<float>(S) * S);
-  const size_t total = static_cast<size_t>(rows) * 64 * 64;
-  for (size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int kk = static_cast<int>(t & 63), o = static_cast<int>((t >> 6) & 63);
-    const size_t r = t >> 12;
-    float v = 0.f;
-    if (kk < 2 * m) {
-      const int kx = kk >> 1;
-      const float w = (kx == 0 ? 1.f : 2.f) * inv;
-      const float2 z = Z[(r * m + kx) * 64 + o];
-      v = (kk & 1) ? -w * z.y : w * z.x;
-    }
-    Zs[t] = __float2bfloat16_rn(v);
-  }
-}
-
 // Tw[x][kk] (bf16): cos / sin of 2 pi kx x / S for kk = 2 kx / 2 kx + 1 < 2m,
 // zero beyond; from twx[kx][x] = (cos, -sin).
 __global__ void fno_tw_table(const float2* __restrict__ twx, int S, int m, __nv_bfloat16* __restrict__ Tw) {
@@ -903,9 +883,6 @@ bool fno_tc_proj_bwd(size_t pix, const __nv_bfloat16* v, const float* Q1, const 
 }
 void fno_tc_to_bf16(const float* a, int n, __nv_bfloat16* b, cudaStream_t st) {
   huv_dev::fno_to_bf16<<<(n + 255) / 256, 256, 0, st>>>(a, n, b);
-}
-void fno_tc_pack_zs(const float2* Z, int rows, int m, int S, __nv_bfloat16* Zs, cudaStream_t st) {
-  huv_dev::fno_zs_pack<<<2048, 256, 0, st>>>(Z, rows, m, S, Zs);
 }
 void fno_tc_tw_table(const float2* twx, int S, int m, __nv_bfloat16* Tw, cudaStream_t st) {
   huv_dev::fno_tw_table<<<(S * 64 + 255) / 256, 256, 0, st>>>(twx, S, m, Tw);
