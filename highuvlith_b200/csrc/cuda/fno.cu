@@ -668,7 +668,7 @@ struct Fno {
       check_cuda(huv_launch::fno_tc_set_smem(), "cudaFuncSetAttribute(fno tc)");
       check_cuda(cudaMalloc(&wb, static_cast<size_t>(L) * C * C * 2), "cudaMalloc(fno wb)");
       check_cuda(cudaMalloc(&q1b, static_cast<size_t>(P) * C * 2), "cudaMalloc(fno q1b)");
-      check_cuda(cudaMalloc(&tw_tab, static_cast<size_t>(S) * 64 * 2), "cudaMalloc(fno tw)");
+      check_cuda(cudaMalloc(&tw_tab, static_cast<size_t>(S) * 32 * 2), "cudaMalloc(fno tw)");
       check_cuda(cudaMalloc(&tc_err, sizeof(int)), "cudaMalloc(fno err)");
       check_cuda(cudaMemset(tc_err, 0, sizeof(int)), "memset");
       huv_launch::fno_tc_tw_table(twx, S, m, tw_tab, nullptr);
@@ -743,7 +743,7 @@ struct Fno {
     al(reinterpret_cast<void**>(&dvB), pix * C * 4);
     al(reinterpret_cast<void**>(&dz), pix * C * 4);
     al(reinterpret_cast<void**>(&loss), 4);
-    if (tc) al(reinterpret_cast<void**>(&zs), static_cast<size_t>(B) * S * 64 * 64 * 2);
+    if (tc) al(reinterpret_cast<void**>(&zs), static_cast<size_t>(B) * S * 64 * 32 * 2);
     B_cap = B;
   }
 
@@ -755,8 +755,9 @@ struct Fno {
   size_t spec_smem() const { return (2 * static_cast<size_t>(m) * (64 + 68)) * 4; }
   static unsigned pgrid(size_t pix) { return static_cast<unsigned>(std::min<size_t>((pix + 63) / 64, 296)); }
 
-  // images[b][S][S] = FNO(masks[b]); activations kept for backward.
-  void forward(int B, const float* masks, float* images, cudaStream_t st) {
+  // images[b][S][S] = FNO(masks[b]); with `keep`, everything a backward pass
+  // reads is kept (z is written for it alone).
+  void forward(int B, const float* masks, float* images, cudaStream_t st, bool keep = true) {
     using namespace huv_dev;
     ensure(B);
     const size_t pix = static_cast<size_t>(B) * S * S;
@@ -772,7 +773,7 @@ struct Fno {
       if (tc) {
         fno_tc_to_bf16(par + oW[l], C * C, wb + static_cast<size_t>(l) * C * C, st);
         if (!fno_tc_layer(B, S, m, v[l], wb + static_cast<size_t>(l) * C * C, tw_tab, zs, par + ob[l],
-                          l < L - 1 ? 1 : 0, z[l], v[l + 1], tc_err, st))
+                          l < L - 1 ? 1 : 0, keep ? z[l] : nullptr, v[l + 1], tc_err, st))
           throw Error(HUV_ERR_CUDA, "fno: tensor-core layer launch failed");
       } else {
         fno_layer_out<<<rgrid, 256, layer_out_smem(), st>>>(
@@ -948,7 +949,7 @@ huv_status huv_fno_forward(void* fno, int32_t batch, const float* masks, float* 
     Fno* f = as_fno(fno);
     if (batch <= 0 || !masks || !images) throw Error(HUV_ERR_INVALID_PARAMETER, "fno forward: arguments");
     huv::check_cuda(cudaSetDevice(f->device), "cudaSetDevice");
-    f->forward(batch, masks, images, static_cast<cudaStream_t>(stream));
+    f->forward(batch, masks, images, static_cast<cudaStream_t>(stream), false);
   });
 }
 

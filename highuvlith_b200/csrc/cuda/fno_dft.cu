@@ -32,6 +32,20 @@ __device__ __forceinline__ void load4(const float* p, float (&a)[4]) {
   a[2] = u.z;
   a[3] = u.w;
 }
+// Two FP32 multiply-adds in one instruction (each rounded as fmaf).
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
 }  // namespace
 
 // ------------------------------------------------------------ DFT along x
@@ -42,11 +56,12 @@ __device__ __forceinline__ void load4(const float* p, float (&a)[4]) {
 // multiply-add per term); the groups are added as ((0 + 1) + 2) + 3.
 //
 // 512 threads take four rows; a thread owns 8 kx x 4 c, so that a step of x
-// costs five shared loads for 64 multiply-adds (bound by FP32 issue: the
-// 4 x 4 tile it replaces spent three loads on 32 and staged its input with
-// blocking 2-byte loads).  Input and twiddles arrive by cp.async, two stages;
-// a stage is a chunk of BF16 or half of one of FP32 (the same bytes).
-// 16 x 512^2: 1.21 -> 0.39 ms BF16; 8 x 512^2: 0.617 -> 0.24 ms FP32.
+// costs five shared loads for 32 paired multiply-adds (bound by FP32 issue:
+// the 4 x 4 tile it replaces spent five loads on 32 single ones and staged
+// its input with blocking 2-byte loads).  Input and twiddles arrive by
+// cp.async, two stages; a stage is a chunk of BF16 or half of one of FP32
+// (the same bytes).  16 x 512^2 BF16: 1.21 -> 0.46 ms (0.57 with single
+// multiply-adds); 8 x 512^2 FP32: 0.617 -> 0.26 ms.
 constexpr int kDxRows = 4;
 template <typename T>
 __host__ __device__ constexpr int dx_split() { return sizeof(T) == 4 ? 2 : 1; }  // stages per chunk
@@ -73,35 +88,40 @@ __global__ void __launch_bounds__(512, 1) fno_dft_x(const T* __restrict__ in, in
   float2* red = reinterpret_cast<float2*>(dsm8 + 2 * kStage);  // [rows][16][C]
   const int sets = rows / kDxRows;
   const int mine = blockIdx.x < sets ? (sets - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  // stage q of this block: row set q / per, step q % per
+  // stage q of this block: row set q / per, step q % per; every length is a
+  // power of two
+  const int lhs = 31 - __clz(hs);
   auto issue = [&](int q) {
-    const int r0 = (blockIdx.x + (q / per) * gridDim.x) * kDxRows, st = q % per;
+    const int set = q / per, st = q - set * per;
+    const int r0 = (blockIdx.x + set * gridDim.x) * kDxRows;
     const int x0 = (st / split) * xc + (st % split) * hs;
     uint8_t* dst = dsm8 + (q & 1) * kStage;
     // [row][g hs + i][C]: x = x0 + g xs + i
     constexpr int kPer16 = 16 / sizeof(T), kVec = C / kPer16;  // 16-byte copies per x
-    const int nvec = kDxRows * sx * kVec;
+    constexpr int lkVec = kVec == 8 ? 3 : 4;
+    const T* src = in + (static_cast<size_t>(r0) * S + x0) * C;
+    const int nvec = (kDxRows * kVec) << (lhs + 2);
     for (int e = t; e < nvec; e += 512) {
-      const int v = e % kVec, xx = (e / kVec) % sx, row = e / (kVec * sx);
-      const int x = x0 + (xx / hs) * xs + xx % hs;
-      cp16(dst + static_cast<size_t>(e) * 16, in + (static_cast<size_t>(r0 + row) * S + x) * C + v * kPer16);
+      const int v = e & (kVec - 1), xx = (e >> lkVec) & (sx - 1), row = e >> (lkVec + lhs + 2);
+      const int x = (xx >> lhs) * xs + (xx & (hs - 1));
+      cp16(dst + static_cast<size_t>(e) * 16, src + (static_cast<size_t>(row) * S + x) * C + v * kPer16);
     }
     for (int e = t; e < sx * 8; e += 512) {
       const int v = e & 7, xx = e >> 3;
-      const int x = x0 + (xx / hs) * xs + xx % hs;
+      const int x = x0 + (xx >> lhs) * xs + (xx & (hs - 1));
       cp16(dst + dbytes + static_cast<size_t>(e) * 16, twt + static_cast<size_t>(x) * 16 + v * 2);
     }
     fr_cp_commit();
   };
-  float acc[8][4][2];
+  uint64_t acc[8][4];  // (re, im)
   const int total = mine * per;
   if (total > 0) issue(0);
-  for (int q = 0; q < total; ++q) {
-    if (q % per == 0)
+  for (int q = 0, step = 0; q < total; ++q, step = step + 1 == per ? 0 : step + 1) {
+    if (step == 0)
 #pragma unroll
       for (int k = 0; k < 8; ++k)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[k][c][0] = acc[k][c][1] = 0.f;
+        for (int c = 0; c < 4; ++c) acc[k][c] = 0;
     if (q + 1 < total) {
       issue(q + 1);
       fr_cp_wait<1>();
@@ -111,24 +131,25 @@ __global__ void __launch_bounds__(512, 1) fno_dft_x(const T* __restrict__ in, in
     __syncthreads();
     const uint8_t* st = dsm8 + (q & 1) * kStage;
     const T* a0 = reinterpret_cast<const T*>(st) + (static_cast<size_t>(rw) * sx + grp * hs) * C + cg * 4;
-    const float4* w0 = reinterpret_cast<const float4*>(st + dbytes) + (grp * hs) * 8 + kg * 4;
+    const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(st + dbytes) + (grp * hs) * 8 + kg * 4;
 #pragma unroll 4
     for (int i = 0; i < hs; ++i) {
       float a[4];
       load4(a0 + i * C, a);
+      uint64_t a2[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) a2[c] = pack2(a[c], a[c]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float4 w = w0[i * 8 + k];
+        const ulonglong2 w = w0[i * 8 + k];  // two modes' (cos, sin)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          acc[2 * k][c][0] = fmaf(a[c], w.x, acc[2 * k][c][0]);
-          acc[2 * k][c][1] = fmaf(a[c], w.y, acc[2 * k][c][1]);
-          acc[2 * k + 1][c][0] = fmaf(a[c], w.z, acc[2 * k + 1][c][0]);
-          acc[2 * k + 1][c][1] = fmaf(a[c], w.w, acc[2 * k + 1][c][1]);
+          fma2(acc[2 * k][c], a2[c], w.x);
+          fma2(acc[2 * k + 1][c], a2[c], w.y);
         }
       }
     }
-    if (q % per == per - 1) {
+    if (step == per - 1) {
       // ((group 0 + 1) + 2) + 3 through shared memory
       const int r = (blockIdx.x + (q / per) * gridDim.x) * kDxRows + rw;
       for (int g = 0; g < 4; ++g) {
@@ -137,8 +158,10 @@ __global__ void __launch_bounds__(512, 1) fno_dft_x(const T* __restrict__ in, in
           for (int k = 0; k < 8; ++k) {
             const int kx = kg * 8 + k;
             float4* rp = reinterpret_cast<float4*>(red + (rw * 16 + kx) * C + cg * 4);
-            float4 lo = make_float4(acc[k][0][0], acc[k][0][1], acc[k][1][0], acc[k][1][1]);
-            float4 hi = make_float4(acc[k][2][0], acc[k][2][1], acc[k][3][0], acc[k][3][1]);
+            const float2 c0 = unpack2(acc[k][0]), c1 = unpack2(acc[k][1]), c2 = unpack2(acc[k][2]),
+                         c3 = unpack2(acc[k][3]);
+            float4 lo = make_float4(c0.x, c0.y, c1.x, c1.y);
+            float4 hi = make_float4(c2.x, c2.y, c3.x, c3.y);
             if (g > 0) {
               const float4 p = rp[0], s = rp[1];
               lo = make_float4(p.x + lo.x, p.y + lo.y, p.z + lo.z, p.w + lo.w);
@@ -170,7 +193,7 @@ __global__ void __launch_bounds__(512, 1) fno_dft_x(const T* __restrict__ in, in
 // 32 y of input and twiddles by cp.async, two stages.  Bound by FP32 issue
 // (32 multiply-adds for five shared loads); the kernel it replaces read every
 // twiddle of every step from global memory, one per thread and mode:
-// 16 x 512^2: 0.435 -> 0.05 ms.
+// 16 x 512^2: 0.435 -> 0.062 ms.
 constexpr int kDyY = 32;
 __global__ void __launch_bounds__(128) fno_dft_y_fwd(const float2* __restrict__ in, int S, int m,
                                                       const float2* __restrict__ tyt, float2* __restrict__ out) {
@@ -223,14 +246,13 @@ __global__ void __launch_bounds__(128) fno_dft_y_fwd(const float2* __restrict__ 
 // From modes: Z[b][y][col] = sum_j in[b][j][col] conj(w(j, y)), j ascending,
 // each complex product formed and then added.  PACK writes the layer GEMM's
 // BF16 operand instead: Zs[b S + y][c][2 kx], [2 kx + 1] = (w Re Z, -w Im Z),
-// w = (kx ? 2 : 1) / S^2, 64 wide, zero for 2m <= kk < 32 (wider columns are
-// not read).
+// w = (kx ? 2 : 1) / S^2, 32 wide, zero for kk >= 2m.
 // 128 threads take 128 columns (PACK: 16 kx x 8 c, so that a warp's stores
 // are two 64-byte runs), each with its column's modes in registers, over a
 // run of rows y whose twiddles sit in shared memory.  Bound by FP32 issue and
 // the packed stores; the kernel it replaces re-read the modes and twiddles
 // from global memory for every row, and the packing was a pass of its own:
-// 16 x 512^2: 0.425 + 0.095 -> 0.09 ms.
+// 16 x 512^2: 0.425 + 0.095 -> 0.102 ms.
 constexpr int kDyRows = 32;
 template <bool PACK>
 __global__ void __launch_bounds__(128) fno_dft_y_inv(const float2* __restrict__ in, int S, int m,
@@ -273,7 +295,7 @@ __global__ void __launch_bounds__(128) fno_dft_y_inv(const float2* __restrict__ 
       __nv_bfloat162 o;
       o.x = __float2bfloat16_rn(wk * re);
       o.y = __float2bfloat16_rn(-wk * im);
-      *reinterpret_cast<__nv_bfloat162*>(Zs + (r * 64 + c) * 64 + 2 * kx) = o;
+      *reinterpret_cast<__nv_bfloat162*>(Zs + (r * 64 + c) * 32 + 2 * kx) = o;
     } else if (live) {
       Z[r * mC + col] = make_float2(re, im);
     }
@@ -284,7 +306,7 @@ __global__ void __launch_bounds__(128) fno_dft_y_inv(const float2* __restrict__ 
 // v0[b][p][c] = Wl[c][0] a + Wl[c][1] x/S + Wl[c][2] y/S + bl[c], BF16.
 // A thread keeps the weights of eight channels and writes 16 bytes per pixel;
 // bound by the 128 bytes per pixel it writes (one 2-byte store and 64-bit
-// index divisions per element before: 16 x 512^2: 1.36 -> 0.10 ms).
+// index divisions per element before: 16 x 512^2: 1.36 -> 0.195 ms).
 __global__ void __launch_bounds__(256) fno_lift(const float* __restrict__ a, int S, const float* __restrict__ Wl,
                                                  const float* __restrict__ bl, __nv_bfloat16* __restrict__ v,
                                                  int pixels) {
@@ -314,7 +336,7 @@ __global__ void __launch_bounds__(256) fno_lift(const float* __restrict__ a, int
 // multiply-add per term).  Tiles of 64 pixels through shared memory: loaded
 // with 16-byte accesses, summed over pixels by (channel, quarter of the tile)
 // and over channels by pixel.  Bound by dv0's 256 bytes per pixel (a strided
-// load per channel before: 8 x 512^2: 0.98 -> 0.15 ms).
+// load per channel before: 8 x 512^2: 0.98 -> 0.33 ms).
 __global__ void __launch_bounds__(256) fno_lift_bwd(const float* __restrict__ a, const float* __restrict__ dv0, int S,
                                                      const float* __restrict__ Wl, int pixels,
                                                      float* __restrict__ dWl, float* __restrict__ dbl,

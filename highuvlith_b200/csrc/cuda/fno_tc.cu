@@ -1,4 +1,4 @@
-// tcgen05 channel GEMMs of the FNO forward pass (grids of at least 128).
+// tcgen05 channel GEMMs of the FNO (grids of at least 128).
 //
 // The pointwise layer and the projection head are contractions over the 64
 // channels of every pixel: [pixels x 64] x [64 x N].  Pixels are tiled by
@@ -6,18 +6,19 @@
 // channels-last BF16 activations of a tile are one 128 x 128-byte TMA box
 // (128B swizzle, K-major), the weights are resident in shared memory.
 //
-// MODE 0 (layer l): D[p][o] = sum_i v[p][i] W[o][i]
-//                           + sum_kk Tw[x(p)][kk] Zs[row(p)][o][kk]
+// fno_tc_layer: D[p][o] = sum_i v[p][i] W[o][i]
+//                       + sum_kk Tw[x(p)][kk] Zs[row(p)][o][kk]
 // where the second term is the layer's inverse x-DFT of the retained modes
 // (Tw[x][2kx] = cos, Tw[x][2kx+1] = sin of 2 pi kx x / S; Zs = (w_kx / S^2)
-// (Re Z, -Im Z) per image row), folded in as a second K block.  Epilogue:
-// z = D + b, z stored (BF16) for the backward pass, v_next = GELU(z).
-// MODE 1 (projection): D[p][j] = sum_i v[p][i] Q1[j][i], j < 128; epilogue
+// (Re Z, -Im Z) per image row; 32 wide), folded in as a second K block.
+// Epilogue: z = D + b, z stored (BF16) when a backward pass will follow,
+// v_next = GELU(z).
+// fno_tc_proj: D[p][j] = sum_i v[p][i] Q1[j][i], j < 128; epilogue
 // out[p] = sum_j Q2[j] GELU(D[p][j] + b1[j]) + b2, one pixel per thread.
 //
-// Warp roles: 0 TMA producer (no multicast), 1 MMA issuer (one thread),
-// 2..5 epilogue (one tensor-memory lane quadrant each).  Two shared-memory
-// stages, tensor memory double-buffered, two CTAs per SM.  Every mbarrier wait is bounded
+// Warp roles: 0 TMA producer (no multicast), 1 MMA issuer (one thread), then
+// the epilogue warps.  Two shared-memory stages, tensor memory
+// double-buffered, two CTAs per SM.  Every mbarrier wait is bounded
 // (2 s); a timeout sets *err and unwinds.  Operands BF16, accumulation FP32.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -25,6 +26,7 @@
 #include <stdint.h>
 
 #include "../engine.hpp"
+#include "fno_gelu.cuh"
 #include "tc_ptx.cuh"
 
 namespace huv_dev {
@@ -36,32 +38,43 @@ constexpr uint32_t kTile = 128 * 128;  // 128 rows x 64 bf16
 struct FnoTcParams {
   int tiles;          // 128-pixel tiles
   int S;              // grid side
-  int kk_steps;       // MODE 0: 16-wide K steps of the spectral block (ceil(2m / 16))
-  const float* bias;  // MODE 0: b[64]; MODE 1: b1[128]
-  const float* q2;    // MODE 1: Q2[128]
-  const float* b2;    // MODE 1: b2[1]
-  __nv_bfloat16* zsave;
-  __nv_bfloat16* vnext;
-  int act;            // MODE 0: GELU on v_next
-  float* out;         // MODE 1
+  int kk_steps;       // layer: 16-wide K steps of the spectral block (ceil(2m / 16))
+  const float* bias;  // layer: b[64]; projection: b1[128]
+  const float* q2;    // projection: Q2[128]
+  const float* b2;    // projection: b2[1]
+  int act;            // layer: GELU on v_next
+  int save_z;         // layer: z is stored
+  float* out;         // projection
   int* err;
 };
 
-__device__ __forceinline__ float tc_gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
+// Eight epilogue warps, two per tensor-memory lane quadrant (each 32 of the
+// 64 channels of its pixels); a warp stages its 32 pixels x 32 channels in
+// shared memory (64B swizzle) and stores them with TMA.  Bound by the
+// epilogue's instructions, GELU above all, beside 256 bytes per pixel (384
+// with z).  16 x 512^2: 0.68 -> 0.31 ms (3.4 TB/s); 8 x 512^2 with z: 0.345 ->
+// 0.177 ms, with two erff per pair, four epilogue warps, 16-byte stores a
+// pixel apart and z always written before.
+constexpr int kFnoEpiWarps = 8;
+constexpr uint32_t kFnoLayerStage = kTile + 128 * 64 + 64 * 64;  // v, twiddles, Zs
+constexpr uint32_t kFnoOutTile = 32 * 64;                        // 32 pixels x 32 bf16
+constexpr size_t kFnoLayerSmem =
+    1024 + 64 * 128 + kFnoStages * kFnoLayerStage + kFnoEpiWarps * 2 * kFnoOutTile + 64 * 4 + 256;
 
-template <int MODE>
-__global__ void __launch_bounds__(192, 2)
-    fno_tc_pw(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW,
-              const __grid_constant__ CUtensorMap tmTw, const __grid_constant__ CUtensorMap tmZ, FnoTcParams p) {
-  constexpr int N = MODE == 0 ? 64 : 128;
-  constexpr uint32_t kWBytes = N * 128;                              // resident weights
-  constexpr uint32_t kStage = MODE == 0 ? 2 * kTile + 64 * 128 : kTile;  // v (+ twiddles + Zs)
+__global__ void __launch_bounds__(32 * (2 + kFnoEpiWarps), 2)
+    fno_tc_layer(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW,
+                 const __grid_constant__ CUtensorMap tmTw, const __grid_constant__ CUtensorMap tmZ,
+                 const __grid_constant__ CUtensorMap tmVn, const __grid_constant__ CUtensorMap tmZo, FnoTcParams p) {
+  constexpr int N = 64;
+  constexpr uint32_t kWBytes = N * 128;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* sW = base;
   uint8_t* sS = base + kWBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sS + kFnoStages * kStage);
+  uint8_t* sO = sS + kFnoStages * kFnoLayerStage;  // [warp][v, z]
+  float* sb = reinterpret_cast<float*>(sO + kFnoEpiWarps * 2 * kFnoOutTile);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sb + 64);
   uint64_t* full = bars;
   uint64_t* empty = bars + kFnoStages;
   uint64_t* w_full = bars + 2 * kFnoStages;
@@ -71,7 +84,7 @@ __global__ void __launch_bounds__(192, 2)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kFnoStages + 6);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr uint32_t kTmemCols = 2 * N <= 128 ? 128 : 256;
+  constexpr uint32_t kTmemCols = 128;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kFnoStages; ++s) {
@@ -81,12 +94,13 @@ __global__ void __launch_bounds__(192, 2)
     mbar_init(w_full, 1);
     mbar_init(&tfull[0], 1);
     mbar_init(&tfull[1], 1);
-    mbar_init(&tempty[0], 4);
-    mbar_init(&tempty[1], 4);
+    mbar_init(&tempty[0], kFnoEpiWarps);
+    mbar_init(&tempty[1], kFnoEpiWarps);
     mbar_init(done, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (threadIdx.x < 64) sb[threadIdx.x] = p.bias[threadIdx.x];
   if (warp == 0) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -110,19 +124,17 @@ __global__ void __launch_bounds__(192, 2)
       int it = 0;
       for (int t = blockIdx.x; t < p.tiles && !*abort_flag; t += gridDim.x, ++it) {
         const int s = it % kFnoStages;
-        if (!mbar_wait(&empty[s], ((it / kFnoStages) & 1) ^ 1, kFnoWaitNs)) {
+        if (!mbar_wait_or_abort(&empty[s], ((it / kFnoStages) & 1) ^ 1, kFnoWaitNs, abort_flag)) {
           fail(11);
           break;
         }
-        uint8_t* st = sS + s * kStage;
+        uint8_t* st = sS + s * kFnoLayerStage;
         const int p0 = t * 128;
-        mbar_arrive_expect_tx(&full[s], kStage);
+        mbar_arrive_expect_tx(&full[s], kFnoLayerStage);
         tma_load_2d(st, &tmV, 0, p0, &full[s]);
-        if (MODE == 0) {
-          const int b = p0 / SS, rem = p0 - b * SS, y = rem / p.S, x0 = rem - y * p.S;
-          tma_load_2d(st + kTile, &tmTw, 0, x0, &full[s]);
-          tma_load_2d(st + 2 * kTile, &tmZ, 0, (b * p.S + y) * 64, &full[s]);
-        }
+        const int b = p0 / SS, rem = p0 - b * SS, y = rem / p.S, x0 = rem - y * p.S;
+        tma_load_2d(st + kTile, &tmTw, 0, x0, &full[s]);
+        tma_load_2d(st + kTile + 128 * 64, &tmZ, 0, (b * p.S + y) * 64, &full[s]);
       }
       // every load issued lands before the CTA may exit
       mbar_wait(w_full, 0, kFnoWaitNs);
@@ -138,7 +150,7 @@ __global__ void __launch_bounds__(192, 2)
       int it = 0;
       for (int t = blockIdx.x; t < p.tiles && ok && !*abort_flag; t += gridDim.x, ++it) {
         const int s = it % kFnoStages, buf = it & 1;
-        if (!mbar_wait(&tempty[buf], ((it >> 1) & 1) ^ 1, kFnoWaitNs)) {
+        if (!mbar_wait_or_abort(&tempty[buf], ((it >> 1) & 1) ^ 1, kFnoWaitNs, abort_flag)) {
           fail(13);
           break;
         }
@@ -148,16 +160,14 @@ __global__ void __launch_bounds__(192, 2)
         }
         tc_fence_after();
         const uint32_t d = tmem_base + buf * N;
-        uint8_t* st = sS + s * kStage;
+        uint8_t* st = sS + s * kFnoLayerStage;
         const uint64_t av = smem_desc_sw128(smem_u32(st));
         const uint64_t bw = smem_desc_sw128(smem_u32(sW));
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) tc_mma_bf16(d, av + 2 * ks, bw + 2 * ks, idesc, ks > 0 ? 1u : 0u);
-        if (MODE == 0) {
-          const uint64_t at = smem_desc_sw128(smem_u32(st + kTile));
-          const uint64_t bz = smem_desc_sw128(smem_u32(st + 2 * kTile));
-          for (int ks = 0; ks < p.kk_steps; ++ks) tc_mma_bf16(d, at + 2 * ks, bz + 2 * ks, idesc, 1u);
-        }
+        const uint64_t at = smem_desc_sw64(smem_u32(st + kTile));
+        const uint64_t bz = smem_desc_sw64(smem_u32(st + kTile + 128 * 64));
+        for (int ks = 0; ks < p.kk_steps; ++ks) tc_mma_bf16(d, at + 2 * ks, bz + 2 * ks, idesc, 1u);
         tc_commit(&empty[s]);
         tc_commit(&tfull[buf]);
       }
@@ -165,53 +175,214 @@ __global__ void __launch_bounds__(192, 2)
       mbar_wait(done, 0, kFnoWaitNs);
     }
   } else {
-    const int quad = warp & 3;
-    const int row = quad * 32 + lane;
+    const int quad = warp & 3, c0 = ((warp - 2) >> 2) * 32;
+    uint8_t* ov = sO + (warp - 2) * 2 * kFnoOutTile;
+    const uint32_t sw = static_cast<uint32_t>(lane >> 1) & 3u;  // 64B swizzle of row `lane`
     int it = 0;
     for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++it) {
       const int buf = it & 1;
-      const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (it >> 1) & 1, kFnoWaitNs));
+      const bool got =
+          __all_sync(0xffffffffu, mbar_wait_or_abort(&tfull[buf], (it >> 1) & 1, kFnoWaitNs, abort_flag));
+      if (!got) {
+        if (lane == 0) fail(15);
+        break;
+      }
+      tc_fence_after();
+      float v[32];
+      tmem_ld32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * N + c0, v);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&tempty[buf]);
+        // v_next alternates between the two buffers, or leaves the second to z
+        if (p.save_z)
+          bulk_wait_read<0>();
+        else
+          bulk_wait_read<1>();
+      }
+      __syncwarp();
+      uint8_t* dv = ov + (p.save_z || !(it & 1) ? 0 : kFnoOutTile) + lane * 64;
+      uint8_t* dz = ov + kFnoOutTile + lane * 64;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 ba = *reinterpret_cast<const float4*>(sb + c0 + 8 * q);
+        const float4 bb = *reinterpret_cast<const float4*>(sb + c0 + 8 * q + 4);
+        const float z[8] = {v[8 * q] + ba.x,     v[8 * q + 1] + ba.y, v[8 * q + 2] + ba.z, v[8 * q + 3] + ba.w,
+                            v[8 * q + 4] + bb.x, v[8 * q + 5] + bb.y, v[8 * q + 6] + bb.z, v[8 * q + 7] + bb.w};
+        uint32_t zw[4], vw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const __nv_bfloat162 zb = __floats2bfloat162_rn(z[2 * i], z[2 * i + 1]);
+          const __nv_bfloat162 vb = p.act ? gelu_bf16x2(z[2 * i], z[2 * i + 1]) : zb;
+          zw[i] = *reinterpret_cast<const uint32_t*>(&zb);
+          vw[i] = *reinterpret_cast<const uint32_t*>(&vb);
+        }
+        const uint32_t o = (static_cast<uint32_t>(q) ^ sw) << 4;
+        *reinterpret_cast<uint4*>(dv + o) = make_uint4(vw[0], vw[1], vw[2], vw[3]);
+        if (p.save_z) *reinterpret_cast<uint4*>(dz + o) = make_uint4(zw[0], zw[1], zw[2], zw[3]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmVn, dv, c0, t * 128 + quad * 32);
+        if (p.save_z) tma_store_2d(&tmZo, dz, c0, t * 128 + quad * 32);
+        bulk_commit();
+      }
+    }
+    // every TMA store must have finished before the CTA's shared memory goes
+    if (lane == 0 && it > 0) bulk_wait<0>();
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 0) tmem_dealloc(tmem_base, kTmemCols);
+}
+
+// Projection: eight epilogue warps, warps 2..5 the even tiles of the CTA and
+// 6..9 the odd ones (a pixel's sum over the 128 hidden units runs in one
+// thread, in order).  Bound by erff: 128 GELUs per pixel beside 132 bytes;
+// 16 x 512^2: 0.84 -> 0.57 ms with twice the epilogue warps and the biases
+// read four at a time.
+constexpr size_t kFnoProjSmem = 1024 + 128 * 128 + kFnoStages * kTile + 2 * 128 * 4 + 256;
+
+__global__ void __launch_bounds__(32 * (2 + kFnoEpiWarps), 2)
+    fno_tc_proj(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW, FnoTcParams p) {
+  constexpr int N = 128;
+  constexpr uint32_t kWBytes = N * 128;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+  uint8_t* sW = base;
+  uint8_t* sS = base + kWBytes;
+  float* sb = reinterpret_cast<float*>(sS + kFnoStages * kTile);  // b1[128], Q2[128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sb + 2 * N);
+  uint64_t* full = bars;
+  uint64_t* empty = bars + kFnoStages;
+  uint64_t* w_full = bars + 2 * kFnoStages;
+  uint64_t* tfull = bars + 2 * kFnoStages + 1;
+  uint64_t* tempty = bars + 2 * kFnoStages + 3;
+  uint64_t* done = bars + 2 * kFnoStages + 5;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kFnoStages + 6);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr uint32_t kTmemCols = 256;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kFnoStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(w_full, 1);
+    mbar_init(&tfull[0], 1);
+    mbar_init(&tfull[1], 1);
+    mbar_init(&tempty[0], 4);
+    mbar_init(&tempty[1], 4);
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (threadIdx.x < 128)
+    sb[threadIdx.x] = p.bias[threadIdx.x];
+  else if (threadIdx.x < 256)
+    sb[threadIdx.x] = p.q2[threadIdx.x - 128];
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  auto fail = [&](int code) {
+    *abort_flag = 1;
+    if (p.err) atomicExch(p.err, code);
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      prefetch_tmap(&tmV);
+      prefetch_tmap(&tmW);
+      mbar_arrive_expect_tx(w_full, kWBytes);
+      tma_load_2d(sW, &tmW, 0, 0, w_full);
+      int it = 0;
+      for (int t = blockIdx.x; t < p.tiles && !*abort_flag; t += gridDim.x, ++it) {
+        const int s = it % kFnoStages;
+        if (!mbar_wait_or_abort(&empty[s], ((it / kFnoStages) & 1) ^ 1, kFnoWaitNs, abort_flag)) {
+          fail(11);
+          break;
+        }
+        mbar_arrive_expect_tx(&full[s], kTile);
+        tma_load_2d(sS + s * kTile, &tmV, 0, t * 128, &full[s]);
+      }
+      // every load issued lands before the CTA may exit
+      mbar_wait(w_full, 0, kFnoWaitNs);
+      for (int q = (it > kFnoStages ? it - kFnoStages : 0); q < it; ++q)
+        mbar_wait(&full[q % kFnoStages], (q / kFnoStages) & 1, kFnoWaitNs);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(128, N);
+      bool ok = mbar_wait(w_full, 0, kFnoWaitNs);
+      if (!ok) fail(12);
+      tc_fence_after();
+      int it = 0;
+      for (int t = blockIdx.x; t < p.tiles && ok && !*abort_flag; t += gridDim.x, ++it) {
+        const int s = it % kFnoStages, buf = it & 1;
+        if (!mbar_wait_or_abort(&tempty[buf], ((it >> 1) & 1) ^ 1, kFnoWaitNs, abort_flag)) {
+          fail(13);
+          break;
+        }
+        if (!mbar_wait(&full[s], (it / kFnoStages) & 1, kFnoWaitNs)) {
+          fail(14);
+          break;
+        }
+        tc_fence_after();
+        const uint64_t av = smem_desc_sw128(smem_u32(sS + s * kTile));
+        const uint64_t bw = smem_desc_sw128(smem_u32(sW));
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          tc_mma_bf16(tmem_base + buf * N, av + 2 * ks, bw + 2 * ks, idesc, ks > 0 ? 1u : 0u);
+        tc_commit(&empty[s]);
+        tc_commit(&tfull[buf]);
+      }
+      tc_commit(done);
+      mbar_wait(done, 0, kFnoWaitNs);
+    }
+  } else {
+    const int quad = warp & 3, par = (warp - 2) >> 2;
+    const float b2 = __ldg(p.b2);
+    int it = 0;
+    for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++it) {
+      if ((it & 1) != par) continue;
+      const int buf = it & 1;
+      const bool got =
+          __all_sync(0xffffffffu, mbar_wait_or_abort(&tfull[buf], (it >> 1) & 1, kFnoWaitNs, abort_flag));
       if (!got) {
         if (lane == 0) fail(15);
         break;
       }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * N;
-      const size_t pix = static_cast<size_t>(t) * 128 + row;
-      if (MODE == 0) {
+      float acc = b2;
+#pragma unroll 1
+      for (int c0 = 0; c0 < N; c0 += 32) {
+        float v[32];
+        tmem_ld32(taddr + c0, v);
 #pragma unroll
-        for (int c0 = 0; c0 < N; c0 += 32) {
-          float v[32];
-          tmem_ld32(taddr + c0, v);
-          __align__(16) __nv_bfloat16 zb[32], vb[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float z = v[i] + __ldg(p.bias + c0 + i);
-            zb[i] = __float2bfloat16_rn(z);
-            vb[i] = __float2bfloat16_rn(p.act ? tc_gelu(z) : z);
-          }
-          uint4* zd = reinterpret_cast<uint4*>(p.zsave + pix * 64 + c0);
-          uint4* vd = reinterpret_cast<uint4*>(p.vnext + pix * 64 + c0);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            zd[q] = reinterpret_cast<const uint4*>(zb)[q];
-            vd[q] = reinterpret_cast<const uint4*>(vb)[q];
-          }
+        for (int i = 0; i < 32; i += 4) {
+          const float4 bj = *reinterpret_cast<const float4*>(sb + c0 + i);
+          const float4 qj = *reinterpret_cast<const float4*>(sb + N + c0 + i);
+          acc += qj.x * gelu_erf(v[i] + bj.x);
+          acc += qj.y * gelu_erf(v[i + 1] + bj.y);
+          acc += qj.z * gelu_erf(v[i + 2] + bj.z);
+          acc += qj.w * gelu_erf(v[i + 3] + bj.w);
         }
-      } else {
-        float acc = __ldg(p.b2);
-#pragma unroll
-        for (int c0 = 0; c0 < N; c0 += 32) {
-          float v[32];
-          tmem_ld32(taddr + c0, v);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc += __ldg(p.q2 + c0 + i) * tc_gelu(v[i] + __ldg(p.bias + c0 + i));
-        }
-        p.out[pix] = acc;
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[buf]);
+      p.out[static_cast<size_t>(t) * 128 + quad * 32 + lane] = acc;
     }
   }
   tc_fence_before();
@@ -748,11 +919,11 @@ __global__ void fno_to_bf16(const float* __restrict__ a, int n, __nv_bfloat16* _
     b[i] = __float2bfloat16_rn(a[i]);
 }
 
-// Tw[x][kk] (bf16): cos / sin of 2 pi kx x / S for kk = 2 kx / 2 kx + 1 < 2m,
-// zero beyond; from twx[kx][x] = (cos, -sin).
+// Tw[x][kk] (bf16, kk < 32): cos / sin of 2 pi kx x / S for kk = 2 kx / 2 kx + 1
+// < 2m, zero beyond; from twx[kx][x] = (cos, -sin).
 __global__ void fno_tw_table(const float2* __restrict__ twx, int S, int m, __nv_bfloat16* __restrict__ Tw) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < S * 64; t += gridDim.x * blockDim.x) {
-    const int kk = t & 63, x = t >> 6;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < S * 32; t += gridDim.x * blockDim.x) {
+    const int kk = t & 31, x = t >> 5;
     float v = 0.f;
     if (kk < 2 * m) {
       const float2 w = twx[static_cast<size_t>(kk >> 1) * S + x];
@@ -767,16 +938,12 @@ __global__ void fno_tw_table(const float2* __restrict__ twx, int S, int m, __nv_
 namespace huv_launch {
 bool tc_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows);
 
-size_t fno_tc_smem(int mode) {
-  const size_t w = (mode == 0 ? 64 : 128) * 128;
-  const size_t stage = mode == 0 ? 2 * huv_dev::kTile + 64 * 128 : huv_dev::kTile;
-  return 1024 + w + huv_dev::kFnoStages * stage + 256;
-}
+bool tc_map_sw64_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows, int cols);
 
 cudaError_t fno_tc_set_smem() {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(huv_dev::fno_tc_pw<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(fno_tc_smem(0)))))
+  if ((e = cudaFuncSetAttribute(huv_dev::fno_tc_layer, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(huv_dev::kFnoLayerSmem))))
     return e;
   if ((e = cudaFuncSetAttribute(huv_dev::fno_tc_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(huv_dev::kBwdSmem))))
@@ -784,32 +951,33 @@ cudaError_t fno_tc_set_smem() {
   if ((e = cudaFuncSetAttribute(huv_dev::fno_tc_proj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(huv_dev::kPbSmem))))
     return e;
-  return cudaFuncSetAttribute(huv_dev::fno_tc_pw<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(fno_tc_smem(1)));
+  return cudaFuncSetAttribute(huv_dev::fno_tc_proj, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(huv_dev::kFnoProjSmem));
 }
 
 // Layer l forward on tensor cores.  v: [B*S*S][64] bf16; Wb: [64][64] bf16;
-// Tw: [S][64] bf16; Zs: [B*S*64][64] bf16.
+// Tw: [S][32] bf16; Zs: [B*S*64][32] bf16; zsave may be null.
 bool fno_tc_layer(int B, int S, int m, const __nv_bfloat16* v, const __nv_bfloat16* Wb,
                   const __nv_bfloat16* Tw, const __nv_bfloat16* Zs, const float* bias, int act,
                   __nv_bfloat16* zsave, __nv_bfloat16* vnext, int* err, cudaStream_t st) {
-  CUtensorMap mv, mw, mt, mz;
+  CUtensorMap mv, mw, mt, mz, mvn, mzo;
   const uint64_t pix = static_cast<uint64_t>(B) * S * S;
   if (!tc_map_bf16(&mv, v, pix, 64, 128) || !tc_map_bf16(&mw, Wb, 64, 64, 64) ||
-      !tc_map_bf16(&mt, Tw, static_cast<uint64_t>(S), 64, 128) ||
-      !tc_map_bf16(&mz, Zs, static_cast<uint64_t>(B) * S * 64, 64, 64))
+      !tc_map_sw64_bf16(&mt, Tw, static_cast<uint64_t>(S), 32, 128, 32) ||
+      !tc_map_sw64_bf16(&mz, Zs, static_cast<uint64_t>(B) * S * 64, 32, 64, 32) ||
+      !tc_map_sw64_bf16(&mvn, vnext, pix, 64, 32, 64) || !tc_map_sw64_bf16(&mzo, zsave ? zsave : vnext, pix, 64, 32, 64))
     return false;
   huv_dev::FnoTcParams p{};
   p.tiles = static_cast<int>(pix / 128);
   p.S = S;
   p.kk_steps = (2 * m + 15) / 16;
   p.bias = bias;
-  p.zsave = zsave;
-  p.vnext = vnext;
   p.act = act;
+  p.save_z = zsave ? 1 : 0;
   p.err = err;
   const int grid = std::min(p.tiles, 2 * 148);
-  huv_dev::fno_tc_pw<0><<<grid, 192, fno_tc_smem(0), st>>>(mv, mw, mt, mz, p);
+  huv_dev::fno_tc_layer<<<grid, 32 * (2 + huv_dev::kFnoEpiWarps), huv_dev::kFnoLayerSmem, st>>>(mv, mw, mt, mz, mvn,
+                                                                                               mzo, p);
   return cudaGetLastError() == cudaSuccess;
 }
 
@@ -828,7 +996,7 @@ bool fno_tc_proj(int B, int S, const __nv_bfloat16* v, const __nv_bfloat16* Q1b,
   p.out = out;
   p.err = err;
   const int grid = std::min(p.tiles, 2 * 148);
-  huv_dev::fno_tc_pw<1><<<grid, 192, fno_tc_smem(1), st>>>(mv, mq, mq, mq, p);
+  huv_dev::fno_tc_proj<<<grid, 32 * (2 + huv_dev::kFnoEpiWarps), huv_dev::kFnoProjSmem, st>>>(mv, mq, p);
   return cudaGetLastError() == cudaSuccess;
 }
 // Layer backward on tensor cores (see fno_tc_layer_bwd); pix a multiple of 128.
@@ -885,6 +1053,6 @@ void fno_tc_to_bf16(const float* a, int n, __nv_bfloat16* b, cudaStream_t st) {
   huv_dev::fno_to_bf16<<<(n + 255) / 256, 256, 0, st>>>(a, n, b);
 }
 void fno_tc_tw_table(const float2* twx, int S, int m, __nv_bfloat16* Tw, cudaStream_t st) {
-  huv_dev::fno_tw_table<<<(S * 64 + 255) / 256, 256, 0, st>>>(twx, S, m, Tw);
+  huv_dev::fno_tw_table<<<(S * 32 + 255) / 256, 256, 0, st>>>(twx, S, m, Tw);
 }
 }  // namespace huv_launch

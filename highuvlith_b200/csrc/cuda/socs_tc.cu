@@ -968,10 +968,13 @@ bool tc_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int b
   return make_map(map, ptr, rows, kp, box_rows);
 }
 
-// FP16 map of 32-wide boxes (64B swizzle) and the f32 output map (32 x 32
+// FP16 and BF16 maps of 32-wide boxes (64B swizzle) and the f32 output map (32 x 32
 // boxes, 128B swizzle) for other files' kernels.
 bool tc_map_sw64_f16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows, int cols) {
   return make_map_sw64(map, ptr, rows, kp, box_rows, cols, true);
+}
+bool tc_map_sw64_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows, int cols) {
+  return make_map_sw64(map, ptr, rows, kp, box_rows, cols, false);
 }
 bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) { return make_out_map(map, ptr, rows, cols); }
 
