@@ -53,9 +53,11 @@ __host__ __device__ constexpr size_t fs_smem(int M, int B) {
   return sizeof(float2) * (static_cast<size_t>(fs_kb(M)) * M * M + static_cast<size_t>(fs_kb(M)) * M * B +
                            static_cast<size_t>(fs_kb(M) + 1) * B * B + M);
 }
-// Blocks per image: about three rounds of KB kernels each, at most a portable
-// cluster.  A function of K and M alone, so that an image does not depend on
-// the batch it is in.
+// Blocks per image: about three rounds of KB of the set's K kernels each, at
+// most a portable cluster.  A function of K and M alone, so that an image does
+// not depend on the batch it is in; real masks keep it for half the kernels,
+// so that the planes of a focus sweep, of which the one in focus folds, share
+// a launch.
 __host__ __device__ inline int fs_split(int M, int K) {
   const int rounds = (K + fs_kb(M) - 1) / fs_kb(M);
   const int s = (rounds + 2) / 3;
@@ -293,10 +295,10 @@ cudaError_t field_small(const huv::SmallPlane* p, int planes, const float2* Mban
                         const float2* tw, float* mean, void* out, cudaStream_t st) {
   const size_t img = static_cast<size_t>(clips) * 2 * M * M;
   for (int a = 0; a < planes;) {
-    const int split = huv_dev::fs_split(M, p[a].K);
+    const int split = p[a].split;
     huv_dev::SmallPlanes pl{};
     int c = 0;
-    for (; a + c < planes && c < huv_dev::kSmallPlanes && huv_dev::fs_split(M, p[a + c].K) == split; ++c) {
+    for (; a + c < planes && c < huv_dev::kSmallPlanes && p[a + c].split == split; ++c) {
       pl.kband[c] = p[a + c].kband;
       pl.W[c] = p[a + c].W;
       pl.K[c] = p[a + c].K;
@@ -353,9 +355,12 @@ void Engine::run_small_form(const huv_batch& b, DeviceSet* const* sets, const in
   void* IM = base + (per_x + per_m) * chunk;
   float* mean = reinterpret_cast<float*>(base + (per_x + per_m + per_i) * chunk);
   std::vector<SmallPlane> pl(planes);
-  for (int p = 0; p < planes; ++p)
-    pl[p] = SmallPlane{sets[p]->kband, W_use && W_use[p] ? W_use[p] : sets[p]->W, K_use && K_use[p] ? K_use[p] : sets[p]->K,
+  for (int p = 0; p < planes; ++p) {
+    const int K = K_use && K_use[p] ? K_use[p] : sets[p]->K;
+    const BandKernels bk = kernels_for(b, *sets[p], K);
+    pl[p] = SmallPlane{bk.kband, W_use && W_use[p] ? W_use[p] : sets[p]->W, bk.K, std::min(huv_dev::fs_split(M, K), bk.K),
                        sets[p]->keep, sets[p]->flare};
+  }
   int lgn = 0;
   while ((1 << lgn) < n) ++lgn;
   const float2* twn = twiddle_n(n);

@@ -1064,7 +1064,8 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
   static std::atomic<uint64_t> smem_set{0};
   once_per_device(smem_set, [] { check_cuda(tc_set_smem(), "cudaFuncSetAttribute(tc)"); });
   const int lgn = ilog2i(n), lgm = ilog2i(M);  // lgm: log2 of M rounded up (M need not be a power of two)
-  const int B = ds.B, K = K_use > 0 ? K_use : ds.K, hb = ds.hb;
+  const BandKernels bk = kernels_for(b, ds, K_use > 0 ? K_use : ds.K);
+  const int B = ds.B, K = bk.K, hb = ds.hb;
   const float* Wf = W_use ? W_use : ds.W;
   const int h2 = 2 * hb, B2 = 2 * h2 + 1;
   const int kcE = 2 * B, kpE = round_up(kcE, 64), kstE = (kcE + 15) / 16;
@@ -1191,13 +1192,13 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
         // one kernel per kernel group: rows and columns in shared memory; the
         // groups' partial sums (if any) in the operand buffer
         prof.begin("socs_field_fused", st);
-        check_cuda(socs_field_fused(ds.kband, Mb, K, hb, M, nc, ds.keep, ds.flare, mean, sep ? nullptr : IM,
+        check_cuda(socs_field_fused(bk.kband, Mb, K, hb, M, nc, ds.keep, ds.flare, mean, sep ? nullptr : IM,
                                     sep ? static_cast<void*>(IM) : nullptr, reinterpret_cast<float*>(BE), twm, st),
                    "socs_field_fused");
         prof.end(st);
       } else {
         prof.begin("socs_rows_inv", st);
-        check_cuda(socs_rows_x(ds.kband, 0.f, Mb, K, hb, M, nc, T, twm, st), "socs_rows");
+        check_cuda(socs_rows_x(bk.kband, 0.f, Mb, K, hb, M, nc, T, twm, st), "socs_rows");
         prof.end(st);
         prof.begin("socs_cols_inv", st);
         if (sep)  // I_M / s as FP16 split planes [clip][2][M][M] (the bytes of the f32 IM)
@@ -1211,13 +1212,13 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
     if (fft_field) {
     } else if (!gemm_rows) {
       // Row transforms as FP32 register-radix FFTs, emitting the split operand.
-      launch_rows(ds.kband, 0.f, Mb, K, hb, 0, B, M, kbE, 0, BE, twm, nc, st);
+      launch_rows(bk.kband, 0.f, Mb, K, hb, 0, B, M, kbE, 0, BE, twm, nc, st);
       check_cuda(cudaGetLastError(), "socs_rows_tc");
     } else {
       // Row transforms of every kernel's band product on tensor cores: the
       // same M-point inverse DFT operand (A_E) against the split products,
       // written straight as the next GEMM's split operand.
-      band_products<<<dim3(K, nc), 256, 0, st>>>(ds.kband, Mb, K, B, rbn, kpE, P);
+      band_products<<<dim3(K, nc), 256, 0, st>>>(bk.kband, Mb, K, B, rbn, kpE, P);
       check_cuda(cudaGetLastError(), "band_products");
       TcGemmParams p{};
       p.kboxes = kpE / 64;

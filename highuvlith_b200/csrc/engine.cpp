@@ -193,15 +193,8 @@ Engine::~Engine() {
     cudaSetDevice(device);
     for (auto& kv : twiddles) cudaFree(kv.second);
     for (auto& kv : row_digits) cudaFree(kv.second);
-    auto free_set = [](DeviceSet& d) {
-      for (auto& kv : d.W_by_k) cudaFree(kv.second);
-      cudaFree(d.kband);
-      cudaFree(d.W);
-      cudaFree(d.ptx);
-      huv_launch::tc_release_all(d.tc);
-    };
-    free_set(focus_dev);
-    for (auto& e : cache) free_set(e.dev);
+    focus_dev.release();
+    for (auto& e : cache) e.dev.release();
     prof.release();
     cudaFree(dev_err);
     cudaFree(ilt_cost_dev);
@@ -260,13 +253,7 @@ void Engine::cache_insert(double z, std::shared_ptr<KernelSet> ks) {
   if (static_cast<int>(cache.size()) >= settings.kernel_cache_capacity) {
     auto it = std::min_element(cache.begin(), cache.end(),
                                [](const CacheEntry& a, const CacheEntry& b) { return a.last_used < b.last_used; });
-    if (device_ready) {
-      for (auto& kv : it->dev.W_by_k) cudaFree(kv.second);
-      cudaFree(it->dev.kband);
-      cudaFree(it->dev.W);
-      cudaFree(it->dev.ptx);
-      huv_launch::tc_release_all(it->dev.tc);
-    }
+    if (device_ready) it->dev.release();
     cache.erase(it);
   }
   CacheEntry e;
@@ -412,14 +399,7 @@ DeviceSet& Engine::device_set(double z) {
     if (!slot) slot = &scratch_dev;
   }
   if (slot->kband && slot->source == ks.get()) return *slot;
-  if (slot->kband) {
-    for (auto& kv : slot->W_by_k) cudaFree(kv.second);
-    cudaFree(slot->kband);
-    cudaFree(slot->W);
-    cudaFree(slot->ptx);
-    huv_launch::tc_release_all(slot->tc);
-    *slot = DeviceSet();
-  }
+  if (slot->kband) slot->release();
   const int h = ks->band_half_width();
   const int B = 2 * h + 1;
   const int K = ks->num_kernels();
@@ -458,15 +438,50 @@ DeviceSet& Engine::device_set(double z) {
   d.flare = optics.flare > 0.0 ? static_cast<float>(optics.flare) : 0.f;
   d.eig_scaled.resize(K);
   for (int k = 0; k < K; ++k) d.eig_scaled[k] = ks->eigenvalues[k] / div;
-  d.host_kband = kb;
-  check_cuda(cudaMalloc(&d.kband, sizeof(float2) * kb.size()), "cudaMalloc(kband)");
+  d.host_kband = std::move(kb);
+  check_cuda(cudaMalloc(&d.kband, sizeof(float2) * d.host_kband.size()), "cudaMalloc(kband)");
   check_cuda(cudaMalloc(&d.W, sizeof(float) * wf.size()), "cudaMalloc(W)");
   check_cuda(cudaMalloc(&d.ptx, sizeof(float) * ptx.size()), "cudaMalloc(ptx)");
-  check_cuda(cudaMemcpy(d.kband, kb.data(), sizeof(float2) * kb.size(), cudaMemcpyHostToDevice), "upload kband");
+  check_cuda(cudaMemcpy(d.kband, d.host_kband.data(), sizeof(float2) * d.host_kband.size(), cudaMemcpyHostToDevice), "upload kband");
   check_cuda(cudaMemcpy(d.W, wf.data(), sizeof(float) * wf.size(), cudaMemcpyHostToDevice), "upload W");
   check_cuda(cudaMemcpy(d.ptx, ptx.data(), sizeof(float) * ptx.size(), cudaMemcpyHostToDevice), "upload ptx");
   *slot = std::move(d);
   return *slot;
+}
+
+void DeviceSet::release() {
+  for (auto& kv : W_by_k) cudaFree(kv.second);
+  for (auto& kv : folded) cudaFree(kv.second.kband);
+  cudaFree(kband);
+  cudaFree(W);
+  cudaFree(ptx);
+  huv_launch::tc_release_all(tc);
+  *this = DeviceSet();
+}
+
+Engine::BandKernels Engine::kernels_for(const huv_batch& b, DeviceSet& ds, int K) {
+  const bool real = b.input_kind == HUV_INPUT_RASTER_U8 || b.input_kind == HUV_INPUT_RASTER_F32 ||
+                    (b.input_kind == HUV_INPUT_RECTS && rect.dv.y == 0.0 && rect.bg.y == 0.0);
+  if (!real) return {ds.kband, K};
+  auto it = ds.folded.find(K);
+  if (it == ds.folded.end()) {
+    DeviceSet::Folded f;
+    FoldedKernels p;
+    double div = ds.source->divisor(settings.normalization);
+    if (div == 0.0) div = 1.0;
+    if (fold_real_kernels(*ds.source, K, div, p)) {
+      std::unique_ptr<float[]> h(new float[2 * p.size]);
+      parallel_for(static_cast<int64_t>(2 * p.size), [&](int64_t lo, int64_t hi) {
+        for (int64_t i = lo; i < hi; ++i) h[i] = static_cast<float>(p.v[i]);
+      });
+      check_cuda(cudaMalloc(&f.kband, sizeof(float2) * p.size), "cudaMalloc(folded kernels)");
+      f.K = (K + 1) / 2;
+      check_cuda(cudaMemcpy(f.kband, h.get(), sizeof(float2) * p.size, cudaMemcpyHostToDevice),
+                 "upload folded kernels");
+    }
+    it = ds.folded.emplace(K, f).first;
+  }
+  return it->second.kband ? BandKernels{it->second.kband, it->second.K} : BandKernels{ds.kband, K};
 }
 
 const float* Engine::flare_weights(DeviceSet& ds, int K) {
@@ -552,10 +567,11 @@ bool Engine::field_fused(const DeviceSet& ds, int M) const {
   return env && std::string(env) == "fused" && huv_launch::field_fused_ok(M, ds.hb);
 }
 
-void Engine::run_fft_form(const huv_batch& b, const DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use,
+void Engine::run_fft_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use,
                           const float* W_use) {
   const int lgn = ilog2(n), lgm = ilog2(M);  // lgm: rounded up where M is 160, 192 or 384
-  const int B = ds.B, K = K_use > 0 ? K_use : ds.K, hb = ds.hb;
+  const BandKernels bk = kernels_for(b, ds, K_use > 0 ? K_use : ds.K);
+  const int B = ds.B, K = bk.K, hb = ds.hb;
   const float* Wf = W_use ? W_use : ds.W;
   const bool coarse = M < n;
   const int h2 = 2 * hb, B2 = 2 * h2 + 1;
@@ -606,14 +622,14 @@ void Engine::run_fft_form(const huv_batch& b, const DeviceSet& ds, int M, float*
     if (fused) {
       // the partial sums of the kernel groups reuse T's bytes (K B M complex per clip)
       prof.begin("socs_field_fused", st);
-      check_cuda(huv_launch::socs_field_fused(ds.kband, Mb, K, hb, M, nc, ds.keep, ds.flare, mean, coarse ? IM : o,
+      check_cuda(huv_launch::socs_field_fused(bk.kband, Mb, K, hb, M, nc, ds.keep, ds.flare, mean, coarse ? IM : o,
                                               nullptr, reinterpret_cast<float*>(T), twm, st),
                  "socs_field_fused");
       prof.end(st);
       prof.launches += huv_launch::field_fused_part_bytes(M, K) ? 2 : 1;
     } else {
       prof.begin("socs_rows_inv", st);
-      check_cuda(huv_launch::socs_rows_x(ds.kband, 0.f, Mb, K, hb, M, nc, T, twm, st), "socs_rows");
+      check_cuda(huv_launch::socs_rows_x(bk.kband, 0.f, Mb, K, hb, M, nc, T, twm, st), "socs_rows");
       prof.end(st);
       prof.begin("socs_cols_inv", st);
       check_cuda(huv_launch::socs_cols_x(T, K, hb, M, nc, ds.keep, ds.flare, mean, coarse ? IM : o, 0, twm, st),

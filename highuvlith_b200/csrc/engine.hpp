@@ -102,6 +102,13 @@ struct DeviceSet {
   float* ptx = nullptr;
   std::vector<double> eig_scaled;
   std::map<int, float*> W_by_k;  // flare weights of kernel-count prefixes
+  // kernels of real masks by kernel-count prefix (Engine::kernels_for)
+  struct Folded {
+    float2* kband = nullptr;  // null: the prefix has no folded form
+    int K = 0;
+  };
+  std::map<int, Folded> folded;
+  void release();  // frees every device buffer
   std::vector<float2> host_kband;
   std::map<int, TcState> tc;  // per evaluation grid (log2 M); kept for the set's lifetime
 };
@@ -184,6 +191,7 @@ struct SmallPlane {
   const float2* kband;
   const float* W;
   int K;
+  int split;  // blocks per image, at most K
   float keep, flare;
 };
 
@@ -258,7 +266,7 @@ struct Engine {
   bool hybrid_supported(const DeviceSet& ds, int M) const;
   bool tc_supported(const DeviceSet& ds, int M) const;
   // K_use / W_use: kernel count and flare weights to use (0 / nullptr = the whole set).
-  void run_fft_form(const huv_batch& b, const DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use = 0,
+  void run_fft_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use = 0,
                     const float* W_use = nullptr);
   void run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use = 0,
                    const float* W_use = nullptr, int core = kTcCoreFftRows);
@@ -284,6 +292,14 @@ struct Engine {
   void interp_matrix(DeviceSet& ds, int M);
   void interp_separable(DeviceSet& ds, int M, int nc, const void* im_split, const float* mean, void* BI, float* out,
                         cudaStream_t st, bool profile);
+  // The band kernels to image the batch's input kind with: the first K of the
+  // set, or, for real masks, their folded form (half as many) where the set
+  // has one.  Built on first use, kept with the set.
+  struct BandKernels {
+    const float2* kband;
+    int K;
+  };
+  BandKernels kernels_for(const huv_batch& b, DeviceSet& ds, int K);
   // Flare weights W = sum_{k < K} lambda_k |u_k|^2 / N^4 of the first K kernels (device, cached).
   const float* flare_weights(DeviceSet& ds, int K);
   // Kernel count for a budget of `max_kernels` under the reference's truncation rule.

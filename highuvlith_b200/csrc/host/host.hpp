@@ -6,6 +6,7 @@
 #include <complex>
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -71,6 +72,16 @@ struct KernelSet {
   int band_half_width() const;     // max |order| over the support
   double divisor(int normalization) const;  // 0 if images stay absolute
 };
+
+// The first K kernels as ceil(K / 2) band kernels [B][B] (scaled by
+// sqrt(lambda / div) / n^2) with the same images of real masks: fold.cpp.
+// False where the set has no such form.
+struct FoldedKernels {
+  std::unique_ptr<double[]> v;  // (re, im) pairs, written in parallel (never zeroed first)
+  size_t size = 0;              // complex values
+  cd operator[](size_t i) const { return cd(v[2 * i], v[2 * i + 1]); }
+};
+bool fold_real_kernels(const KernelSet& ks, int K, double div, FoldedKernels& folded);
 
 int select_kernel_count(const std::vector<double>& values, double trace, int max_kernels,
                         double fraction);
