@@ -461,8 +461,11 @@ class SimulationEngine:
     def _rect_clips(clips, feature, background):
         """ctypes view of rectangle clips (centre x, y and size w, h in nm,
         field-centred coordinates); keeps the arrays alive on the view."""
-        flat = [tuple(map(float, r)) for c in clips for r in c]
-        rects = np.ascontiguousarray(np.asarray(flat, dtype=np.float64).reshape(-1, 4))
+        try:
+            rects = np.concatenate([np.asarray(c, dtype=np.float64).reshape(len(c), 4) for c in clips] or [np.zeros((0, 4))])
+        except (TypeError, ValueError):  # rectangles of other number types
+            flat = [tuple(map(float, r)) for c in clips for r in c]
+            rects = np.ascontiguousarray(np.asarray(flat, dtype=np.float64).reshape(-1, 4))
         offs = np.zeros(len(clips) + 1, dtype=np.int32)
         offs[1:] = np.cumsum([len(c) for c in clips])
         f, bgd = complex(feature), complex(background)

@@ -325,7 +325,7 @@ bool Engine::sweep_small(const huv_batch& b, const double* z, int planes, float*
     if (!m || (p > 0 && (m != M || sets[p]->hb != sets[0]->hb))) return false;
     M = m;
   }
-  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b);
+  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, st);
   run_small_form(b, sets.data(), nullptr, nullptr, planes, M, out, st);
   return true;
 }
@@ -680,7 +680,7 @@ void Engine::image_batch(const huv_batch& b, float* out, cudaStream_t st) {
   check_batch(b, out);
   if (b.n_clips == 0) return;
   ensure_device();
-  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b);
+  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, st);
   DeviceSet& ds = device_set(b.defocus_nm == 0.0 ? 0.0 : b.defocus_nm);
   int form = b.form;
   // FFT and hybrid forms evaluate on the smallest supported grid above 4h

@@ -220,7 +220,7 @@ struct Engine {
   void image_batch_host(const huv_batch& b, float* out_host, cudaStream_t st);
   // Rectangle clips (HUV_INPUT_RECTS): the batch's row/run table on the
   // device, then the exact band spectrum of clips [c0, c0 + nc).
-  void upload_rects(const huv_batch& b);
+  void upload_rects(const huv_batch& b, cudaStream_t st);
   void rect_band(int c0, int nc, int hb, const float* W, float2* Mband, float* mean, cudaStream_t st);
   // Kernel sets of the focus planes not cached yet, built concurrently (one
   // plane per host thread) and cached.
@@ -357,6 +357,11 @@ struct Engine {
     void *clip_rows = nullptr, *rows = nullptr, *runs = nullptr, *coef = nullptr;
     size_t clip_rows_cap = 0, rows_cap = 0, runs_cap = 0, coef_cap = 0;
     int n_rows = 0;
+    // resolved on the device: rows holds the rectangles and, after them, the
+    // clips' offsets; most = rectangles of the largest clip
+    bool on_device = false;
+    std::vector<uint8_t> stage;
+    int most = 0, total = 0, clips = 0;
     double2 dv{0, 0}, bg{0, 0};
   } rect;
   cudaStream_t io_h2d = nullptr, io_d2h = nullptr;
