@@ -253,6 +253,253 @@ __global__ void __launch_bounds__(fs_threads(M))
   cl.sync();  // no block leaves while another reads its partial sums
 }
 
+// Adjoint of the field pass on the same grids: Q = sum_k conj(kappa_k) .
+// band(FFT(G0 . E_k)), G0 = keep G + flare_over_n sums[mask][1].  The fields
+// E_k are made again from the mask band (as socs_field_small makes them),
+// multiplied by G0 at each thread's own points, transformed back along y and x
+// within the band, and conj(kappa_k) times the result is summed in registers
+// over the block's kernels, then over the cluster in order.  Nothing but Q is
+// written: the two radix-4 kernels it replaces kept every field's transform in
+// memory and ran all kernels of a strip in one block (3 masks of 256^2, M =
+// 64, 20 kernels: 69 -> 13 us).
+// grid: (split, masks), clusters of split.
+template <int M>
+__global__ void __launch_bounds__(fs_threads(M))
+    ilt_adj_small(const float2* __restrict__ kband, const float2* __restrict__ Mband, const float* __restrict__ G, int K,
+                  int hb, float keep, const double* __restrict__ sums, float flare_over_n,
+                  const float2* __restrict__ tw, float2* __restrict__ Q) {
+  constexpr int R = M / 16, KB = fs_kb(M), T = fs_work(M), NT = fs_threads(M);
+  constexpr int SR = KB * M / 2, SC = KB * M;
+  constexpr int NR = R > 1 ? (16 * SR + T - 1) / T : 1;
+  constexpr int NC = R > 1 ? (16 * SC + T - 1) / T : 1;
+  constexpr int RO = R > 1 ? R : 16;  // outputs of one butterfly of the last pass
+  extern __shared__ float2 smem[];
+  const int t = threadIdx.x, B = 2 * hb + 1, BB = B * B;
+  const int ks = blockIdx.x, nsplit = gridDim.x, mask = blockIdx.y;
+  float2* buf = smem;               // [M][SC], rows [M][SR]
+  float2* rows = buf + KB * M * M;  // [SC][B]
+  float2* sM = rows + KB * M * B;   // [B][B]
+  float2* sU = sM + BB;             // [2][KB][B][B]
+  float2* sw = sU + 2 * KB * BB;    // [M] exp(+2 pi i t / M)
+  const int k0 = K * ks / nsplit, k1 = K * (ks + 1) / nsplit;
+  auto fetch = [&](int k) {
+    const int n = min(KB, k1 - k) * BB;
+    const float2* src = kband + static_cast<size_t>(k) * BB;
+    float2* dst = sU + (((k - k0) / KB) & 1) * KB * BB;
+    for (int e = t; e < n; e += NT) fr_cp_async8(dst + e, src + e);
+    fr_cp_commit();
+  };
+  fetch(k0);
+  for (int e = t; e < BB; e += NT) sM[e] = Mband[static_cast<size_t>(mask) * BB + e];
+  for (int e = t; e < M; e += NT) {
+    const float2 w = tw[e];
+    sw[e] = make_float2(w.x, -w.y);
+  }
+  // G0 at the thread's points of the last inverse pass
+  const float add = flare_over_n * static_cast<float>(sums[mask * 2 + 1]);
+  const float* Gm = G + static_cast<size_t>(mask) * M * M;
+  float g[NC][RO];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int u = R > 1 ? t + c * T : t;
+    const int x = (u % SC) % M, j = R > 1 ? (u / SC) % 16 : 0;  // guarded butterflies read a valid point
+#pragma unroll
+    for (int p = 0; p < RO; ++p) g[c][p] = keep * Gm[(R > 1 ? j + p * 16 : p) * M + x] + add;
+  }
+  float2 acc[NR][RO];
+#pragma unroll
+  for (int c = 0; c < NR; ++c)
+#pragma unroll
+    for (int p = 0; p < RO; ++p) acc[c][p] = make_float2(0.f, 0.f);
+  auto band = [&](int i) { return i <= hb ? i + hb : (i >= M - hb ? i - M + hb : -1); };
+
+  for (int k = k0; k < k1; k += KB) {
+    const float2* U = sU + (((k - k0) / KB) & 1) * KB * BB;
+    fr_cp_wait<0>();
+    __syncthreads();
+    if (k + KB < k1) fetch(k + KB);  // the other buffer: its last readers passed the barrier above
+    // ---- fields, as in socs_field_small
+    if (t < T / 2) {
+      const int s = t % SR, j = t / SR, kk = s / (M / 2), my = s % (M / 2);
+      float2 v[16];
+      if (my < B && k + kk < k1) {
+        const float2 *u = U + kk * BB + my * B, *m = sM + my * B;
+        fs_band16<R>(j, hb, v, [&](int q) { return fr_mul(u[q], m[q]); });
+      } else {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = make_float2(0.f, 0.f);
+      }
+      if constexpr (R > 1) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) buf[(j * 16 + r) * SR + s] = v[r];
+      } else if (my < B) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) rows[(kk * M + r) * B + my] = v[r];
+      }
+    }
+    __syncthreads();
+    if constexpr (R > 1) {
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        const int u = t + c * T;
+        if (t >= T || u >= 16 * SR) break;
+        const int s = u % SR, j = u / SR, kk = s / (M / 2), my = s % (M / 2);
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = buf[(j + r * 16) * SR + s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = fr_mul(v[r], sw[r * j]);
+        fr_dft<R, +1>(v);
+        if (my < B)
+#pragma unroll
+          for (int p = 0; p < R; ++p) rows[(kk * M + j + p * 16) * B + my] = v[p];
+      }
+      __syncthreads();
+    }
+    float2 f[16];  // a column butterfly
+    if (t < T) {
+      const int s = t % SC, j = t / SC;
+      const float2* col = rows + s * B;
+      fs_band16<R>(j, hb, f, [&](int q) { return col[q]; });
+      if constexpr (R > 1) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) buf[(j * 16 + r) * SC + s] = f[r];
+      } else {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) f[r] = make_float2(f[r].x * g[0][r], f[r].y * g[0][r]);
+      }
+    }
+    __syncthreads();
+    // ---- times G0 (in place: a butterfly reads and writes the points j + 16 r), and back along y
+    if constexpr (R > 1) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int u = t + c * T;
+        if (t >= T || u >= 16 * SC) break;
+        const int s = u % SC, j = u / SC;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = buf[(j + r * 16) * SC + s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = fr_mul(v[r], sw[r * j]);
+        fr_dft<R, +1>(v);
+#pragma unroll
+        for (int p = 0; p < R; ++p) buf[(j + p * 16) * SC + s] = make_float2(v[p].x * g[c][p], v[p].y * g[c][p]);
+      }
+      __syncthreads();
+      if (t < T) {
+        const int s = t % SC, j = t / SC;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) f[r] = buf[(j + r * R) * SC + s];
+      }
+      __syncthreads();
+    }
+    if (t < T) {
+      const int s = t % SC, j = t / SC;
+      fr_dft<16, -1>(f);
+      if constexpr (R > 1) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) buf[(j * 16 + r) * SC + s] = f[r];
+      } else {
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+          if (band(r) >= 0) rows[s * B + band(r)] = f[r];
+      }
+    }
+    __syncthreads();
+    if constexpr (R > 1) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int u = t + c * T;
+        if (t >= T || u >= 16 * SC) break;
+        const int s = u % SC, j = u / SC;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = buf[(j + r * 16) * SC + s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = fr_mul(v[r], make_float2(sw[r * j].x, -sw[r * j].y));
+        fr_dft<R, -1>(v);
+#pragma unroll
+        for (int p = 0; p < R; ++p) {
+          const int m = band(j + p * 16);
+          if (m >= 0) rows[s * B + m] = v[p];
+        }
+      }
+      __syncthreads();
+    }
+    // ---- back along x, times conj(kappa)
+    if (t < T / 2) {
+      const int s = t % SR, j = t / SR, kk = s / (M / 2), my = s % (M / 2);
+      float2 v[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = my < B ? rows[(kk * M + j + r * R) * B + my] : make_float2(0.f, 0.f);
+      fr_dft<16, -1>(v);
+      if constexpr (R > 1) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) buf[(j * 16 + r) * SR + s] = v[r];
+      } else if (my < B && k + kk < k1) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+          if (band(r) >= 0) {
+            const float2 u = U[kk * BB + my * B + band(r)];
+            acc[0][r].x += u.x * v[r].x + u.y * v[r].y;
+            acc[0][r].y += u.x * v[r].y - u.y * v[r].x;
+          }
+      }
+    }
+    if constexpr (R > 1) {
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        const int u = t + c * T;
+        if (t >= T || u >= 16 * SR) break;
+        const int s = u % SR, j = u / SR, kk = s / (M / 2), my = s % (M / 2);
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = buf[(j + r * 16) * SR + s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = fr_mul(v[r], make_float2(sw[r * j].x, -sw[r * j].y));
+        fr_dft<R, -1>(v);
+        if (my < B && k + kk < k1)
+#pragma unroll
+          for (int p = 0; p < R; ++p) {
+            const int m = band(j + p * 16);
+            if (m >= 0) {
+              const float2 q = U[kk * BB + my * B + m];
+              acc[c][p].x += q.x * v[p].x + q.y * v[p].y;
+              acc[c][p].y += q.x * v[p].y - q.y * v[p].x;
+            }
+          }
+      }
+    }
+  }
+  // partial sums [kk][my][mx] over buf, then the cluster's in order
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < NR; ++c) {
+    const int u = R > 1 ? t + c * T : t;
+    if (R > 1 ? (t >= T || u >= 16 * SR) : t >= T / 2) break;
+    const int s = u % SR, j = u / SR, kk = s / (M / 2), my = s % (M / 2);
+    if (my < B)
+#pragma unroll
+      for (int p = 0; p < RO; ++p) {
+        const int m = band(R > 1 ? j + p * 16 : p);
+        if (m >= 0) buf[kk * BB + my * B + m] = acc[c][p];
+      }
+  }
+  cgx::cluster_group cl = cgx::this_cluster();
+  cl.sync();
+  for (int e = ks * NT + t; e < BB; e += nsplit * NT) {
+    float2 s = make_float2(0.f, 0.f);
+    for (int q = 0; q < nsplit; ++q) {
+      const float2* src = cl.map_shared_rank(buf, q) + e;
+      for (int kk = 0; kk < KB; ++kk) s = fr_add(s, src[kk * BB]);
+    }
+    Q[static_cast<size_t>(mask) * BB + e] = s;
+  }
+  cl.sync();  // no block leaves while another reads its partial sums
+}
+
 }  // namespace huv_dev
 
 namespace huv_launch {
@@ -286,7 +533,44 @@ cudaError_t launch_small(const huv_dev::SmallPlanes& pl, int planes, int split, 
   return cudaLaunchKernelEx(&cfg, huv_dev::socs_field_small<M>, pl, Mband, hb, clips, tw, mean,
                             static_cast<__half*>(out));
 }
+template <int M>
+cudaError_t launch_adj(const float2* kband, const float2* Mband, const float* G, int K, int hb, float keep,
+                       const double* sums, float flare_over_n, int masks, const float2* tw, float2* Q, cudaStream_t st) {
+  static std::atomic<uint64_t> attr{0};
+  auto smem = [](int B) { return huv_dev::fs_smem(M, B) + sizeof(float2) * huv_dev::fs_kb(M) * B * B; };
+  huv::once_per_device(attr, [&] {
+    huv::check_cuda(cudaFuncSetAttribute(huv_dev::ilt_adj_small<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem(M / 2))),
+                    "cudaFuncSetAttribute(ilt_adj_small)");
+  });
+  const int split = std::min(huv_dev::fs_split(M, K), K);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(split, masks);
+  cfg.blockDim = dim3(huv_dev::fs_threads(M));
+  cfg.dynamicSmemBytes = smem(2 * hb + 1);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = split;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, huv_dev::ilt_adj_small<M>, kband, Mband, G, K, hb, keep, sums, flare_over_n, tw, Q);
+}
 }  // namespace
+
+// Q of every mask on the power-of-two grids that the ILT uses below 128.
+bool ilt_adj_small_ok(int M, int hb) { return (M == 16 || M == 32 || M == 64) && field_small_ok(M, hb); }
+cudaError_t ilt_adj_small(const float2* kband, const float2* Mband, const float* G, int M, int K, int hb, float keep,
+                          const double* sums, float flare_over_n, int masks, const float2* tw, float2* Q,
+                          cudaStream_t st) {
+  switch (M) {
+    case 16: return launch_adj<16>(kband, Mband, G, K, hb, keep, sums, flare_over_n, masks, tw, Q, st);
+    case 32: return launch_adj<32>(kband, Mband, G, K, hb, keep, sums, flare_over_n, masks, tw, Q, st);
+    case 64: return launch_adj<64>(kband, Mband, G, K, hb, keep, sums, flare_over_n, masks, tw, Q, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 // I_M / interp_scale(mean) of every plane and clip as FP16 planes
 // [plane][clip][2][M][M], and the flare means [plane][clip].  The planes' sets

@@ -738,6 +738,12 @@ cudaError_t socs_cols_split(const float2* T, int K, int hb, int L, int clips, fl
 
 bool xt_ok(int L, int hb);
 bool interp_fused_ok(int M, int n);
+cudaError_t socs_cols_few(const float2* T, int K, int hb, int lgm, int clips, float keep, float flare,
+                          const float* mean, float2* E, float* out, const float2* tw, cudaStream_t st);
+bool ilt_adj_small_ok(int M, int hb);
+cudaError_t ilt_adj_small(const float2* kband, const float2* Mband, const float* G, int M, int K, int hb, float keep,
+                          const double* sums, float flare_over_n, int masks, const float2* tw, float2* Q,
+                          cudaStream_t st);
 
 cudaError_t ilt_set_smem() {
   const int big = 200 * 1024;
@@ -841,6 +847,9 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   const size_t s_V = grad ? a256(sizeof(float2) * static_cast<size_t>(K) * B * M) : 0;
   const size_t s_q = grad ? a256(sizeof(float2) * B * B) : 0;
   const size_t s_t2 = grad ? a256(sizeof(float2) * static_cast<size_t>(B) * n) : 0;
+  // few masks of a narrow band: the fields kept one by one (socs_cols_few)
+  const bool few = !xt_fwd && coarse && M <= 64 && masks * (M / 8) < 148;
+  const size_t s_ef = few ? a256(sizeof(float2) * static_cast<size_t>(K) * mpix) : 0;
   const size_t s_parts = a256(sizeof(double) * kRedBlocks * 2);
   // 64 x 64 regulariser tiles where the grid allows (fewer, longer blocks),
   // else 32 x 32, else the untiled kernel
@@ -849,7 +858,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   const int reg_parts = tiled ? (n / tile) * (n / tile) : kRedBlocks;
   const size_t s_preg = a256(sizeof(double) * std::max(reg_parts, 2 * kRedBlocks));
   const size_t per = s_t + s_x + s_m + s_mean + s_T + s_im + s_c + s_x2 + s_img + s_V + s_q + s_t2 + 2 * s_parts +
-                     s_preg + s_bi + a256(sizeof(double) * 4);
+                     s_preg + s_bi + s_ef + a256(sizeof(double) * 4);
   const size_t budget = chunk_budget();
   const int chunk = balanced_chunk(static_cast<int>(std::max<size_t>(1, budget / per)), masks);
   char* base = static_cast<char*>(workspace(per * chunk + 4096));
@@ -875,6 +884,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   double* preg = reinterpret_cast<double*>(take(s_preg));
   double* sums = reinterpret_cast<double*>(take(s_parts));
   double* regsum = reinterpret_cast<double*>(take(a256(sizeof(double) * 4)));
+  float2* Ef = reinterpret_cast<float2*>(take(s_ef));
   void* BI = sep ? static_cast<void*>(take(s_bi)) : nullptr;
   huv_batch real_kind{};
   real_kind.input_kind = HUV_INPUT_RASTER_F32;
@@ -903,7 +913,10 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       check_cuda(socs_cols_x(T, K, hb, M, nc, keep, flare, mean, coarse ? IM : img, 0, twm, st), "ilt socs_cols");
     } else {
       check_cuda(socs_rows(ds.kband, 0.f, Mb, K, hb, lgm, nc, T, twm, st), "ilt socs_rows");
-      check_cuda(socs_cols(T, K, hb, lgm, nc, keep, flare, mean, coarse ? IM : img, 0, twm, st), "ilt socs_cols");
+      if (few)
+        check_cuda(socs_cols_few(T, K, hb, lgm, nc, keep, flare, mean, Ef, IM, twm, st), "ilt socs_cols");
+      else
+        check_cuda(socs_cols(T, K, hb, lgm, nc, keep, flare, mean, coarse ? IM : img, 0, twm, st), "ilt socs_cols");
     }
     if (coarse && !sep) {
       check_cuda(band_forward(IM, HUV_INPUT_RASTER_F32, M, lgm, h2, nc, X2, C, nullptr, nullptr, nullptr, twm, st, nullptr,
@@ -935,7 +948,8 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       // The adjoint's kernels: t is real, so the folded set (half as many
       // transforms, Engine::kernels_for) gives the same gradient; its row
       // transforms replace the forward's, which the image has consumed.
-      const BandKernels ak = xt ? kernels_for(real_kind, ds, K) : BandKernels{ds.kband, K};
+      const bool adj_small = !xt && ilt_adj_small_ok(M, hb);
+      const BandKernels ak = xt || adj_small ? kernels_for(real_kind, ds, K) : BandKernels{ds.kband, K};
       if (xt && ak.K < K)
         check_cuda(socs_rows_x(ak.kband, 0.f, Mb, ak.K, hb, M, nc, T, twm, st), "ilt adjoint rows");
       if (xt) {
@@ -957,6 +971,9 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
           default: throw Error(HUV_ERR_UNSUPPORTED, "ILT adjoint: no register-radix instance for this grid");
         }
 #undef HUV_ILT_ADJ
+      } else if (adj_small) {
+        check_cuda(ilt_adj_small(ak.kband, Mb, Gm, M, ak.K, hb, keep, sums, flare / static_cast<float>(npix), nc, twm, Q, st),
+                   "ilt adjoint");
       } else {
         const int Wc = fit_units(8, 2 * (sizeof(float2) << lgm) + (sizeof(float) << lgm));
         const size_t sm = 2 * (static_cast<size_t>(Wc) << lgm) * sizeof(float2) +
