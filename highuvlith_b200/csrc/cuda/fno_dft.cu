@@ -62,7 +62,7 @@ __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
 // cp.async, two stages; a stage is a chunk of BF16 or half of one of FP32
 // (the same bytes).  16 x 512^2 BF16: 1.21 -> 0.46 ms (0.57 with single
 // multiply-adds); 8 x 512^2 FP32: 0.617 -> 0.26 ms.
-constexpr int kDxRows = 4;
+constexpr int kDxRows = 2, kDxThreads = 128 * kDxRows;
 template <typename T>
 __host__ __device__ constexpr int dx_split() { return sizeof(T) == 4 ? 2 : 1; }  // stages per chunk
 template <typename T>
@@ -71,7 +71,7 @@ __host__ __device__ constexpr size_t dx_stage_bytes() {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(512, 1) fno_dft_x(const T* __restrict__ in, int S, int m,
+__global__ void __launch_bounds__(kDxThreads, 2) fno_dft_x(const T* __restrict__ in, int S, int m,
                                                      const float2* __restrict__ twt, float2* __restrict__ out,
                                                      int rows) {
   constexpr int C = 64;
@@ -101,12 +101,12 @@ __global__ void __launch_bounds__(512, 1) fno_dft_x(const T* __restrict__ in, in
     constexpr int lkVec = kVec == 8 ? 3 : 4;
     const T* src = in + (static_cast<size_t>(r0) * S + x0) * C;
     const int nvec = (kDxRows * kVec) << (lhs + 2);
-    for (int e = t; e < nvec; e += 512) {
+    for (int e = t; e < nvec; e += kDxThreads) {
       const int v = e & (kVec - 1), xx = (e >> lkVec) & (sx - 1), row = e >> (lkVec + lhs + 2);
       const int x = (xx >> lhs) * xs + (xx & (hs - 1));
       cp16(dst + static_cast<size_t>(e) * 16, src + (static_cast<size_t>(row) * S + x) * C + v * kPer16);
     }
-    for (int e = t; e < sx * 8; e += 512) {
+    for (int e = t; e < sx * 8; e += kDxThreads) {
       const int v = e & 7, xx = e >> 3;
       const int x = x0 + (xx >> lhs) * xs + (xx & (hs - 1));
       cp16(dst + dbytes + static_cast<size_t>(e) * 16, twt + static_cast<size_t>(x) * 16 + v * 2);
@@ -415,7 +415,7 @@ template <typename T>
 cudaError_t dft_x(const T* in, int S, int m, const float2* twt, float2* out, int rows, cudaStream_t st) {
   static std::atomic<uint64_t> attr{0};
   constexpr size_t smem = 2 * dx_stage_bytes<T>() + kRedBytes;
-  static_assert(smem <= 232448, "fno_dft_x: shared memory");
+  static_assert(smem <= 232448 / 2 - 1024, "fno_dft_x: shared memory");
   huv::once_per_device(attr, [] {
     huv::check_cuda(cudaFuncSetAttribute(fno_dft_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                     "cudaFuncSetAttribute(fno_dft_x)");
@@ -424,7 +424,7 @@ cudaError_t dft_x(const T* in, int S, int m, const float2* twt, float2* out, int
   cudaError_t e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  fno_dft_x<T><<<std::min(rows / kDxRows, sms), 512, smem, st>>>(in, S, m, twt, out, rows);
+  fno_dft_x<T><<<std::min(rows / kDxRows, 2 * sms), kDxThreads, smem, st>>>(in, S, m, twt, out, rows);
   return cudaGetLastError();
 }
 }  // namespace
