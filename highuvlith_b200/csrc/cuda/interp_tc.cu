@@ -29,6 +29,7 @@
 
 #include "../engine.hpp"
 #include "fft_reg.cuh"
+#include "pdl.cuh"
 #include "tc_ptx.cuh"
 
 namespace huv_dev {
@@ -71,6 +72,7 @@ template <int OUTBUFS>
 __global__ void __launch_bounds__(192, 1)
     tc_interp_fused(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmI,
                     const __grid_constant__ CUtensorMap tmO, InterpParams p) {
+  pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -360,9 +362,9 @@ cudaError_t interp_fused(const CUtensorMap& map_p, const void* im_split, int M, 
   p.probe_wait_ns = probe_wait_ns();
   const dim3 g(n / 256, (p.mt + p.mt_per - 1) / p.mt_per, nc);
   if (huv_dev::if_out_bufs(M) == 1)
-    huv_dev::tc_interp_fused<1><<<g, 192, huv_dev::if_smem_bytes(M), st>>>(map_p, mi, mo, p);
+    pdl(huv_dev::tc_interp_fused<1>, g, 192, huv_dev::if_smem_bytes(M), st, map_p, mi, mo, p);
   else
-    huv_dev::tc_interp_fused<2><<<g, 192, huv_dev::if_smem_bytes(M), st>>>(map_p, mi, mo, p);
+    pdl(huv_dev::tc_interp_fused<2>, g, 192, huv_dev::if_smem_bytes(M), st, map_p, mi, mo, p);
   return cudaGetLastError();
 }
 
