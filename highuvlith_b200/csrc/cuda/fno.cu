@@ -102,39 +102,51 @@ __global__ void fno_mix(const float2* __restrict__ X, const float2* __restrict__
   }
 }
 
-// dX = sum_o dY conj(R); dR += conj(X) dY (summed over the batch).
-__global__ void fno_mix_bwd(const float2* __restrict__ X, const float2* __restrict__ dY, const float2* __restrict__ R,
-                            int C, int modes, int B, float2* __restrict__ dX, float2* __restrict__ dR) {
-  extern __shared__ float2 sh[];  // [B][C] dY then [B][C] X
+// dX = sum_o dY conj(R) (o ascending); dR += conj(X) dY, summed over the batch;
+// dY scaled here by w_kx / S^2, the adjoint of the forward output weights.
+// One block per mode; R's 32 KB are staged once in shared memory (rows padded
+// to 65: both products read it without conflicts) and reused by every sample.
+// 8 samples: 0.088 + 0.008 (the scaling, a launch of its own) -> 0.03 ms.
+// Dynamic shared memory: [64][65] R, [B][64] dY, [B][64] X (float2).
+__global__ void __launch_bounds__(256) fno_mix_bwd(const float2* __restrict__ X, const float2* __restrict__ dY,
+                                                    const float2* __restrict__ R, int m, int modes, int B, float inv_s2,
+                                                    float2* __restrict__ dX, float2* __restrict__ dR) {
+  constexpr int C = 64, LD = 65;
+  extern __shared__ float2 sh[];
   const int md = blockIdx.x;
-  float2* sdy = sh;
-  float2* sxx = sh + B * C;
-  for (int t = threadIdx.x; t < B * C; t += blockDim.x) {
-    const int b = t / C, c = t - b * C;
-    sdy[t] = dY[(static_cast<size_t>(b) * modes + md) * C + c];
-    sxx[t] = X[(static_cast<size_t>(b) * modes + md) * C + c];
+  float2* sR = sh;
+  float2* sdy = sR + C * LD;
+  float2* sxx = sdy + B * C;
+  const float w = (md % m == 0 ? 1.f : 2.f) * inv_s2;
+  const float2* rr = R + static_cast<size_t>(md) * C * C;
+  for (int t = threadIdx.x; t < C * C; t += 256) sR[(t >> 6) * LD + (t & 63)] = rr[t];
+  for (int t = threadIdx.x; t < B * C; t += 256) {
+    const size_t g = (static_cast<size_t>(t >> 6) * modes + md) * C + (t & 63);
+    const float2 d = dY[g];
+    sdy[t] = make_float2(d.x * w, d.y * w);
+    sxx[t] = X[g];
   }
   __syncthreads();
-  const float2* rr = R + static_cast<size_t>(md) * C * C;
   float2* drr = dR + static_cast<size_t>(md) * C * C;
-  for (int t = threadIdx.x; t < C * C; t += blockDim.x) {
-    const int i = t / C, o = t - i * C;
+  for (int t = threadIdx.x; t < C * C; t += 256) {
+    const int i = t >> 6, o = t & 63;
     float re = 0.f, im = 0.f;
     for (int b = 0; b < B; ++b) {
       const float2 x = sxx[b * C + i], d = sdy[b * C + o];
       re += x.x * d.x + x.y * d.y;
       im += x.x * d.y - x.y * d.x;
     }
-    drr[t].x += re;
-    drr[t].y += im;
+    const float2 old = drr[t];
+    drr[t] = make_float2(old.x + re, old.y + im);
   }
-  for (int t = threadIdx.x; t < B * C; t += blockDim.x) {
-    const int b = t / C, i = t - b * C;
+  for (int t = threadIdx.x; t < B * C; t += 256) {
+    const int b = t >> 6, i = t & 63;
     float re = 0.f, im = 0.f;
+#pragma unroll 8
     for (int o = 0; o < C; ++o) {
-      const float2 d = sdy[b * C + o], w = rr[i * C + o];
-      re += d.x * w.x + d.y * w.y;
-      im += d.y * w.x - d.x * w.y;
+      const float2 d = sdy[b * C + o], w2 = sR[i * LD + o];
+      re += d.x * w2.x + d.y * w2.y;
+      im += d.y * w2.x - d.x * w2.y;
     }
     dX[(static_cast<size_t>(b) * modes + md) * C + i] = make_float2(re, im);
   }
@@ -275,13 +287,18 @@ __global__ void __launch_bounds__(256) fno_layer_bwd(const float* __restrict__ d
   if (t < C) atomicAdd(db + t, gb);
 }
 
-// dv[r][x][c] += Re sum_kx Z[r][kx][c] e^{+2 pi i kx x / S} (weight 1); rows
-// grid-strided, tiles of 64 pixels, thread (pg, cg) owns 4 x 4.
-// Dynamic shared memory: 2m * (64 + 68) floats.
+// dv[r][x][c] += Re sum_kx Z[r][kx][c] e^{+2 pi i kx x / S} (weight 1): the sum
+// over kk = (kx, re / im) ascending, then added to dv.  Rows grid-strided,
+// tiles of 128 pixels (S if smaller); thread (pg, cg) owns 8 pixels x 4
+// channels as pairs of channels, so that a step of kk costs three shared loads
+// for 16 paired multiply-adds, and fetches its dv before the sums.  Bound by
+// dv's 512 bytes per pixel and FP32 issue (8 x 512^2: 0.327 -> 0.27 ms against
+// 4 x 4 tiles of single multiply-adds).
+// Dynamic shared memory: 2m * (64 + 132) floats.
 __global__ void __launch_bounds__(256) fno_spec_to_dv(const float2* __restrict__ Z, int S, int m,
                                                        const float2* __restrict__ twx, float* __restrict__ dv,
                                                        int rows) {
-  constexpr int C = 64, XT = 64, LD = 68;
+  constexpr int C = 64, XT = 128, LD = 132;
   extern __shared__ __align__(16) float dsm[];
   float* sZ = dsm;              // [2m][C]
   float* sT = sZ + 2 * m * C;   // [2m][LD]
@@ -291,7 +308,7 @@ __global__ void __launch_bounds__(256) fno_spec_to_dv(const float2* __restrict__
     __syncthreads();
     const float2* Zr = Z + static_cast<size_t>(r) * m * C;
     for (int e = t; e < m * C; e += 256) {
-      const int kx = e / C, c = e - kx * C;
+      const int kx = e >> 6, c = e & 63;
       const float2 zz = Zr[e];
       sZ[(2 * kx) * C + c] = zz.x;
       sZ[(2 * kx + 1) * C + c] = -zz.y;
@@ -299,43 +316,44 @@ __global__ void __launch_bounds__(256) fno_spec_to_dv(const float2* __restrict__
     const size_t row = static_cast<size_t>(r) * S * C;
     for (int x0 = 0; x0 < S; x0 += xt) {
       __syncthreads();
-      for (int e = t; e < 2 * m * xt; e += 256) {
-        const int kk = e / xt, px = e - kk * xt;
-        const float2 w = __ldg(twx + static_cast<size_t>(kk >> 1) * S + x0 + px);
-        sT[kk * LD + px] = (kk & 1) ? -w.y : w.x;
+      for (int e = t; e < m * xt; e += 256) {
+        const int kx = e / xt, px = e - kx * xt;
+        const float2 w = __ldg(twx + static_cast<size_t>(kx) * S + x0 + px);  // (cos, -sin)
+        sT[(2 * kx) * LD + px] = w.x;
+        sT[(2 * kx + 1) * LD + px] = -w.y;
       }
+      const bool live = pg * 8 < xt;
+      float4* d = reinterpret_cast<float4*>(dv + row + static_cast<size_t>(x0 + pg * 8) * C + cg * 4);
+      float4 cur[8];
+#pragma unroll
+      for (int p = 0; p < 8; ++p) cur[p] = live ? d[p * (C / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
       __syncthreads();
-      if (pg * 4 < xt) {
-        float acc[4][4];
+      if (live) {
+        uint64_t acc[8][2];
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
+        for (int p = 0; p < 8; ++p) acc[p][0] = acc[p][1] = 0;
+#pragma unroll 4
+        for (int kk = 0; kk < 2 * m; ++kk) {
+          const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(sZ + kk * C + cg * 4);
+          const float4 t0 = ld4(sT + kk * LD + pg * 8), t1 = ld4(sT + kk * LD + pg * 8 + 4);
+          const float tv[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
 #pragma unroll
-          for (int q = 0; q < 4; ++q) acc[p][q] = 0.f;
-        for (int kk = 0; kk < 2 * m; ++kk) fma44(acc, ld4(sT + kk * LD + pg * 4), ld4(sZ + kk * C + cg * 4));
+          for (int p = 0; p < 8; ++p) {
+            uint64_t a;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(a) : "f"(tv[p]));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[p][0]) : "l"(a), "l"(z.x));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[p][1]) : "l"(a), "l"(z.y));
+          }
+        }
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          float4* d = reinterpret_cast<float4*>(dv + row + static_cast<size_t>(x0 + pg * 4 + p) * C + cg * 4);
-          float4 cur = *d;
-          cur.x += acc[p][0];
-          cur.y += acc[p][1];
-          cur.z += acc[p][2];
-          cur.w += acc[p][3];
-          *d = cur;
+        for (int p = 0; p < 8; ++p) {
+          float4 s;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(s.x), "=f"(s.y) : "l"(acc[p][0]));
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(s.z), "=f"(s.w) : "l"(acc[p][1]));
+          d[p * (C / 4)] = make_float4(cur[p].x + s.x, cur[p].y + s.y, cur[p].z + s.z, cur[p].w + s.w);
         }
       }
     }
-  }
-}
-
-// Scale dY(j, kx) by w_kx / S^2 (the adjoint of the forward output weights).
-__global__ void fno_scale_modes(float2* __restrict__ Y, int B, int J, int m, int C, float inv_s2) {
-  const size_t total = static_cast<size_t>(B) * J * m * C;
-  for (size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int kx = static_cast<int>((t / C) % m);
-    const float w = (kx == 0 ? 1.f : 2.f) * inv_s2;
-    Y[t].x *= w;
-    Y[t].y *= w;
   }
 }
 
@@ -662,6 +680,7 @@ struct Fno {
       check_cuda(cudaFuncSetAttribute(huv_dev::fno_layer_out, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
       check_cuda(cudaFuncSetAttribute(huv_dev::fno_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
       check_cuda(cudaFuncSetAttribute(huv_dev::fno_spec_to_dv, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
+      check_cuda(cudaFuncSetAttribute(huv_dev::fno_mix_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, big), "attr");
     });
     tc = S >= 128 && S % 128 == 0 && C == 64 && P == 128 && m <= 16;
     if (tc) {
@@ -752,7 +771,7 @@ struct Fno {
   static constexpr size_t kProjBwdSmem = (2 * 64 * 128 + 2 * 64 * 68 + 64 * 132 + 128 * 68 + 64) * 4;
   static constexpr size_t kLayerBwdSmem = (64 * 64 + 3 * 64 * 68) * 4;
   size_t layer_out_smem() const { return (2 * 64 * 68 + 2 * static_cast<size_t>(m) * (64 + 68)) * 4; }
-  size_t spec_smem() const { return (2 * static_cast<size_t>(m) * (64 + 68)) * 4; }
+  size_t spec_smem() const { return (2 * static_cast<size_t>(m) * (64 + 132)) * 4; }
   static unsigned pgrid(size_t pix) { return static_cast<unsigned>(std::min<size_t>((pix + 63) / 64, 296)); }
 
   // images[b][S][S] = FNO(masks[b]); with `keep`, everything a backward pass
@@ -820,10 +839,9 @@ struct Fno {
       }
       check_cuda(huv_launch::fno_dft_x_f32(dz, S, m, twt, Xa, rows, st), "fno dft x");
       check_cuda(huv_launch::fno_dft_y(Xa, B, S, m, tyt, Y, st), "fno dft y");
-      fno_scale_modes<<<256, 256, 0, st>>>(Y, B, J, m, C, 1.f / (static_cast<float>(S) * S));
-      fno_mix_bwd<<<modes, 256, static_cast<size_t>(2) * B * C * 8, st>>>(
-          Xl[l], Y, reinterpret_cast<const float2*>(par + oR[l]), C, modes, B, dX,
-          reinterpret_cast<float2*>(grad + oR[l]));
+      fno_mix_bwd<<<modes, 256, (static_cast<size_t>(2) * B * C + C * 65) * 8, st>>>(
+          Xl[l], Y, reinterpret_cast<const float2*>(par + oR[l]), m, modes, B,
+          1.f / (static_cast<float>(S) * S), dX, reinterpret_cast<float2*>(grad + oR[l]));
       check_cuda(huv_launch::fno_idft_y(dX, B, S, m, tyt, Za, nullptr, st), "fno inverse dft y");
       fno_spec_to_dv<<<rgrid, 256, spec_smem(), st>>>(Za, S, m, twx, dcur, rows);
       std::swap(dnext, dcur);

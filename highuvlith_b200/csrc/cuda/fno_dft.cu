@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128) fno_dft_y_inv(const float2* __restrict__ 
 // v0[b][p][c] = Wl[c][0] a + Wl[c][1] x/S + Wl[c][2] y/S + bl[c], BF16.
 // A thread keeps the weights of eight channels and writes 16 bytes per pixel;
 // bound by the 128 bytes per pixel it writes (one 2-byte store and 64-bit
-// index divisions per element before: 16 x 512^2: 1.36 -> 0.195 ms).
+// index divisions per element before: 16 x 512^2: 1.36 -> 0.17 ms).
 __global__ void __launch_bounds__(256) fno_lift(const float* __restrict__ a, int S, const float* __restrict__ Wl,
                                                  const float* __restrict__ bl, __nv_bfloat16* __restrict__ v,
                                                  int pixels) {
@@ -320,9 +320,11 @@ __global__ void __launch_bounds__(256) fno_lift(const float* __restrict__ a, int
     b[i] = bl[c0 + i];
   }
   const unsigned SS = static_cast<unsigned>(S) * S;
+  const int lgS = 31 - __clz(S);
+  const float inv_s = 1.f / S;  // S is a power of two: the product is the quotient
   for (int bp = (blockIdx.x * 256 + threadIdx.x) >> 3; bp < pixels; bp += (gridDim.x * 256) >> 3) {
-    const unsigned p = static_cast<unsigned>(bp) & (SS - 1);  // S is a power of two
-    const float gx = static_cast<float>(p & (S - 1)) / S, gy = static_cast<float>(p / S) / S;
+    const unsigned p = static_cast<unsigned>(bp) & (SS - 1);
+    const float gx = static_cast<float>(p & (S - 1)) * inv_s, gy = static_cast<float>(p >> lgS) * inv_s;
     const float av = a[bp];
     __align__(16) __nv_bfloat16 o[8];
 #pragma unroll
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(256) fno_lift(const float* __restrict__ a, int
 // multiply-add per term).  Tiles of 64 pixels through shared memory: loaded
 // with 16-byte accesses, summed over pixels by (channel, quarter of the tile)
 // and over channels by pixel.  Bound by dv0's 256 bytes per pixel (a strided
-// load per channel before: 8 x 512^2: 0.98 -> 0.33 ms).
+// load per channel before: 8 x 512^2: 0.98 -> 0.11 ms).
 __global__ void __launch_bounds__(256) fno_lift_bwd(const float* __restrict__ a, const float* __restrict__ dv0, int S,
                                                      const float* __restrict__ Wl, int pixels,
                                                      float* __restrict__ dWl, float* __restrict__ dbl,
@@ -349,6 +351,8 @@ __global__ void __launch_bounds__(256) fno_lift_bwd(const float* __restrict__ a,
   if (t < C) sw[t] = Wl[t * 3];
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   const unsigned SS = static_cast<unsigned>(S) * S;
+  const int lgS = 31 - __clz(S);
+  const float inv_s = 1.f / S;
   const int tiles = pixels / PT;  // S >= 8: a multiple of 64 pixels
   float4 next[4];
   auto fetch = [&](int tile) {
@@ -374,7 +378,7 @@ __global__ void __launch_bounds__(256) fno_lift_bwd(const float* __restrict__ a,
     for (int i = 0; i < PT / 4; ++i) {
       const int px = grp * (PT / 4) + i;
       const unsigned p = static_cast<unsigned>(tile * PT + px) & (SS - 1);
-      const float gx = static_cast<float>(p & (S - 1)) / S, gy = static_cast<float>(p / S) / S;
+      const float gx = static_cast<float>(p & (S - 1)) * inv_s, gy = static_cast<float>(p >> lgS) * inv_s;
       const float d = sd[px * LD + c];
       s0 += d * sa[px];
       s1 += d * gx;
