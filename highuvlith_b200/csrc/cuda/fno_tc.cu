@@ -396,22 +396,27 @@ __global__ void __launch_bounds__(32 * (2 + kFnoEpiWarps), 2)
 //   dz = dvnext * GELU'(z)  (or dvnext for the last layer), stored (f32);
 //   dv = dz W               (M 128 pixels, N 64 inputs, K 64 outputs), stored (f32);
 //   dW += dz^T v, db += sum dz over the CTA's tiles.
-// The elementwise part runs on CUDA cores (warps 5..20, two 8-channel chunks
-// of 32 pixels per thread, coalesced 32-byte rows) and writes the operands of
-// both GEMMs straight into shared memory in the 128B-swizzled K-major layout:
-// sA[px][o] = dz (A of dv), sX[ch][px] = (dz^T; v^T) (A of dW, 128 rows x 128
-// pixels in two 64-wide boxes; its rows 64..127, v^T, are also the B operand),
-// sWT[i][o] = W[o][i] (B of dv, converted from the f32 weights once per CTA).
-// dW is the top half of the 128 x 64 product (dz^T; v^T) v, accumulated in
-// tensor memory over every tile of the CTA and added to global memory once;
-// the bottom half (v^T v) is not used.  Warp 0 issues the MMAs (one thread),
-// warps 1..4 drain dv from tensor memory (one lane quadrant each).  Operand
-// stages and dv accumulators are double-buffered; one CTA per SM, persistent.
-// Every mbarrier wait is bounded; a timeout sets *err and unwinds.
-constexpr int kBwdXWarps = 16;                      // elementwise warps
-constexpr int kBwdThreads = 32 * (5 + kBwdXWarps);  // MMA + 4 epilogue + elementwise
-constexpr uint32_t kBwdStage = 16384 + 2 * 16384;   // sA + sX
-constexpr size_t kBwdSmem = 1024 + 8192 + 2 * static_cast<size_t>(kBwdStage) + 256;
+// The elementwise part runs on CUDA cores (warps 6..13; eight lanes take the
+// eight 8-channel octets of a pixel, so that a warp reads and writes whole
+// 256-byte rows) and writes dz as BF16 into shared memory in the 128B-swizzled
+// layout of a pixel row of 64 channels, where both GEMMs read it: K-major
+// [px][o] for dv, and MN-major (the same bytes, pixels as K) for dW, whose
+// other operand is the v tile as TMA loads it, MN-major too.  dW is the top
+// half of the 128 x 64 product (dz^T; v^T) v, accumulated in tensor memory
+// over every tile of the CTA and added to global memory once.  Warp 0 issues
+// the MMAs (one thread), warp 1 loads v, warps 2..5 drain dv from tensor
+// memory and store it with TMA.  Operand stages and dv accumulators are
+// double-buffered; two CTAs per SM, persistent.  Every mbarrier wait is
+// bounded; a timeout sets *err and unwinds.
+//
+// What bounds it: 1 KB per pixel, and GELU' (erff and expf).  With one pixel
+// per lane (32 rows of 16 bytes per access) and operands transposed by 2-byte
+// stores it was bound by L1 (87 %), 0.66 ms at 8 x 512^2; now 0.43 ms.
+constexpr int kBwdXWarps = 8;                       // elementwise warps
+constexpr int kBwdThreads = 32 * (6 + kBwdXWarps);  // MMA + TMA + 4 epilogue + elementwise
+constexpr uint32_t kBwdStage = 2 * 16384;           // dz [128 px][64 o], v [128 px][64 i]
+constexpr uint32_t kBwdOut = 32 * 32 * 4;           // dv staging tile: 32 px x 32 channels
+constexpr size_t kBwdSmem = 1024 + 8192 + 2 * static_cast<size_t>(kBwdStage) + 4 * 2 * kBwdOut + 256;
 
 __device__ __forceinline__ float tc_gelu_grad(float x) {
   const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
@@ -430,28 +435,29 @@ struct FnoBwdParams {
   int act;
   const float* dvnext;      // [pix][64]
   const __nv_bfloat16* z;   // [pix][64]
-  const __nv_bfloat16* v;   // [pix][64]
   const float* W;           // [64 o][64 i]
   float* dz;                // [pix][64]
-  float* dv;                // [pix][64]
   float* dW;                // [64][64], accumulated
   float* db;                // [64], accumulated
   int* err;
 };
 
-__global__ void __launch_bounds__(kBwdThreads, 1) fno_tc_layer_bwd(FnoBwdParams p) {
+__global__ void __launch_bounds__(kBwdThreads, 2)
+    fno_tc_layer_bwd(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDv, FnoBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* sWT = base;               // [64 i][64 o]
-  uint8_t* sS = base + 8192;         // [stage] { sA [128 px][64 o], sX [2 boxes][128 ch][64 px] }
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sS + 2 * kBwdStage);
+  uint8_t* sS = base + 8192;         // [stage] { dz, v }
+  uint8_t* sO = sS + 2 * kBwdStage;  // [epilogue warp][2]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + 4 * 2 * kBwdOut);
   uint64_t* full = bars;             // [2], one arrival per elementwise warp
-  uint64_t* empty = bars + 2;        // [2], MMA commit
-  uint64_t* tfull = bars + 4;        // [2]
-  uint64_t* tempty = bars + 6;       // [2], one arrival per epilogue warp
-  uint64_t* done = bars + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  uint64_t* vfull = bars + 2;        // [2], TMA
+  uint64_t* empty = bars + 4;        // [2], MMA commit
+  uint64_t* tfull = bars + 6;        // [2]
+  uint64_t* tempty = bars + 8;       // [2], one arrival per epilogue warp
+  uint64_t* done = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr uint32_t kTmemCols = 256;  // dv accumulators at 0 / 64, dW at 128
@@ -459,6 +465,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fno_tc_layer_bwd(FnoBwdParams 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&full[s], kBwdXWarps);
+      mbar_init(&vfull[s], 1);
       mbar_init(&empty[s], 1);
       mbar_init(&tfull[s], 1);
       mbar_init(&tempty[s], 4);
@@ -482,41 +489,58 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fno_tc_layer_bwd(FnoBwdParams 
 
   if (warp == 0) {
     if (lane == 0) {
-      const uint32_t idesc = idesc_bf16(128, 64);
+      const uint32_t idk = idesc_bf16(128, 64), idm = idk | kIdescAMn | kIdescBMn;
       const uint64_t bw = smem_desc_sw128(smem_u32(sWT));
       int it = 0;
       for (int t = blockIdx.x; t < p.tiles && !*abort_flag; t += gridDim.x, ++it) {
         const int s = it & 1;
-        if (!mbar_wait_or_abort(&tempty[s], ((it >> 1) & 1) ^ 1, kFnoWaitNs, abort_flag)) {
+        const uint32_t ph = (it >> 1) & 1;
+        if (!mbar_wait_or_abort(&tempty[s], ph ^ 1, kFnoWaitNs, abort_flag)) {
           fail(31);
           break;
         }
-        if (!mbar_wait_or_abort(&full[s], (it >> 1) & 1, kFnoWaitNs, abort_flag)) {
+        if (!mbar_wait_or_abort(&full[s], ph, kFnoWaitNs, abort_flag) ||
+            !mbar_wait_or_abort(&vfull[s], ph, kFnoWaitNs, abort_flag)) {
           fail(32);
           break;
         }
         tc_fence_after();
-        uint8_t* sA = sS + s * kBwdStage;
-        uint8_t* sX = sA + 16384;
-        const uint64_t aa = smem_desc_sw128(smem_u32(sA));
+        const uint32_t sA = smem_u32(sS + s * kBwdStage), sV = sA + 16384;
+        const uint64_t aa = smem_desc_sw128(sA);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) tc_mma_bf16(tmem_base + s * 64, aa + 2 * ks, bw + 2 * ks, idesc, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks) tc_mma_bf16(tmem_base + s * 64, aa + 2 * ks, bw + 2 * ks, idk, ks > 0 ? 1u : 0u);
         tc_commit(&tfull[s]);
+        // rows 0..63: dz^T, rows 64..127: v^T (the v tile follows dz's)
+        const uint64_t ax = smem_desc_sw128_mn(sA, 16384), bx = smem_desc_sw128_mn(sV, 16384);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          uint8_t* box = sX + (ks >> 2) * 16384;
-          const uint64_t ax = smem_desc_sw128(smem_u32(box)) + 2 * (ks & 3);
-          const uint64_t bx = smem_desc_sw128(smem_u32(box + 8192)) + 2 * (ks & 3);
-          tc_mma_bf16(tmem_base + 128, ax, bx, idesc, (it > 0 || ks > 0) ? 1u : 0u);
-        }
+        for (int ks = 0; ks < 8; ++ks)
+          tc_mma_bf16(tmem_base + 128, ax + kMnStep * ks, bx + kMnStep * ks, idm, (it > 0 || ks > 0) ? 1u : 0u);
         tc_commit(&empty[s]);
       }
       tc_commit(done);
       mbar_wait(done, 0, kFnoWaitNs);
     }
-  } else if (warp <= 4) {
+  } else if (warp == 1) {
+    if (lane == 0) {
+      prefetch_tmap(&tmV);
+      prefetch_tmap(&tmDv);
+      int it = 0;
+      for (int t = blockIdx.x; t < p.tiles && !*abort_flag; t += gridDim.x, ++it) {
+        const int s = it & 1;
+        if (!mbar_wait_or_abort(&empty[s], ((it >> 1) & 1) ^ 1, kFnoWaitNs, abort_flag)) {
+          fail(36);
+          break;
+        }
+        mbar_arrive_expect_tx(&vfull[s], kTile);
+        tma_load_2d(sS + s * kBwdStage + 16384, &tmV, 0, t * 128, &vfull[s]);
+      }
+      // every load issued lands before the CTA may exit
+      for (int q = (it > 2 ? it - 2 : 0); q < it; ++q) mbar_wait(&vfull[q & 1], (q >> 1) & 1, kFnoWaitNs);
+    }
+  } else if (warp <= 5) {
     // dv epilogue: lane quadrant warp % 4, one pixel row per lane
     const int quad = warp & 3;
+    uint8_t* st = sO + quad * 2 * kBwdOut;
     int it = 0;
     for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++it) {
       const int s = it & 1;
@@ -528,40 +552,54 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fno_tc_layer_bwd(FnoBwdParams 
       }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + s * 64;
-      float a[32], b[32];
-      tmem_ld32(taddr, a);
-      tmem_ld32(taddr + 32, b);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[s]);
-      float4* o = reinterpret_cast<float4*>(p.dv + (static_cast<size_t>(t) * 128 + quad * 32 + lane) * 64);
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        float a[32];
+        tmem_ld32(taddr + 32 * h, a);
+        if (h == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[s]);
+        }
+        if (lane == 0) bulk_wait_read<1>();  // this half's buffer was last stored one tile ago
+        __syncwarp();
+        uint8_t* o = st + h * kBwdOut;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) o[q] = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) o[8 + q] = make_float4(b[4 * q], b[4 * q + 1], b[4 * q + 2], b[4 * q + 3]);
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<float4*>(o + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+              make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tmDv, o, 32 * h, t * 128 + quad * 32);
+          bulk_commit();
+        }
+      }
     }
+    if (lane == 0 && it > 0) bulk_wait<0>();
+    __syncwarp();
     // dW rows o = lanes 0..63 of the second accumulator, once every MMA is complete
     if (quad < 2) {
       const bool fin = __all_sync(0xffffffffu, mbar_wait(done, 0, kFnoWaitNs));
       if (fin && !*abort_flag) {
         tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + 128;
-        float a[32], b[32];
-        tmem_ld32(taddr, a);
-        tmem_ld32(taddr + 32, b);
         float* w = p.dW + (quad * 32 + lane) * 64;
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          float a[32];
+          tmem_ld32(taddr + 32 * h, a);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) atomicAdd(w + i, a[i]);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) atomicAdd(w + 32 + i, b[i]);
+          for (int i = 0; i < 32; ++i) atomicAdd(w + 32 * h + i, a[i]);
+        }
       } else if (!fin && lane == 0) {
         fail(34);
       }
     }
   } else {
-    // elementwise warps: channel group og (8 channels), pixels 32 (2 jb + c) + lane
-    const int xw = warp - 5, og = xw & 7, jb = xw >> 3, o0 = 8 * og;
-    const int xt = threadIdx.x - 5 * 32;
+    // elementwise warps: lane = (pixel of four, octet of channels)
+    const int xw = warp - 6, o0 = 8 * (lane & 7);
+    const int xt = threadIdx.x - 6 * 32;
     // W^T into sWT once: element (o, i) of W is row i, column o of the B operand
     for (int e = xt; e < 64 * 64; e += 32 * kBwdXWarps) {
       const int o = e >> 6, i = e & 63;
@@ -573,52 +611,46 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fno_tc_layer_bwd(FnoBwdParams 
     int it = 0;
     for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++it) {
       const int s = it & 1;
-      float4 g[2][2];
-      uint4 zz[2], vv[2];
+      uint8_t* sA = sS + s * kBwdStage;
+      bool ok = true;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        float4 g[2][2];
+        uint4 zz[2];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int px = 32 * (2 * jb + c) + lane;
-        const size_t off = (static_cast<size_t>(t) * 128 + px) * 64 + o0;
-        g[c][0] = *reinterpret_cast<const float4*>(p.dvnext + off);
-        g[c][1] = *reinterpret_cast<const float4*>(p.dvnext + off + 4);
-        zz[c] = p.act ? *reinterpret_cast<const uint4*>(p.z + off) : make_uint4(0, 0, 0, 0);
-        vv[c] = *reinterpret_cast<const uint4*>(p.v + off);
+        for (int c = 0; c < 2; ++c) {
+          const int px = 16 * xw + 8 * h + 4 * c + (lane >> 3);
+          const size_t off = (static_cast<size_t>(t) * 128 + px) * 64 + o0;
+          g[c][0] = *reinterpret_cast<const float4*>(p.dvnext + off);
+          g[c][1] = *reinterpret_cast<const float4*>(p.dvnext + off + 4);
+          zz[c] = p.act ? *reinterpret_cast<const uint4*>(p.z + off) : make_uint4(0, 0, 0, 0);
+        }
+        if (h == 0)  // stage s was last read by the MMAs of tile it - 2
+          ok = __all_sync(0xffffffffu, mbar_wait_or_abort(&empty[s], ((it >> 1) & 1) ^ 1, kFnoWaitNs, abort_flag));
+        if (!ok) break;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int px = 16 * xw + 8 * h + 4 * c + (lane >> 3);
+          const size_t off = (static_cast<size_t>(t) * 128 + px) * 64 + o0;
+          const float gv[8] = {g[c][0].x, g[c][0].y, g[c][0].z, g[c][0].w, g[c][1].x, g[c][1].y, g[c][1].z, g[c][1].w};
+          const __nv_bfloat16* zb = reinterpret_cast<const __nv_bfloat16*>(&zz[c]);
+          float d[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            d[e] = p.act ? gv[e] * tc_gelu_grad(__bfloat162float(zb[e])) : gv[e];
+            dbp[e] += d[e];
+          }
+          reinterpret_cast<float4*>(p.dz + off)[0] = make_float4(d[0], d[1], d[2], d[3]);
+          reinterpret_cast<float4*>(p.dz + off)[1] = make_float4(d[4], d[5], d[6], d[7]);
+          __align__(16) __nv_bfloat16 db16[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) db16[e] = __float2bfloat16_rn(d[e]);
+          *reinterpret_cast<uint4*>(sA + sw128_off(px, o0)) = *reinterpret_cast<const uint4*>(db16);
+        }
       }
-      // stage s was last read by the MMAs of tile it - 2
-      const bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(&empty[s], ((it >> 1) & 1) ^ 1, kFnoWaitNs, abort_flag));
       if (!ok) {
         if (lane == 0) fail(35);
         break;
-      }
-      uint8_t* sA = sS + s * kBwdStage;
-      uint8_t* sX = sA + 16384;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int px = 32 * (2 * jb + c) + lane;
-        const size_t off = (static_cast<size_t>(t) * 128 + px) * 64 + o0;
-        const float gv[8] = {g[c][0].x, g[c][0].y, g[c][0].z, g[c][0].w, g[c][1].x, g[c][1].y, g[c][1].z, g[c][1].w};
-        const __nv_bfloat16* zb = reinterpret_cast<const __nv_bfloat16*>(&zz[c]);
-        const __nv_bfloat16* vb = reinterpret_cast<const __nv_bfloat16*>(&vv[c]);
-        float d[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          d[e] = p.act ? gv[e] * tc_gelu_grad(__bfloat162float(zb[e])) : gv[e];
-          dbp[e] += d[e];
-        }
-        reinterpret_cast<float4*>(p.dz + off)[0] = make_float4(d[0], d[1], d[2], d[3]);
-        reinterpret_cast<float4*>(p.dz + off)[1] = make_float4(d[4], d[5], d[6], d[7]);
-        __align__(16) __nv_bfloat16 db16[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) db16[e] = __float2bfloat16_rn(d[e]);
-        // A of dv: row px, 16-byte chunk og
-        *reinterpret_cast<uint4*>(sA + sw128_off(px, o0)) = *reinterpret_cast<const uint4*>(db16);
-        // A of dW: rows o (dz^T) and 64 + i (v^T), column px
-        uint8_t* box = sX + (px >> 6) * 16384;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          *reinterpret_cast<__nv_bfloat16*>(box + sw128_off(o0 + e, px & 63)) = db16[e];
-          *reinterpret_cast<__nv_bfloat16*>(box + sw128_off(64 + o0 + e, px & 63)) = vb[e];
-        }
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -628,9 +660,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fno_tc_layer_bwd(FnoBwdParams 
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         float x = dbp[e];
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) x += __shfl_xor_sync(0xffffffffu, x, sh);
-        if (lane == 0) atomicAdd(p.db + o0 + e, x);
+        x += __shfl_xor_sync(0xffffffffu, x, 8);
+        x += __shfl_xor_sync(0xffffffffu, x, 16);
+        if (lane < 8) atomicAdd(p.db + o0 + e, x);
       }
     }
   }
@@ -938,6 +970,7 @@ __global__ void fno_tw_table(const float2* __restrict__ twx, int S, int m, __nv_
 namespace huv_launch {
 bool tc_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows);
 
+bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols);
 bool tc_map_sw64_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows, int cols);
 
 cudaError_t fno_tc_set_smem() {
@@ -1003,23 +1036,23 @@ bool fno_tc_proj(int B, int S, const __nv_bfloat16* v, const __nv_bfloat16* Q1b,
 bool fno_tc_layer_bwd(size_t pix, const float* dvnext, const __nv_bfloat16* z, const __nv_bfloat16* v, const float* W,
                       int act, float* dz, float* dv, float* dW, float* db, int* err, cudaStream_t st) {
   if (pix % 128 != 0) return false;
+  CUtensorMap mv, mo;
+  if (!tc_map_bf16(&mv, v, pix, 64, 128) || !tc_map_out(&mo, dv, pix, 64)) return false;
   huv_dev::FnoBwdParams p{};
   p.tiles = static_cast<int>(pix / 128);
   p.act = act;
   p.dvnext = dvnext;
   p.z = z;
-  p.v = v;
   p.W = W;
   p.dz = dz;
-  p.dv = dv;
   p.dW = dW;
   p.db = db;
   p.err = err;
   int sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
-  const int grid = std::min(p.tiles, sms);
-  huv_dev::fno_tc_layer_bwd<<<grid, huv_dev::kBwdThreads, huv_dev::kBwdSmem, st>>>(p);
+  const int grid = std::min(p.tiles, 2 * sms);
+  huv_dev::fno_tc_layer_bwd<<<grid, huv_dev::kBwdThreads, huv_dev::kBwdSmem, st>>>(mv, mo, p);
   return cudaGetLastError() == cudaSuccess;
 }
 // Projection backward on tensor cores (see fno_tc_proj_bwd); v: [pix][64]

@@ -204,6 +204,23 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   return d;
 }
 
+// Shared-memory matrix descriptor: MN-major, 128-byte swizzle, for an operand
+// stored with its K index as rows: each row of 128 bytes holds 64 consecutive
+// M (or N) elements, 8-row groups are 1024 B apart, and further blocks of 64
+// elements lie `block` bytes apart.  A 16-wide K step advances it by kMnStep.
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t saddr, uint32_t block) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);       // start address
+  d |= static_cast<uint64_t>(block >> 4) << 16;               // leading byte offset: next 64 elements
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;                // stride byte offset: 8 K rows x 128 B
+  d |= static_cast<uint64_t>(1) << 46;                        // descriptor version (sm_100)
+  d |= static_cast<uint64_t>(2) << 61;                        // layout: SWIZZLE_128B
+  return d;
+}
+constexpr uint64_t kMnStep = 16 * 128 / 16;
+// Instruction-descriptor bits: A or B is MN-major.
+constexpr uint32_t kIdescAMn = 1u << 15, kIdescBMn = 1u << 16;
+
 // Shared-memory matrix descriptor: K-major, 64-byte swizzle, rows of 64 B,
 // 8-row groups 512 B apart (the layout TMA writes with SWIZZLE_64B).
 __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
