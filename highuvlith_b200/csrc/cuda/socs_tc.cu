@@ -978,6 +978,19 @@ bool tc_map_sw64_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, 
 }
 bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) { return make_out_map(map, ptr, rows, cols); }
 
+// f32 map over [rows][cols] with boxes of 8 columns x 32 rows, unswizzled.
+bool tc_map_out8(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) {
+  auto fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
+  cuuint32_t box[2] = {8, 32};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 cudaError_t tc_set_smem() {
   const int bytes = static_cast<int>(tc_smem_bytes(3));
   cudaError_t e;
