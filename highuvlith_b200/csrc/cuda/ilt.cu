@@ -918,7 +918,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
     const float* tg = target + npix * c0;
     pdl(ilt_transmittance, 1184, 256, 0, st, th, npix * nc, static_cast<float>(p.beta),
                                             static_cast<float>(p.absorber), tbuf);
-    check_cuda(band_forward(tbuf, HUV_INPUT_RASTER_F32, n, lgn, hb, nc, X, Mb, nullptr, ds.W, mean, twn, st, nullptr, nullptr),
+    check_cuda(band_forward(tbuf, HUV_INPUT_RASTER_F32, n, lgn, hb, nc, X, Mb, nullptr, ds.W, mean, twn, st, nullptr, nullptr, true),
                "ilt band_forward");
     // fields of every kernel on the evaluation grid, the image on it, then on N x N
     // x-major row transforms (register-radix kernels) when the adjoint's
@@ -943,7 +943,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
     }
     if (coarse && !sep) {
       check_cuda(band_forward(IM, HUV_INPUT_RASTER_F32, M, lgm, h2, nc, X2, C, nullptr, nullptr, nullptr, twm, st, nullptr,
-                              nullptr),
+                              nullptr, true),
                  "ilt band(I)");
       const float scale = 1.0f / static_cast<float>(mpix);
       check_cuda(socs_rows_x(nullptr, scale, C, 1, h2, n, nc, X2, twn, st), "ilt interp rows");

@@ -525,6 +525,74 @@ __global__ void __launch_bounds__(fr_threads(L, S), (L >= 384 ? 4 : 1))
   }
 }
 
+// band_rows_reg for shorter f32 rows and for complex rows.  CPLX: one row per
+// sequence, S rows per block, read straight in the first pass; X:
+// [clip][y][B].  Real: 2 S rows per block, sequence s packing rows s and s + S
+// as re / im, staged first with 16-byte copies (rows padded by 16 bytes: the
+// first pass's 8 sequences x 4 elements then touch 32 banks); X:
+// [clip][y][hb + 1] as in band_rows_reg.  Bound by FP32 issue; the radix-4
+// kernel took 33 us for 27 maps of 512^2 and 19.5 us for 7 complex ones, this
+// 15 and 11.  grid: clips * L / (rows per block).
+template <int L, int S, bool CPLX>
+__global__ void __launch_bounds__(fr_threads(L, S), 3)
+    band_rows_img(const void* __restrict__ in, int hb, float2* __restrict__ X, const float2* __restrict__ tw) {
+  pdl_begin();
+  constexpr int T = fr_threads(L, S), NP = fr_passes(L), LD = L + 4;
+  extern __shared__ __align__(16) float2 smem[];
+  const int t = threadIdx.x;
+  float2* b0 = smem;
+  const size_t row0 = static_cast<size_t>(blockIdx.x) * (CPLX ? S : 2 * S);
+  float* stage = reinterpret_cast<float*>(b0 + fr_buf(L, S));
+  if (!CPLX) {
+    const float* src = static_cast<const float*>(in) + row0 * L;
+    for (int e = t; e < 2 * S * (L / 4); e += T) {
+      const int r = e / (L / 4), c = (e - r * (L / 4)) * 4;
+      fr_cp_async16(stage + r * LD + c, src + static_cast<size_t>(r) * L + c);
+    }
+    fr_cp_commit();
+    fr_cp_wait<0>();
+    __syncthreads();
+  }
+  if (t < fr_nb(L, S, 0)) {
+    const int s = t % S, j = t / S;
+    float2 v[16];
+    if (CPLX) {
+      const float2* r0 = static_cast<const float2*>(in) + (row0 + s) * L + j;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = r0[r * (L / 16)];
+    } else {
+      const float* ra = stage + s * LD + j;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = make_float2(ra[r * (L / 16)], ra[S * LD + r * (L / 16)]);
+    }
+    fr_first_pass_vals<L, S, -1>(t, v, b0);
+  }
+  __syncthreads();
+  fr_mid_pass_inplace<L, S, -1, 1>(t, b0, tw);
+  if constexpr (NP == 3) {
+    __syncthreads();
+    fr_mid_pass_inplace<L, S, -1, 2>(t, b0, tw);
+  }
+  __syncthreads();
+  if (CPLX) {
+    const int B = 2 * hb + 1;
+    for (int e = t; e < S * B; e += T) {
+      const int s = e / B, m = e - s * B - hb;
+      X[row0 * B + e] = b0[fr_idx<S>(m < 0 ? m + L : m, s)];
+    }
+  } else {
+    const int H = hb + 1;
+    for (int e = t; e < S * H; e += T) {
+      const int s = e / H, m = e - s * H;
+      const float2 z = b0[fr_idx<S>(m, s)];
+      const float2 zc = cconj(b0[fr_idx<S>(m == 0 ? 0 : L - m, s)]);
+      const float2 d = csub(z, zc);
+      X[(row0 + s) * H + m] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
+      X[(row0 + s + S) * H + m] = make_float2(0.5f * d.y, -0.5f * d.x);
+    }
+  }
+}
+
 // band_cols_fwd with register-radix passes: forward FFT along y of S band
 // columns per block, the first pass reading X directly.  X is [clip][y][B]
 // (every order mx = -hb..hb), or, with `half`, the orders mx = 0..hb of a
@@ -651,7 +719,8 @@ cudaError_t socs_cols(const float2* T, int K, int hb, int lgm, int clips, float 
 // receives that kernel's timeout code.
 cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int clips, float2* X,
                          float2* Mband, const float* ptx, const float* W, float* mean,
-                         const float2* tw, cudaStream_t st, const uint8_t* row_digits, int* err) {
+                         const float2* tw, cudaStream_t st, const uint8_t* row_digits, int* err,
+                         bool radix4_rows) {
   // n need not be a power of two when the register-radix kernels serve it
   // (160 = 16 x 10, 192 = 16 x 12); the radix-4 kernels use lg = log2 n.
   const bool pow2 = (n & (n - 1)) == 0;
@@ -671,7 +740,7 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
   const bool cols_reg = xt_ok(n, hb);
   // (and then, as the register-radix rows do, only the orders m = 0..hb of
   // the real rasters: `half`)
-  bool x_transposed = false, half = false;
+  bool x_transposed = false, half = false, rows_done = false;
   if (kind == 0 && row_digits) {
     rows_tc = mask_rows_tc(in, n, hb, clips, X, row_digits, err, st, cols_reg);
     x_transposed = half = rows_tc == cudaSuccess && cols_reg;
@@ -705,6 +774,31 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     rows_tc = cudaSuccess;
     half = true;
   }
+  // f32 rows of 128 to 512 points and complex rows, unless the caller wants
+  // the radix-4 kernel's bits
+  if (rows_tc != cudaSuccess && cols_reg && !radix4_rows && n <= 2048 &&
+      (kind == 2 ? n >= 128 : (kind == 1 && n <= 512))) {
+    const int Sr = xt_S(n);
+    const unsigned blocks = static_cast<unsigned>(static_cast<size_t>(clips) * n / (kind == 2 ? Sr : 2 * Sr));
+    const size_t smr = xt_buf_bytes(n) + (kind == 2 ? 0 : static_cast<size_t>(2) * Sr * (n + 4) * sizeof(float));
+    cudaError_t e = cudaErrorNotSupported;
+#define HUV_ROWS_IMG(LL, SS)                                                                            \
+  case LL:                                                                                              \
+    if (kind == 2)                                                                                      \
+      e = pdl(band_rows_img<LL, SS, true>, blocks, 256, smr, st, in, hb, X, tw);                        \
+    else if (LL <= 512)                                                                                 \
+      e = pdl(band_rows_img<(LL <= 512 ? LL : 512), (LL <= 512 ? SS : 8), false>, blocks, 256, smr, st, in, hb, X, tw); \
+    break;
+    switch (n) {
+      HUV_ROWS_IMG(128, 32) HUV_ROWS_IMG(256, 16) HUV_ROWS_IMG(512, 8) HUV_ROWS_IMG(1024, 4) HUV_ROWS_IMG(2048, 2)
+    }
+#undef HUV_ROWS_IMG
+    if (e == cudaSuccess) {
+      rows_tc = cudaSuccess;
+      half = kind == 1;
+      rows_done = true;
+    }
+  }
   if (!pow2 && rows_tc != cudaSuccess) return cudaErrorInvalidValue;  // no radix-4 kernel for this length
   // Only device rasters come here (rectangle clips take the analytic path).
   switch (kind) {
@@ -714,7 +808,8 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     case 1:
       if (rows_tc != cudaSuccess) pdl(band_rows_fwd<1>, g1, th, sm1, st, in, lg, rows_per_block, hb, X, tw);
       break;
-    case 2: pdl(band_rows_fwd<2>, g1, th, sm1, st, in, lg, rows_per_block, hb, X, tw); break;
+    case 2:
+      if (!rows_done) pdl(band_rows_fwd<2>, g1, th, sm1, st, in, lg, rows_per_block, hb, X, tw); break;
     default: return cudaErrorInvalidValue;
   }
   const int B = 2 * hb + 1;
@@ -905,6 +1000,10 @@ cudaError_t set_smem_limits() {
   HUV_XT_ATTR((band_rows_reg<1024, 4>)) HUV_XT_ATTR((band_rows_reg<160, 16>))
   HUV_XT_ATTR((band_rows_reg<192, 16>)) HUV_XT_ATTR((band_rows_reg<2048, 2>)) HUV_XT_ATTR((band_rows_reg<384, 8>))
   HUV_XT_ATTR((band_rows_reg<2048, 2, uint8_t>))
+  HUV_XT_ATTR((band_rows_img<128, 32, true>)) HUV_XT_ATTR((band_rows_img<256, 16, true>))
+  HUV_XT_ATTR((band_rows_img<512, 8, true>)) HUV_XT_ATTR((band_rows_img<1024, 4, true>))
+  HUV_XT_ATTR((band_rows_img<2048, 2, true>)) HUV_XT_ATTR((band_rows_img<128, 32, false>))
+  HUV_XT_ATTR((band_rows_img<256, 16, false>)) HUV_XT_ATTR((band_rows_img<512, 8, false>))
 #undef HUV_XT_ALL
 #undef HUV_XT_ATTR
   return field_fused_set_smem();

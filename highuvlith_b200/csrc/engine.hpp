@@ -19,7 +19,7 @@ namespace huv_launch {
 // one declaration every caller sees.
 cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int clips, float2* X, float2* Mband,
                          const float* ptx, const float* W, float* mean, const float2* tw, cudaStream_t st,
-                         const uint8_t* row_digits, int* err);
+                         const uint8_t* row_digits, int* err, bool radix4_rows = false);
 }  // namespace huv_launch
 
 namespace huv {
