@@ -613,6 +613,119 @@ __global__ void __launch_bounds__(256, 4) ilt_finish_tiled(const float* __restri
   if (threadIdx.x == 0) parts[static_cast<size_t>(mask) * gridDim.x + blockIdx.x] = cs;
 }
 
+// ilt_finish_tiled on 64 x 64 tiles with 4 x 4 pixels per thread: a thread
+// holds its pixels' m with a ring of one around them in registers, so that the
+// difference quotients' rsqrt of a pixel serves the pixel itself, its right
+// and its lower neighbour (24 per 16 pixels instead of 48) and m costs 18
+// shared loads per 16 pixels instead of 7 per pixel; theta arrives in 16-byte
+// loads.  Bound by instruction issue beside 12 bytes per pixel: 64 masks of
+// 1024^2 0.248 -> 0.226 ms.
+__global__ void __launch_bounds__(256, 3)
+    ilt_finish_4x4(const float* __restrict__ theta, const float* __restrict__ dcdm, int n, float beta, float tv_w,
+                   float tv_eps, float bin_w, float* __restrict__ grad, double* __restrict__ parts) {
+  pdl_begin();
+  constexpr int TS = 64, LD = 72, C0 = 4;  // column j of the tile at C0 + j: whole 16-byte runs
+  __shared__ __align__(16) float sm[TS + 2][LD];
+  __shared__ double red[32];
+  const int mask = blockIdx.y, t = threadIdx.x;
+  const size_t npix = static_cast<size_t>(n) * n;
+  const int tiles_x = n / TS;
+  const int ti = blockIdx.x / tiles_x, tj = blockIdx.x - ti * tiles_x;
+  const float* th = theta + mask * npix;
+  const float inv_n = 1.f / static_cast<float>(npix);
+  const int tx = t & 15, ty = t >> 4;
+  auto wrap = [&](int i) { return i < 0 ? i + n : (i >= n ? i - n : i); };
+  // the tile's rows -1 .. 64: 16 runs of four each, and the columns -1 and 64
+  float4 tv[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int e = t + 256 * q;
+    if (e < (TS + 2) * 16)
+      tv[q] = *reinterpret_cast<const float4*>(th + static_cast<size_t>(wrap(ti * TS - 1 + (e >> 4))) * n + tj * TS + (e & 15) * 4);
+  }
+  float th_side = 0.f;
+  if (t < 2 * (TS + 2))
+    th_side = th[static_cast<size_t>(wrap(ti * TS - 1 + (t >> 1))) * n + wrap(tj * TS + ((t & 1) ? TS : -1))];
+  const size_t gp = mask * npix + static_cast<size_t>(ti * TS + ty * 4) * n + tj * TS + tx * 4;
+  float4 d4[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    d4[q] = dcdm ? *reinterpret_cast<const float4*>(dcdm + gp + static_cast<size_t>(q) * n) : make_float4(0.f, 0.f, 0.f, 0.f);
+  auto sig = [&](float v) { return 1.f / (1.f + __expf(-beta * v)); };
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int e = t + 256 * q;
+    if (e < (TS + 2) * 16)
+      *reinterpret_cast<float4*>(&sm[e >> 4][C0 + (e & 15) * 4]) =
+          make_float4(sig(tv[q].x), sig(tv[q].y), sig(tv[q].z), sig(tv[q].w));
+  }
+  if (t < 2 * (TS + 2)) sm[t >> 1][(t & 1) ? C0 + TS : C0 - 1] = sig(th_side);
+  __syncthreads();
+  float m[6][6];  // rows -1 .. 4, columns -1 .. 4 of the thread's pixels
+#pragma unroll
+  for (int r = 0; r < 6; ++r) {
+    const float* row = &sm[ty * 4 + r][C0 + tx * 4];
+    const float4 v = *reinterpret_cast<const float4*>(row);
+    m[r][0] = row[-1];
+    m[r][1] = v.x;
+    m[r][2] = v.y;
+    m[r][3] = v.z;
+    m[r][4] = v.w;
+    m[r][5] = row[4];
+  }
+  const float eps2 = tv_eps * tv_eps;
+  float tv_part = 0.f, bin_part = 0.f;
+  float up[4];  // (m(r) - m(r - 1)) rsqrt(...) of the pixels above
+  // rsqrt of pixel (r, c) of the 6 x 6 block, its value under the root in q
+  auto root = [&](int r, int c, float& q) {
+    const float gx = m[r][c + 1] - m[r][c], gy = m[r + 1][c] - m[r][c];
+    q = gx * gx + gy * gy + eps2;
+    return rsqrtf(q);
+  };
+  if (tv_w > 0.f && grad) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float q;
+      up[c] = (m[1][c + 1] - m[0][c + 1]) * root(0, c + 1, q);
+    }
+  }
+#pragma unroll
+  for (int r = 1; r < 5; ++r) {
+    const float dv[4] = {d4[r - 1].x, d4[r - 1].y, d4[r - 1].z, d4[r - 1].w};
+    float out[4];
+    float left = 0.f;  // (m(c) - m(c - 1)) rsqrt(...) of the pixel to the left
+    if (tv_w > 0.f && grad) {
+      float q;
+      left = (m[r][1] - m[r][0]) * root(r, 0, q);
+    }
+#pragma unroll
+    for (int c = 1; c < 5; ++c) {
+      const float mm = m[r][c];
+      float g = 0.f;
+      if (tv_w > 0.f) {
+        float q;
+        const float iv = root(r, c, q);
+        const float gx = (m[r][c + 1] - mm) * iv, gy = (m[r + 1][c] - mm) * iv;
+        tv_part += q * iv - tv_eps;
+        if (grad) {
+          g += tv_w * inv_n * (left + up[c - 1] - gx - gy);
+          left = gx;
+          up[c - 1] = gy;
+        }
+      }
+      if (bin_w > 0.f) {
+        bin_part += mm * (1.f - mm);
+        g += bin_w * 4.f * (1.f - 2.f * mm) * inv_n;
+      }
+      out[c - 1] = (dv[c - 1] + g) * beta * mm * (1.f - mm);
+    }
+    if (grad) *reinterpret_cast<float4*>(grad + gp + static_cast<size_t>(r - 1) * n) = make_float4(out[0], out[1], out[2], out[3]);
+  }
+  const double cost = (static_cast<double>(tv_w) * tv_part + 4.0 * static_cast<double>(bin_w) * bin_part) * inv_n;
+  const double cs = block_sum_double(cost, red);
+  if (t == 0) parts[static_cast<size_t>(mask) * gridDim.x + blockIdx.x] = cs;
+}
+
 // ------------------------------------------------------------ optimizer algebra
 // Per-mask reductions over n elements: out[mask] = sum a*b (dot) or max |a|.
 __global__ void batched_dot(const float* __restrict__ a, const float* __restrict__ b, size_t n,
@@ -1026,8 +1139,10 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
         check_cuda(socs_cols_x(T2, 1, hb, n, nc, 1.f, 0.f, nullptr, dcdm, 1, twn, st), "ilt grad cols");
       }
     }
+    // 16-byte accesses of theta and the gradient (a caller's planes may lie anywhere)
+    const bool vec16 = ((reinterpret_cast<uintptr_t>(th) | reinterpret_cast<uintptr_t>(grad)) & 15u) == 0;
     if (tile == 64)
-      pdl(ilt_finish_tiled<64>, dim3(reg_parts, nc), 256, 0, st, 
+      pdl(vec16 ? ilt_finish_4x4 : ilt_finish_tiled<64>, dim3(reg_parts, nc), 256, 0, st, 
           th, dcdm, n, static_cast<float>(p.beta), static_cast<float>(p.tv_weight),
           static_cast<float>(p.tv_epsilon), static_cast<float>(p.binarization_weight),
           grad ? grad + npix * c0 : nullptr, preg);
