@@ -15,13 +15,16 @@
 //      the epilogue multiplying interp_scale back and storing with TMA.
 // Every product is hi.hi + hi.lo + lo.hi with FP32 accumulation.
 //
-// What bounds it: the latency of P's stream.  Z^T stays on chip and an output
-// tile streams P's 80 KB from L2 through a ring of 8 KB stages, where the
-// two-kernel path wrote Z^T to HBM and streamed 160 KB of it back per tile;
-// 256 clips of 1024^2 at M = 160: 0.382 -> 0.317 ms (3.4 TB/s of image).
-// With a third of the products it still took 0.347 ms (at 4 stages), with no
-// stores 0.281; 256-bit stores straight from registers, which leave room for
-// 8 stages, 0.375; the same with eight epilogue warps 0.370.
+// What bounds it: the latency of P's stream and the set-up of a CTA (I_M, the
+// first product and its split: a fifth of its time).  Z^T stays on chip and an
+// output tile streams P's 80 KB from L2, in contiguous 8 KB copies of the
+// tiled operand, where the two-kernel path wrote Z^T to HBM and streamed
+// 160 KB of it back per tile.  256 clips of 1024^2 at M = 160: 0.382 -> 0.300 ms
+// (3.6 TB/s of image).  On the way: four epilogue warps with 4 KB tiles, P by
+// tensor copies of 64-byte rows, 4 stages 0.367, 6 stages 0.317; eight warps
+// with 2 KB tiles 0.308; contiguous copies 0.300 (0.349 with 4 stages).  With a
+// third of the products 0.266, without stores 0.291, with neither 0.232;
+// 256-bit stores from registers 0.375.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -37,17 +40,17 @@ namespace huv_dev {
 constexpr int kIfMaxM = 160;
 constexpr uint32_t kIfPBox = 128 * 64;    // 128 rows of P x 32 fp16, one plane
 constexpr uint32_t kIfZBox = 256 * 64;    // 256 rows X of Z^T x 32 fp16, one plane
-constexpr uint32_t kIfOutTile = 32 * 32 * 4;
-// staging tiles per epilogue warp: one where Z^T leaves little room, since the
-// kernel is bound by how much of P is in flight (256 clips, M = 160: two
-// staging tiles and 4 stages 0.367 ms, one and 6 stages 0.317 ms)
+constexpr uint32_t kIfOutTile = 32 * 16 * 4;  // 32 rows Y x 16 columns X
+constexpr int kIfEpiWarps = 8;            // two per tensor-memory lane quadrant
+// staging tiles per epilogue warp: one where Z^T leaves little room for P's
+// stages, of which the kernel wants many
 __host__ __device__ constexpr int if_out_bufs(int M) { return M > 96 ? 1 : 2; }
 constexpr int kIfMaxStages = 10;
 constexpr uint64_t kIfWaitNs = 2000000000ull;
 
 __host__ __device__ constexpr int if_boxes(int M) { return (M + 31) / 32; }
 __host__ __device__ constexpr size_t if_fixed_bytes(int M) {
-  return 1024 + 2 * static_cast<size_t>(if_boxes(M)) * kIfZBox + 4 * if_out_bufs(M) * static_cast<size_t>(kIfOutTile) + 256;
+  return 1024 + 2 * static_cast<size_t>(if_boxes(M)) * kIfZBox + kIfEpiWarps * if_out_bufs(M) * static_cast<size_t>(kIfOutTile) + 256;
 }
 // P stages of 8 KB: what one CTA's shared memory holds beside Z^T (6 at M = 160)
 __host__ __device__ constexpr int if_stages(int M) {
@@ -63,15 +66,15 @@ struct InterpParams {
   int M, stages;
   int n;               // output grid side (rows of P per plane)
   int mt, mt_per;      // 128-row output tiles, and tiles per CTA
+  const uint8_t* P;    // [row tile][box][plane] x 8 KB, 64B-swizzled
   const float* mean;
   int* err;
   unsigned long long probe_wait_ns;
 };
 
 template <int OUTBUFS>
-__global__ void __launch_bounds__(192, 1)
-    tc_interp_fused(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmI,
-                    const __grid_constant__ CUtensorMap tmO, InterpParams p) {
+__global__ void __launch_bounds__(32 * (2 + kIfEpiWarps), 1)
+    tc_interp_fused(const __grid_constant__ CUtensorMap tmI, const __grid_constant__ CUtensorMap tmO, InterpParams p) {
   pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -80,7 +83,7 @@ __global__ void __launch_bounds__(192, 1)
   uint8_t* sZ = base;                               // [plane][box] Z^T; first [plane][box] I_M
   uint8_t* sP = sZ + 2 * nbox * kIfZBox;            // [stage] one plane, one box
   uint8_t* sO = sP + p.stages * kIfPBox;            // [epilogue warp][buffer]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + 4 * OUTBUFS * kIfOutTile);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + kIfEpiWarps * OUTBUFS * kIfOutTile);
   uint64_t* full = bars;
   uint64_t* empty = bars + kIfMaxStages;
   uint64_t* i_full = bars + 2 * kIfMaxStages;
@@ -104,11 +107,11 @@ __global__ void __launch_bounds__(192, 1)
     }
     mbar_init(i_full, 1);
     mbar_init(z_full, 1);
-    mbar_init(z_ready, 4);
+    mbar_init(z_ready, kIfEpiWarps);
     mbar_init(&tfull[0], 1);
     mbar_init(&tfull[1], 1);
-    mbar_init(&tempty[0], 4);
-    mbar_init(&tempty[1], 4);
+    mbar_init(&tempty[0], kIfEpiWarps);
+    mbar_init(&tempty[1], kIfEpiWarps);
     mbar_init(done, 1);
     *abort_flag = 0;
     fence_barrier_init();
@@ -129,7 +132,6 @@ __global__ void __launch_bounds__(192, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      prefetch_tmap(&tmP);
       prefetch_tmap(&tmI);
       prefetch_tmap(&tmO);
       mbar_arrive_expect_tx(i_full, 2u * nbox * ibox);
@@ -141,7 +143,8 @@ __global__ void __launch_bounds__(192, 1)
       bool ok = true;
       const int tiles = 2 + m1 - m0;
       for (int t = 0; t < tiles && ok && !*abort_flag; ++t) {
-        const int row = t < 2 ? xt * 256 + t * 128 : (m0 + t - 2) * 128;
+        // the row tile's boxes are contiguous: [box][plane] x 8 KB
+        const uint8_t* src = p.P + static_cast<size_t>(t < 2 ? xt * 2 + t : m0 + t - 2) * 2 * nbox * kIfPBox;
         for (int kb = 0; kb < nbox && ok; ++kb)
           for (int pl = 0; pl < 2; ++pl, ++it) {
             const int s = it % p.stages;
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(192, 1)
               break;
             }
             mbar_arrive_expect_tx(&full[s], kIfPBox);
-            tma_load_2d(sP + s * kIfPBox, &tmP, kb * 32, pl * p.n + row, &full[s]);
+            bulk_load(sP + s * kIfPBox, src + (kb * 2 + pl) * kIfPBox, kIfPBox, &full[s]);
           }
       }
       // every load issued must have landed before the CTA may exit
@@ -230,7 +233,8 @@ __global__ void __launch_bounds__(192, 1)
       mbar_wait(done, 0, kIfWaitNs);
     }
   } else {
-    // epilogue warps 2..5: tensor-memory lane quadrant = warp % 4
+    // epilogue warps 2..9: tensor-memory lane quadrant = warp % 4; warps 2..5
+    // take the first tile of Z^T and half of an output tile's columns, 6..9 the second
     const int quad = warp & 3;
     const uint32_t lrow = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     int nst = 0;  // TMA-store tiles issued by this warp
@@ -239,8 +243,8 @@ __global__ void __launch_bounds__(192, 1)
       tc_fence_after();
       // Z^T -> FP16 hi/lo planes: row X of a box holds 32 y in four 16-byte
       // chunks (64B swizzle: chunk ^ (row / 2) % 4)
-#pragma unroll 1
-      for (int t = 0; t < 2; ++t) {
+      {
+        const int t = warp >= 6;
         const int row = t * 128 + quad * 32 + lane;
         const uint32_t sw = static_cast<uint32_t>(row >> 1) & 3u;
 #pragma unroll 1
@@ -285,24 +289,26 @@ __global__ void __launch_bounds__(192, 1)
       }
       tc_fence_after();
 #pragma unroll 1
-      for (int c0 = 0; c0 < 256; c0 += 32) {
+      for (int c0 = (warp >= 6 ? 128 : 0); c0 < (warp >= 6 ? 256 : 128); c0 += 32) {
         float v[32];
         tmem_ld32(lrow + buf * 256 + c0, v);
-        // buffer `sb` was last read by the store issued OUTBUFS tiles ago
-        if (lane == 0 && nst >= OUTBUFS) bulk_wait_read<OUTBUFS - 1>();
-        __syncwarp();
-        uint8_t* sb = sO + (quad * OUTBUFS + nst % OUTBUFS) * kIfOutTile;
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<float4*>(sb + lane * 128 + ((q ^ (lane & 7)) << 4)) =
-              make_float4(osc * v[4 * q], osc * v[4 * q + 1], osc * v[4 * q + 2], osc * v[4 * q + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(&tmO, sb, xt * 256 + c0, prob * p.n + (m0 + i) * 128 + quad * 32);
-          bulk_commit();
+        for (int h = 0; h < 2; ++h) {
+          if (lane == 0 && nst >= OUTBUFS) bulk_wait_read<OUTBUFS - 1>();
+          __syncwarp();
+          uint8_t* sb = sO + ((warp - 2) * OUTBUFS + nst % OUTBUFS) * kIfOutTile;
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<float4*>(sb + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) =
+                make_float4(osc * v[16 * h + 4 * q], osc * v[16 * h + 4 * q + 1], osc * v[16 * h + 4 * q + 2], osc * v[16 * h + 4 * q + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tmO, sb, xt * 256 + c0 + 16 * h, prob * p.n + (m0 + i) * 128 + quad * 32);
+            bulk_commit();
+          }
+          ++nst;
         }
-        ++nst;
       }
       tc_fence_before();
       __syncwarp();
@@ -323,15 +329,26 @@ __global__ void __launch_bounds__(192, 1)
 namespace huv_launch {
 
 bool tc_map_sw64_f16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows, int cols);
-bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols);
+bool tc_map_out16(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols);
 unsigned long long probe_wait_ns();
 
 // Whether one kernel does the whole separable interpolation from M to n.
 bool interp_fused_ok(int M, int n) { return M % 16 == 0 && M >= 16 && M <= huv_dev::kIfMaxM && n % 256 == 0 && M < n; }
 
-// Images of nc clips: P's planes [2][n][192] (map over 32-wide boxes of 128
-// rows), I_M / interp_scale(mean) as FP16 planes [nc][2][M][M].
-cudaError_t interp_fused(const CUtensorMap& map_p, const void* im_split, int M, int n, int nc, const float* mean,
+// Byte offset of P's element (row, column) of plane pl in the tiled operand
+// that the kernel streams, and the operand's size.
+size_t interp_tiled_offset(int row, int col, int pl, int M) {
+  const int nbox = huv_dev::if_boxes(M), r = row % 128, c = col % 32;
+  return ((static_cast<size_t>(row / 128) * nbox + col / 32) * 2 + pl) * huv_dev::kIfPBox + r * 64 +
+         ((c / 8) ^ ((r / 2) & 3)) * 16 + (c % 8) * 2;
+}
+size_t interp_tiled_bytes(int M, int n) {
+  return static_cast<size_t>(n / 128) * huv_dev::if_boxes(M) * 2 * huv_dev::kIfPBox;
+}
+
+// Images of nc clips: P as tiled by interp_tiled_offset, I_M /
+// interp_scale(mean) as FP16 planes [nc][2][M][M].
+cudaError_t interp_fused(const void* P, const void* im_split, int M, int n, int nc, const float* mean,
                          float* out, int* err, cudaStream_t st) {
   static std::atomic<uint64_t> smem_set{0};
   huv::once_per_device(smem_set, [] {
@@ -341,7 +358,7 @@ cudaError_t interp_fused(const CUtensorMap& map_p, const void* im_split, int M, 
   });
   CUtensorMap mi, mo;
   if (!tc_map_sw64_f16(&mi, im_split, static_cast<uint64_t>(nc) * 2 * M, M, M, M) ||
-      !tc_map_out(&mo, out, static_cast<uint64_t>(nc) * n, n))
+      !tc_map_out16(&mo, out, static_cast<uint64_t>(nc) * n, n))
     return cudaErrorInvalidValue;
   int sms = 0, dev = 0;
   cudaError_t e;
@@ -357,14 +374,15 @@ cudaError_t interp_fused(const CUtensorMap& map_p, const void* im_split, int M, 
   int split = 1;
   while (split < p.mt && static_cast<long long>(n / 256) * split * 2 * nc <= sms) split *= 2;
   p.mt_per = (p.mt + split - 1) / split;
+  p.P = static_cast<const uint8_t*>(P);
   p.mean = mean;
   p.err = err;
   p.probe_wait_ns = probe_wait_ns();
   const dim3 g(n / 256, (p.mt + p.mt_per - 1) / p.mt_per, nc);
   if (huv_dev::if_out_bufs(M) == 1)
-    pdl(huv_dev::tc_interp_fused<1>, g, 192, huv_dev::if_smem_bytes(M), st, map_p, mi, mo, p);
+    pdl(huv_dev::tc_interp_fused<1>, g, 32 * (2 + huv_dev::kIfEpiWarps), huv_dev::if_smem_bytes(M), st, mi, mo, p);
   else
-    pdl(huv_dev::tc_interp_fused<2>, g, 192, huv_dev::if_smem_bytes(M), st, map_p, mi, mo, p);
+    pdl(huv_dev::tc_interp_fused<2>, g, 32 * (2 + huv_dev::kIfEpiWarps), huv_dev::if_smem_bytes(M), st, mi, mo, p);
   return cudaGetLastError();
 }
 

@@ -31,6 +31,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <numeric>
 #include <vector>
 
 #include "../engine.hpp"
@@ -818,7 +819,9 @@ cudaError_t socs_field_fused(const float2* kband, const float2* Mband, int K, in
                              cudaStream_t st);
 unsigned long long probe_wait_ns() { return g_probe_wait_ns.load(std::memory_order_relaxed); }
 bool interp_fused_ok(int M, int n);
-cudaError_t interp_fused(const CUtensorMap& map_p, const void* im_split, int M, int n, int nc, const float* mean,
+size_t interp_tiled_offset(int row, int col, int pl, int M);
+size_t interp_tiled_bytes(int M, int n);
+cudaError_t interp_fused(const void* P, const void* im_split, int M, int n, int nc, const float* mean,
                          float* out, int* err, cudaStream_t st);
 bool xt_ok(int L, int hb);
 cudaError_t socs_rows_x(const float2* kband, float scale, const float2* Mband, int K, int hb, int L, int clips,
@@ -876,15 +879,16 @@ bool make_map_sw64(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int
 
 // 2-D f32 tensor map over [rows][cols] (row stride cols floats), 32 x 32
 // boxes with 128B swizzle: the TMA-store target of the interpolation GEMM.
-bool make_out_map(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) {
+// (`width` 16: 32 x 16 boxes with 64B swizzle)
+bool make_out_map(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols, int width = 32) {
   auto fn = encode_fn();
   if (!fn || (reinterpret_cast<uintptr_t>(ptr) & 15u) != 0 || (cols * 4) % 16 != 0) return false;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
-  cuuint32_t box[2] = {32, 32};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(width), 32};
   cuuint32_t estr[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+            width == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -977,6 +981,9 @@ bool tc_map_sw64_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, 
   return make_map_sw64(map, ptr, rows, kp, box_rows, cols, false);
 }
 bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) { return make_out_map(map, ptr, rows, cols); }
+bool tc_map_out16(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) {
+  return make_out_map(map, ptr, rows, cols, 16);
+}
 
 // f32 map over [rows][cols] with boxes of 8 columns x 32 rows, unswizzled.
 bool tc_map_out8(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols) {
@@ -1034,6 +1041,7 @@ void tc_release(huv::TcState& tc) {
   cudaFree(tc.gy);
   cudaFree(tc.gx);
   cudaFree(tc.gp);
+  cudaFree(tc.gpt);
   tc = huv::TcState();
 }
 
@@ -1351,19 +1359,39 @@ void Engine::interp_matrix(DeviceSet& ds, int M) {
   using namespace huv_launch;
   TcState& tc = ds.tc[M];
   const int h2 = 2 * ds.hb;
-  if (!tc.gp) {
+  const bool tiled = interp_fused_ok(M, n);  // which of the two operands the grid needs
+  if (tiled ? !tc.gpt : !tc.gp) {
     constexpr int kpP = 192;
-    std::vector<double> pm(static_cast<size_t>(n) * M);
+    // t = Y/N - m/M = q / (N M); sum_{|f|<=H} e^{2 pi i f t} = sin((2H+1) pi t) /
+    // sin(pi t), even in q, and q is a multiple of g = gcd(N, M): N M / g values
+    const int g = std::gcd(n, M), rows = n / g, cols = M / g;
     const double nm = static_cast<double>(n) * M;
-    for (int y = 0; y < n; ++y)
-      for (int m = 0; m < M; ++m) {
-        // t = Y/N - m/M = q / (N M); sum_{|f|<=H} e^{2 pi i f t} = sin((2H+1) pi t) / sin(pi t)
-        const long long q = static_cast<long long>(y) * M - static_cast<long long>(m) * n;
-        const double v = q == 0 ? static_cast<double>(2 * h2 + 1)
-                                : std::sin((2 * h2 + 1) * kPi * static_cast<double>(q) / nm) /
-                                      std::sin(kPi * static_cast<double>(q) / nm);
-        pm[static_cast<size_t>(y) * M + m] = v / M;
+    std::vector<double> val(static_cast<size_t>(rows) * M);
+    for (size_t j = 0; j < val.size(); ++j) {
+      const double q = static_cast<double>(j) * g;
+      val[j] = (j == 0 ? static_cast<double>(2 * h2 + 1) : std::sin((2 * h2 + 1) * kPi * q / nm) / std::sin(kPi * q / nm)) / M;
+    }
+    auto index = [&](int y, int m) { return static_cast<size_t>(std::abs(y * cols - m * rows)); };
+    if (tiled) {
+      std::vector<uint16_t> hi(val.size()), lo(val.size()), t(interp_tiled_bytes(M, n) / 2, 0);
+      for (size_t j = 0; j < val.size(); ++j) {
+        const float f = static_cast<float>(val[j]);
+        const __half h = __float2half_rn(f);
+        hi[j] = static_cast<__half_raw>(h).x;
+        lo[j] = static_cast<__half_raw>(__float2half_rn(f - __half2float(h))).x;
       }
+      for (int y = 0; y < n; ++y)
+        for (int m = 0; m < M; ++m) {
+          t[interp_tiled_offset(y, m, 0, M) / 2] = hi[index(y, m)];
+          t[interp_tiled_offset(y, m, 1, M) / 2] = lo[index(y, m)];
+        }
+      check_cuda(cudaMalloc(&tc.gpt, t.size() * 2), "cudaMalloc(P tiles)");
+      check_cuda(cudaMemcpy(tc.gpt, t.data(), t.size() * 2, cudaMemcpyHostToDevice), "upload P tiles");
+      return;
+    }
+    std::vector<double> pm(static_cast<size_t>(n) * M);
+    for (int y = 0; y < n; ++y)
+      for (int m = 0; m < M; ++m) pm[static_cast<size_t>(y) * M + m] = val[index(y, m)];
     const auto pp = split_planes_f16(pm, n, M, kpP);
     check_cuda(cudaMalloc(&tc.gp, pp.size() * 2), "cudaMalloc(P)");
     check_cuda(cudaMemcpy(tc.gp, pp.data(), pp.size() * 2, cudaMemcpyHostToDevice), "upload P");
@@ -1382,7 +1410,7 @@ void Engine::interp_separable(DeviceSet& ds, int M, int nc, const void* im_split
   TcState& tc = ds.tc[M];
   if (interp_fused_ok(M, n)) {
     if (profile) prof.begin("tc_interp_fused", st);
-    check_cuda(interp_fused(tc.map_pi32, im_split, M, n, nc, mean, o, dev_err, st), "tc_interp_fused");
+    check_cuda(interp_fused(tc.gpt, im_split, M, n, nc, mean, o, dev_err, st), "tc_interp_fused");
     if (profile) prof.end(st);
     return;
   }

@@ -471,9 +471,7 @@ Engine::BandKernels Engine::kernels_for(const huv_batch& b, DeviceSet& ds, int K
     if (div == 0.0) div = 1.0;
     if (fold_real_kernels(*ds.source, K, div, p)) {
       std::unique_ptr<float[]> h(new float[2 * p.size]);
-      parallel_for(static_cast<int64_t>(2 * p.size), [&](int64_t lo, int64_t hi) {
-        for (int64_t i = lo; i < hi; ++i) h[i] = static_cast<float>(p.v[i]);
-      });
+      for (size_t i = 0; i < 2 * p.size; ++i) h[i] = static_cast<float>(p.v[i]);
       check_cuda(cudaMalloc(&f.kband, sizeof(float2) * p.size), "cudaMalloc(folded kernels)");
       f.K = (K + 1) / 2;
       check_cuda(cudaMemcpy(f.kband, h.get(), sizeof(float2) * p.size, cudaMemcpyHostToDevice),

@@ -82,6 +82,7 @@ struct TcState {
   int lgm = 0;          // evaluation grid the state was built for (log2, rounded up)
   void* gy = nullptr;   // A_E planes [2][2M][kpE] bf16
   void* gx = nullptr;   // A_I planes [2][N][kpI] bf16
+  void* gpt = nullptr;  // the separable interpolation matrix as tc_interp_fused streams it
   void* gp = nullptr;   // separable interpolation matrix planes [2][N][192] fp16 (M <= 192)
   CUtensorMap map_ae, map_ai, map_pi;
   CUtensorMap map_ai32, map_pi32;  // the same planes in 32-wide boxes (64B swizzle)
