@@ -23,6 +23,7 @@
 
 #include "../../../include/huv_b200.h"
 #include "../engine.hpp"
+#include "fft_reg.cuh"
 
 namespace huv_launch {
 // tensor-core forward of the FNO (csrc/cuda/fno_tc.cu)
@@ -37,7 +38,8 @@ bool fno_tc_layer(int B, int S, int m, const __nv_bfloat16* v, const __nv_bfloat
                   int* err, cudaStream_t st);
 bool fno_tc_proj(int B, int S, const __nv_bfloat16* v, const __nv_bfloat16* Q1b, const float* b1, const float* q2,
                  const float* b2, float* out, int* err, cudaStream_t st);
-void fno_tc_to_bf16(const float* a, int n, __nv_bfloat16* b, cudaStream_t st);
+void fno_tc_weights(const float* W, size_t stride, int layers, int n, __nv_bfloat16* wb, const float* Q1, int nq,
+                    __nv_bfloat16* q1b, cudaStream_t st);
 void fno_tc_tw_table(const float2* twx, int S, int m, __nv_bfloat16* Tw, cudaStream_t st);
 // DFTs over the retained modes and the lift (csrc/cuda/fno_dft.cu)
 cudaError_t fno_dft_x_bf16(const __nv_bfloat16* in, int S, int m, const float2* twt, float2* out, int rows,
@@ -82,23 +84,43 @@ __device__ __forceinline__ void st_bf16x4(__nv_bfloat16* p, float a, float b, fl
 }
 
 // ------------------------------------------------------------ mode mixing
-// Y[b][j][kx][o] = sum_i X[b][j][kx][i] R[j][kx][i][o]; grid: (J*m, B), block C.
-__global__ void fno_mix(const float2* __restrict__ X, const float2* __restrict__ R, int C, int modes,
-                        float2* __restrict__ Y) {
-  extern __shared__ float2 sx[];
-  const int md = blockIdx.x, b = blockIdx.y;
-  const float2* xr = X + (static_cast<size_t>(b) * modes + md) * C;
-  for (int t = threadIdx.x; t < C; t += blockDim.x) sx[t] = xr[t];
-  __syncthreads();
+// Y[b][j][kx][o] = sum_i X[b][j][kx][i] R[j][kx][i][o], i ascending.  One block
+// per mode: R's 32 KB arrive by 16-byte cp.async once for every sample (a block
+// per mode and sample read them from L2 four at a time: 26 us for 16 samples,
+// 15 us for one).  grid: J m, block 256; dynamic shared memory [64][64] R,
+// [16][64] X (float2).
+__global__ void __launch_bounds__(256) fno_mix(const float2* __restrict__ X, const float2* __restrict__ R, int B,
+                                                int modes, float2* __restrict__ Y) {
+  constexpr int C = 64;
+  extern __shared__ __align__(16) float2 smx[];
+  float2* sR = smx;
+  float2* sx = smx + C * C;
+  const int md = blockIdx.x, t = threadIdx.x, o = t & 63, bq = t >> 6;
   const float2* rr = R + static_cast<size_t>(md) * C * C;
-  for (int o = threadIdx.x; o < C; o += blockDim.x) {
-    float re = 0.f, im = 0.f;
-    for (int i = 0; i < C; ++i) {
-      const float2 x = sx[i], w = rr[i * C + o];
-      re += x.x * w.x - x.y * w.y;
-      im += x.x * w.y + x.y * w.x;
+  // (the parameters are only known to be 8-byte aligned: R follows an odd
+  // number of floats for some layer counts)
+  const bool a16 = (reinterpret_cast<uintptr_t>(rr) & 15u) == 0;
+  if (a16)
+    for (int e = t; e < C * C / 2; e += 256) fr_cp_async16(sR + 2 * e, rr + 2 * e);
+  else
+    for (int e = t; e < C * C; e += 256) fr_cp_async8(sR + e, rr + e);
+  fr_cp_commit();
+  for (int b0 = 0; b0 < B; b0 += 16) {
+    const int nb = min(16, B - b0);
+    for (int e = t; e < nb * C; e += 256) sx[e] = X[(static_cast<size_t>(b0 + (e >> 6)) * modes + md) * C + (e & 63)];
+    if (b0 == 0) fr_cp_wait<0>();
+    __syncthreads();
+    for (int b = bq; b < nb; b += 4) {
+      float re = 0.f, im = 0.f;
+#pragma unroll 8
+      for (int i = 0; i < C; ++i) {
+        const float2 x = sx[b * C + i], w = sR[i * C + o];
+        re += x.x * w.x - x.y * w.y;
+        im += x.x * w.y + x.y * w.x;
+      }
+      Y[(static_cast<size_t>(b0 + b) * modes + md) * C + o] = make_float2(re, im);
     }
-    Y[(static_cast<size_t>(b) * modes + md) * C + o] = make_float2(re, im);
+    __syncthreads();
   }
 }
 
@@ -552,8 +574,9 @@ __global__ void __launch_bounds__(256) fno_proj_bwd(const __nv_bfloat16* __restr
   }
 }
 
-// MSE loss on [B][S][S]: dout = 2 (out - tgt) / n (and loss parts).
-__global__ void fno_mse(const float* __restrict__ out, const float* __restrict__ tgt, size_t n,
+// MSE loss on [B][S][S]: dout = 2 (out - tgt) / n (and loss parts).  One wide
+// block per SM: the blocks' atomics on the one sum take turns.
+__global__ void __launch_bounds__(1024) fno_mse(const float* __restrict__ out, const float* __restrict__ tgt, size_t n,
                         float* __restrict__ dout, float* __restrict__ loss) {
   __shared__ float red[32];
   float s = 0.f;
@@ -783,14 +806,14 @@ struct Fno {
     const int rows = B * S;
     const dim3 rgrid(std::min(rows, 4096));
     using namespace huv_launch;
+    if (tc) fno_tc_weights(par + oW[0], L > 1 ? oW[1] - oW[0] : 0, L, C * C, wb, par + oQ1, P * C, q1b, st);
     check_cuda(fno_lift_fwd(masks, B, S, par + oWl, par + obl, v[0], st), "fno lift");
     for (int l = 0; l < L; ++l) {
       check_cuda(fno_dft_x_bf16(v[l], S, m, twt, Xa, rows, st), "fno dft x");
       check_cuda(fno_dft_y(Xa, B, S, m, tyt, Xl[l], st), "fno dft y");
-      fno_mix<<<dim3(modes, B), C, C * 8, st>>>(Xl[l], reinterpret_cast<const float2*>(par + oR[l]), C, modes, Y);
+      fno_mix<<<modes, 256, (C * C + 16 * C) * 8, st>>>(Xl[l], reinterpret_cast<const float2*>(par + oR[l]), B, modes, Y);
       check_cuda(fno_idft_y(Y, B, S, m, tyt, Za, tc ? zs : nullptr, st), "fno inverse dft y");
       if (tc) {
-        fno_tc_to_bf16(par + oW[l], C * C, wb + static_cast<size_t>(l) * C * C, st);
         if (!fno_tc_layer(B, S, m, v[l], wb + static_cast<size_t>(l) * C * C, tw_tab, zs, par + ob[l],
                           l < L - 1 ? 1 : 0, keep ? z[l] : nullptr, v[l + 1], tc_err, st))
           throw Error(HUV_ERR_CUDA, "fno: tensor-core layer launch failed");
@@ -800,7 +823,6 @@ struct Fno {
       }
     }
     if (tc) {
-      huv_launch::fno_tc_to_bf16(par + oQ1, P * C, q1b, st);
       if (!huv_launch::fno_tc_proj(B, S, v[L], q1b, par + ob1, par + oQ2, par + ob2, images ? images : out, tc_err, st))
         throw Error(HUV_ERR_CUDA, "fno: tensor-core projection launch failed");
     } else {
@@ -868,7 +890,7 @@ struct Fno {
     using namespace huv_dev;
     const size_t pix = static_cast<size_t>(B) * S * S;
     check_cuda(cudaMemsetAsync(loss, 0, 4, st), "memset loss");
-    fno_mse<<<1184, 256, 0, st>>>(out, targets, pix, dout, loss);
+    fno_mse<<<148, 1024, 0, st>>>(out, targets, pix, dout, loss);
     float h = 0;
     check_cuda(cudaMemcpyAsync(&h, loss, 4, cudaMemcpyDeviceToHost, st), "D2H loss");
     check_cuda(cudaStreamSynchronize(st), "sync");

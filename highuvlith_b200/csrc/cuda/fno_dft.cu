@@ -252,15 +252,16 @@ __global__ void __launch_bounds__(128) fno_dft_y_fwd(const float2* __restrict__ 
 // run of rows y whose twiddles sit in shared memory.  Bound by FP32 issue and
 // the packed stores; the kernel it replaces re-read the modes and twiddles
 // from global memory for every row, and the packing was a pass of its own:
-// 16 x 512^2: 0.425 + 0.095 -> 0.102 ms.
+// 16 x 512^2: 0.425 + 0.095 -> 0.102 ms.  `run` rows per block: 32, or 8 where
+// that would leave SMs without a block.
 constexpr int kDyRows = 32;
 template <bool PACK>
 __global__ void __launch_bounds__(128) fno_dft_y_inv(const float2* __restrict__ in, int S, int m,
-                                                      const float2* __restrict__ tyt, float2* __restrict__ Z,
-                                                      __nv_bfloat16* __restrict__ Zs) {
+                                                      const float2* __restrict__ tyt, int run,
+                                                      float2* __restrict__ Z, __nv_bfloat16* __restrict__ Zs) {
   __shared__ __align__(16) float2 sw[kDyRows][32];
-  const int t = threadIdx.x, b = blockIdx.z, y0 = blockIdx.y * kDyRows;
-  const int J = 2 * m, mC = m * 64, ny = min(kDyRows, S - y0);
+  const int t = threadIdx.x, b = blockIdx.z, y0 = blockIdx.y * run;
+  const int J = 2 * m, mC = m * 64, ny = min(run, S - y0);
   const int kx = PACK ? (t & 15) : 0, c = PACK ? blockIdx.x * 8 + (t >> 4) : 0;
   const int col = PACK ? kx * 64 + c : blockIdx.x * 128 + t;
   const bool live = PACK ? kx < m : col < mC;
@@ -338,7 +339,8 @@ __global__ void __launch_bounds__(256) fno_lift(const float* __restrict__ a, int
 // multiply-add per term).  Tiles of 64 pixels through shared memory: loaded
 // with 16-byte accesses, summed over pixels by (channel, quarter of the tile)
 // and over channels by pixel.  Bound by dv0's 256 bytes per pixel (a strided
-// load per channel before: 8 x 512^2: 0.98 -> 0.11 ms).
+// load per channel before: 8 x 512^2: 0.98 -> 0.11 ms).  Two blocks per SM:
+// their atomics on the 256 sums take turns.
 __global__ void __launch_bounds__(256) fno_lift_bwd(const float* __restrict__ a, const float* __restrict__ dv0, int S,
                                                      const float* __restrict__ Wl, int pixels,
                                                      float* __restrict__ dWl, float* __restrict__ dbl,
@@ -447,11 +449,12 @@ cudaError_t fno_dft_y(const float2* in, int B, int S, int m, const float2* tyt, 
 // Z (float2, [b][y][kx][c]) or, with Zs, the packed BF16 operand of the tensor-core layer.
 cudaError_t fno_idft_y(const float2* in, int B, int S, int m, const float2* tyt, float2* Z, __nv_bfloat16* Zs,
                        cudaStream_t st) {
-  const unsigned ry = (S + kDyRows - 1) / kDyRows;
+  const int run = static_cast<long long>(8) * ((S + kDyRows - 1) / kDyRows) * B >= 148 ? kDyRows : 8;
+  const unsigned ry = (S + run - 1) / run;
   if (Zs)
-    fno_dft_y_inv<true><<<dim3(8, ry, B), 128, 0, st>>>(in, S, m, tyt, nullptr, Zs);
+    fno_dft_y_inv<true><<<dim3(8, ry, B), 128, 0, st>>>(in, S, m, tyt, run, nullptr, Zs);
   else
-    fno_dft_y_inv<false><<<dim3((m * 64 + 127) / 128, ry, B), 128, 0, st>>>(in, S, m, tyt, Z, nullptr);
+    fno_dft_y_inv<false><<<dim3((m * 64 + 127) / 128, ry, B), 128, 0, st>>>(in, S, m, tyt, run, Z, nullptr);
   return cudaGetLastError();
 }
 cudaError_t fno_lift_fwd(const float* a, int B, int S, const float* Wl, const float* bl, __nv_bfloat16* v,
@@ -464,7 +467,7 @@ cudaError_t fno_lift_fwd(const float* a, int B, int S, const float* Wl, const fl
 cudaError_t fno_lift_back(const float* a, const float* dv0, int B, int S, const float* Wl, float* dWl, float* dbl,
                           float* da, cudaStream_t st) {
   const size_t pix = static_cast<size_t>(B) * S * S;
-  fno_lift_bwd<<<static_cast<unsigned>(std::min<size_t>(pix / 64, 148 * 6)), 256, 0, st>>>(
+  fno_lift_bwd<<<static_cast<unsigned>(std::min<size_t>(pix / 64, 148 * 2)), 256, 0, st>>>(
       a, dv0, S, Wl, static_cast<int>(pix), dWl, dbl, da);
   return cudaGetLastError();
 }

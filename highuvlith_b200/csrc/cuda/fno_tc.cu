@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(32 * (2 + kFnoEpiWarps), 2)
 //
 // What bounds it: 1 KB per pixel, and GELU' (erff and expf).  With one pixel
 // per lane (32 rows of 16 bytes per access) and operands transposed by 2-byte
-// stores it was bound by L1 (87 %), 0.66 ms at 8 x 512^2; now 0.43 ms.
+// stores it was bound by L1 (87 %), 0.66 ms at 8 x 512^2; now 0.36 ms.
 constexpr int kBwdXWarps = 8;                       // elementwise warps
 constexpr int kBwdThreads = 32 * (6 + kBwdXWarps);  // MMA + TMA + 4 epilogue + elementwise
 constexpr uint32_t kBwdStage = 2 * 16384;           // dz [128 px][64 o], v [128 px][64 i]
@@ -460,6 +460,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ float sdb[kBwdXWarps * 64];
   constexpr uint32_t kTmemCols = 256;  // dv accumulators at 0 / 64, dW at 128
 
   if (threadIdx.x == 0) {
@@ -584,13 +585,23 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
       if (fin && !*abort_flag) {
         tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + 128;
-        float* w = p.dW + (quad * 32 + lane) * 64;
+        // through the staging tiles, so that a warp's atomics cover 128
+        // consecutive bytes (a row per lane: 8 times the L2 operations, 0.1 ms
+        // of every launch for 296 CTAs)
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           float a[32];
           tmem_ld32(taddr + 32 * h, a);
+          uint8_t* o = st + h * kBwdOut;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) atomicAdd(w + 32 * h + i, a[i]);
+          for (int q = 0; q < 8; ++q)
+            *reinterpret_cast<float4*>(o + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+          __syncwarp();
+          float* w = p.dW + quad * 32 * 64 + 32 * h + lane;
+#pragma unroll 8
+          for (int r = 0; r < 32; ++r)
+            atomicAdd(w + r * 64, *reinterpret_cast<const float*>(o + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4));
         }
       } else if (!fin && lane == 0) {
         fail(34);
@@ -656,14 +667,22 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[s]);
     }
-    if (!*abort_flag) {
+    // db: the CTA's warps first, then one atomic per channel (atomics on one
+    // address take about 40 ns each: with one per warp they were 0.1 ms of a
+    // launch of 296 CTAs)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        float x = dbp[e];
-        x += __shfl_xor_sync(0xffffffffu, x, 8);
-        x += __shfl_xor_sync(0xffffffffu, x, 16);
-        if (lane < 8) atomicAdd(p.db + o0 + e, x);
-      }
+    for (int e = 0; e < 8; ++e) {
+      float x = dbp[e];
+      x += __shfl_xor_sync(0xffffffffu, x, 8);
+      x += __shfl_xor_sync(0xffffffffu, x, 16);
+      if (lane < 8) sdb[xw * 64 + o0 + e] = x;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kBwdXWarps) : "memory");
+    if (xt < 64 && !*abort_flag) {
+      float x = 0.f;
+#pragma unroll
+      for (int w = 0; w < kBwdXWarps; ++w) x += sdb[w * 64 + xt];
+      atomicAdd(p.db + xt, x);
     }
   }
   tc_fence_before();
@@ -688,12 +707,13 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
 // tensor memory over all tiles of the CTA and are added to global memory once.
 // Two CTAs per SM, persistent: one's GEMMs run under the other's elementwise
 // part, which bounds it (erff and expf for 128 hidden units per pixel):
-// 8 x 512^2: 0.87 -> 0.60 ms against one CTA with operands transposed by
+// 8 x 512^2: 0.87 -> 0.57 ms against one CTA with operands transposed by
 // 2-byte stores and dv stored one pixel per lane.
 constexpr int kPbThreads = 320;
 constexpr uint32_t kPbQ1 = 0, kPbOnes = 16384, kPbV = 20480, kPbDH = 36864, kPbG = 69632, kPbOut = 102400,
                    kPbVec = 110592, kPbBars = 111616;
 constexpr size_t kPbSmem = 1024 + kPbBars + 128;
+static_assert(10 * 8 + 4 * 4 <= 128, "barriers, slot, flag and four sums");
 static_assert(2 * (kPbSmem + 1024) <= 228 * 1024, "fno_tc_proj_bwd: two CTAs per SM");
 
 struct FnoProjBwdParams {
@@ -727,6 +747,7 @@ __global__ void __launch_bounds__(kPbThreads, 2)
   uint64_t* done = bars + 7;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* sd2 = reinterpret_cast<float*>(tmem_slot + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr uint32_t kTmemCols = 256;
   constexpr uint32_t cH = 0, cDV = 0, cQ = 128, cB = 192, cG = 208;  // accumulator columns
@@ -930,8 +951,18 @@ __global__ void __launch_bounds__(kPbThreads, 2)
       const int j = quad * 32 + lane;
       float a[32];
       tmem_ld32(tmem_base + lrow + cQ + half * 32, a);
+      // eight columns at a time through the staging tile: whole sectors per atomic
+      float* sf = reinterpret_cast<float*>(so);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) atomicAdd(p.dQ1 + j * 64 + half * 32 + i, a[i]);
+      for (int q = 0; q < 4; ++q) {
+        __syncwarp();
+        *reinterpret_cast<float4*>(sf + lane * 8) = make_float4(a[8 * q], a[8 * q + 1], a[8 * q + 2], a[8 * q + 3]);
+        *reinterpret_cast<float4*>(sf + lane * 8 + 4) = make_float4(a[8 * q + 4], a[8 * q + 5], a[8 * q + 6], a[8 * q + 7]);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          atomicAdd(p.dQ1 + (quad * 32 + 4 * r + (lane >> 3)) * 64 + half * 32 + 8 * q + (lane & 7), sf[32 * r + lane]);
+      }
       if (half == 0) {
         float b[16], g[16];
         tmem_ld16(tmem_base + lrow + cB, b);
@@ -940,7 +971,9 @@ __global__ void __launch_bounds__(kPbThreads, 2)
         atomicAdd(p.dQ2 + j, g[0]);
 #pragma unroll
         for (int sh = 16; sh > 0; sh >>= 1) gd2 += __shfl_xor_sync(0xffffffffu, gd2, sh);
-        if (lane == 0) atomicAdd(p.db2, gd2);
+        if (lane == 0) sd2[quad] = gd2;
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        if (quad == 0 && lane == 0) atomicAdd(p.db2, (sd2[0] + sd2[1]) + (sd2[2] + sd2[3]));
       }
     } else if (!fin && lane == 0) {
       fail(47);
@@ -952,10 +985,17 @@ __global__ void __launch_bounds__(kPbThreads, 2)
   if (warp == 0) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-// bf16 copy of an fp32 matrix (weights for the tensor-core operands).
-__global__ void fno_to_bf16(const float* __restrict__ a, int n, __nv_bfloat16* __restrict__ b) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    b[i] = __float2bfloat16_rn(a[i]);
+// bf16 copies of a forward's weights, one launch for all of them (one per
+// matrix before): the layers' matrices W (n values each, `stride` apart) into
+// wb, then Q1 (nq values) into q1b.  grid: (blocks, layers + 1).
+__global__ void __launch_bounds__(256) fno_to_bf16(const float* __restrict__ W, size_t stride, int layers, int n,
+                                                    __nv_bfloat16* __restrict__ wb, const float* __restrict__ Q1, int nq,
+                                                    __nv_bfloat16* __restrict__ q1b) {
+  const int l = blockIdx.y;
+  const float* a = l < layers ? W + l * stride : Q1;
+  __nv_bfloat16* b = l < layers ? wb + static_cast<size_t>(l) * n : q1b;
+  const int m = l < layers ? n : nq;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < m; i += gridDim.x * 256) b[i] = __float2bfloat16_rn(a[i]);
 }
 
 // Tw[x][kk] (bf16, kk < 32): cos / sin of 2 pi kx x / S for kk = 2 kx / 2 kx + 1
@@ -1089,8 +1129,9 @@ bool fno_tc_proj_bwd(size_t pix, const __nv_bfloat16* v, const float* Q1, const 
   huv_dev::fno_tc_proj_bwd<<<grid, huv_dev::kPbThreads, huv_dev::kPbSmem, st>>>(mv, mo, p);
   return cudaGetLastError() == cudaSuccess;
 }
-void fno_tc_to_bf16(const float* a, int n, __nv_bfloat16* b, cudaStream_t st) {
-  huv_dev::fno_to_bf16<<<(n + 255) / 256, 256, 0, st>>>(a, n, b);
+void fno_tc_weights(const float* W, size_t stride, int layers, int n, __nv_bfloat16* wb, const float* Q1, int nq,
+                    __nv_bfloat16* q1b, cudaStream_t st) {
+  huv_dev::fno_to_bf16<<<dim3(8, layers + 1), 256, 0, st>>>(W, stride, layers, n, wb, Q1, nq, q1b);
 }
 void fno_tc_tw_table(const float2* twx, int S, int m, __nv_bfloat16* Tw, cudaStream_t st) {
   huv_dev::fno_tw_table<<<(S * 32 + 255) / 256, 256, 0, st>>>(twx, S, m, Tw);
