@@ -768,18 +768,6 @@ __global__ void max_parts(const double* __restrict__ parts, int nparts, int mask
   out[m] = r;
 }
 
-// y[mask] = alpha[mask] * x[mask] + gamma[mask] * y[mask]   (per-mask scalars)
-__global__ void batched_axpby(const float* __restrict__ x, float* __restrict__ y, size_t n,
-                              const float* __restrict__ alpha, const float* __restrict__ gamma,
-                              float* __restrict__ out) {
-  pdl_begin();
-  const int mask = blockIdx.y;
-  const float al = alpha[mask], ga = gamma[mask];
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x)
-    out[mask * n + i] = al * x[mask * n + i] + ga * y[mask * n + i];
-}
-
 __global__ void scale_inplace(float* __restrict__ x, size_t n, float s) {
   pdl_begin();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;

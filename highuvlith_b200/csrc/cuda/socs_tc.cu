@@ -1020,9 +1020,6 @@ cudaError_t tc_set_smem() {
   if ((e = cudaFuncSetAttribute(tc_dft_gemm<3, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(tc_smem_bytes(2, 64, false, false, tc_stages(3, 64))))))
     return e;
-  if ((e = cudaFuncSetAttribute(tc_dft_gemm<3, 80>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(tc_smem_bytes(3, 80, false, false, tc_stages(3, 80))))))
-    return e;
   if ((e = cudaFuncSetAttribute(tc_dft_gemm<3, 96>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(tc_smem_bytes(3, 96, false, false, tc_stages(3, 96))))))
     return e;
@@ -1431,8 +1428,10 @@ void Engine::interp_separable(DeviceSet& ds, int M, int nc, const void* im_split
     // Z^T[clip][plane][Y][y] = sum_x P(Y, x) I_M(y, x) / s, FP16 split planes:
     // A = P (rows Y), B = I_M / s (rows y, K = x), s = interp_scale(mean);
     // G1 clips per CTA share the A tile.  Each CTA takes half of the M
-    // columns (N = M / 2), so that two clips' B tiles fit the ring
-    // (tc_stages: 7 / 6 / 5 stages at M = 128 / 160 / 192).
+    // columns (N = M / 2), so that two clips' B tiles fit the ring (tc_stages:
+    // 7 / 5 stages at M = 128 / 192).  The grids left on this path: 192, which
+    // does not fit tc_interp_fused's shared memory, and 128 at n = 128, where
+    // the rows are not a multiple of its 256-wide tiles.
     const int bn1 = M / 2;
     const int ntile1 = M / bn1, mtiles = n / 128;
     // Clips per CTA: the fewest (up to 32) whose grid fits one wave of one
@@ -1475,9 +1474,6 @@ void Engine::interp_separable(DeviceSet& ds, int M, int nc, const void* im_split
     if (bn1 == 64)
       tc_dft_gemm<3, 64><<<g, 192, tc_smem_bytes(p.kboxes, 64, false, false, tc_stages(3, 64)), st>>>(
           tc.map_pi, mbS, tc.map_pi, p);
-    else if (bn1 == 80)
-      tc_dft_gemm<3, 80><<<g, 192, tc_smem_bytes(p.kboxes, 80, false, false, tc_stages(3, 80)), st>>>(
-          tc.map_pi, mbS, tc.map_pi, p);
     else if (bn1 == 96)
       tc_dft_gemm<3, 96><<<g, 192, tc_smem_bytes(p.kboxes, 96, false, false, tc_stages(3, 96)), st>>>(
           tc.map_pi, mbS, tc.map_pi, p);
@@ -1509,16 +1505,12 @@ void Engine::interp_separable(DeviceSet& ds, int M, int nc, const void* im_split
   dim3 g(1, n / 128, nc);
   CUtensorMap mbZ64;
   const int abox = (p.ksteps + 1) / 2;  // 32-wide A boxes
-  const bool w256 = p.out_tma && n % 256 == 0 && abox <= 6 &&
-                    make_map_sw64(&mbZ64, BI, static_cast<uint64_t>(nc) * 2 * n, M, 256, M, true);
+  const bool w256 = p.out_tma && n % 256 == 0 && make_map_sw64(&mbZ64, BI, static_cast<uint64_t>(nc) * 2 * n, M, 256, M, true);
   prof.begin("tc_dft_gemm<interp>", st);
   if (w256) {  // 128 x 256 tiles, A and B through 32-wide boxes
     p.G = n / 256;
     p.kboxes = abox;
-    if (abox <= 5)
-      tc_interp_w256<5, 7, 2><<<g, 192, w256_smem_bytes(5, 7, 2), st>>>(tc.map_pi32, mbZ64, mo, p);
-    else
-      tc_interp_w256<6, 6, 2><<<g, 192, w256_smem_bytes(6, 6, 2), st>>>(tc.map_pi32, mbZ64, mo, p);
+    tc_interp_w256<6, 6, 2><<<g, 192, w256_smem_bytes(6, 6, 2), st>>>(tc.map_pi32, mbZ64, mo, p);
   } else {
     tc_dft_gemm<1><<<g, 192, tc_smem_bytes(3, kTcBN, false, true), st>>>(tc.map_pi, mbZ, mo, p);
   }
