@@ -29,7 +29,6 @@
 
 #include "../engine.hpp"
 #include "fft_reg.cuh"
-#include "pdl.cuh"
 
 namespace huv_dev {
 
@@ -83,7 +82,6 @@ template <int M>
 __global__ void __launch_bounds__(fs_threads(M))
     socs_field_small(const __grid_constant__ SmallPlanes pl, const float2* __restrict__ Mband, int hb, int clips,
                      const float2* __restrict__ tw, float* __restrict__ mean, __half* __restrict__ split) {
-  pdl_begin();
   constexpr int R = M / 16, KB = fs_kb(M), T = fs_work(M), NT = fs_threads(M);
   constexpr int SR = KB * M / 2, SC = KB * M;           // row and column sequences
   constexpr int NR = R > 1 ? (16 * SR + T - 1) / T : 1;  // last-pass butterflies per thread, rows
@@ -270,7 +268,6 @@ __global__ void __launch_bounds__(fs_threads(M))
     ilt_adj_small(const float2* __restrict__ kband, const float2* __restrict__ Mband, const float* __restrict__ G, int K,
                   int hb, float keep, const double* __restrict__ sums, float flare_over_n,
                   const float2* __restrict__ tw, float2* __restrict__ Q) {
-  pdl_begin();
   constexpr int R = M / 16, KB = fs_kb(M), T = fs_work(M), NT = fs_threads(M);
   constexpr int SR = KB * M / 2, SC = KB * M;
   constexpr int NR = R > 1 ? (16 * SR + T - 1) / T : 1;
@@ -527,14 +524,12 @@ cudaError_t launch_small(const huv_dev::SmallPlanes& pl, int planes, int split, 
   cfg.blockDim = dim3(huv_dev::fs_threads(M));
   cfg.dynamicSmemBytes = huv_dev::fs_smem(M, 2 * hb + 1);
   cfg.stream = st;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = split;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_ok(cfg.gridDim, st) ? 2 : 1;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, huv_dev::socs_field_small<M>, pl, Mband, hb, clips, tw, mean,
                             static_cast<__half*>(out));
 }
@@ -554,14 +549,12 @@ cudaError_t launch_adj(const float2* kband, const float2* Mband, const float* G,
   cfg.blockDim = dim3(huv_dev::fs_threads(M));
   cfg.dynamicSmemBytes = smem(2 * hb + 1);
   cfg.stream = st;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = split;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_ok(cfg.gridDim, st) ? 2 : 1;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, huv_dev::ilt_adj_small<M>, kband, Mband, G, K, hb, keep, sums, flare_over_n, tw, Q);
 }
 }  // namespace

@@ -21,7 +21,6 @@
 #include "../engine.hpp"
 #include "fft_block.cuh"
 #include "fft_reg.cuh"
-#include "pdl.cuh"
 
 namespace huv_dev {
 
@@ -29,7 +28,6 @@ namespace huv_dev {
 // t = a + (1 - a) sigmoid(beta theta) (the transmittance fed to the band FFT).
 __global__ void ilt_transmittance(const float* __restrict__ theta, size_t n, float beta, float absorber,
                                   float* __restrict__ t) {
-  pdl_begin();
   // float4 body when both arrays are 16-byte aligned, scalar tail
   const bool vec = ((reinterpret_cast<uintptr_t>(theta) | reinterpret_cast<uintptr_t>(t)) & 15u) == 0;
   const size_t n4 = vec ? n / 4 : 0;
@@ -62,7 +60,6 @@ __device__ __forceinline__ double block_sum_double(double v, double* red) {
 __global__ void ilt_data(const float* __restrict__ img, const float* __restrict__ target, size_t npix,
                          int kind, float thr, float steep, float dose, float* __restrict__ G,
                          double* __restrict__ parts) {
-  pdl_begin();
   __shared__ double red[32];
   const int mask = blockIdx.y;
   const float* im = img + mask * npix;
@@ -120,7 +117,6 @@ __global__ void ilt_data(const float* __restrict__ img, const float* __restrict_
 // 64 masks of 256 parts, 4 now).
 __global__ void __launch_bounds__(128) sum_parts(const double* __restrict__ parts, int nparts, int ncomp, int masks,
                                                   double* __restrict__ out) {
-  pdl_begin();
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= masks * ncomp) return;
   const int mask = t / ncomp, c = t % ncomp;
@@ -136,7 +132,6 @@ __global__ void __launch_bounds__(128) sum_parts(const double* __restrict__ part
 // separable interpolation's operand (csrc/cuda/interp_tc.cu).  grid: masks.
 __global__ void __launch_bounds__(1024) split_signed(const float* __restrict__ v, int n, float* __restrict__ mean,
                                                       __half* __restrict__ planes) {
-  pdl_begin();
   __shared__ float red[32];
   const float* x = v + static_cast<size_t>(blockIdx.x) * n;
   float m = 0.f;
@@ -166,7 +161,6 @@ __global__ void __launch_bounds__(1024) split_signed(const float* __restrict__ v
 __global__ void ilt_cols_adj(const float2* __restrict__ T, const float* __restrict__ G, int K, int hb, int lg,
                              int Wc, float keep, const double* __restrict__ sums, float flare_over_n,
                              float2* __restrict__ V, const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   const int L = 1 << lg;
   const int B = 2 * hb + 1;
@@ -220,7 +214,6 @@ __global__ void __launch_bounds__(fr_threads(L, S), (L == 160 || L == 192) ? 3 :
     ilt_cols_adj_xt(const float2* __restrict__ Tt, const float* __restrict__ G, int K, int hb, float keep,
                     const double* __restrict__ sums, float flare_over_n, float2* __restrict__ V,
                     const float2* __restrict__ tw) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L);
   constexpr int R = fr_radix(L, NP - 1);
   extern __shared__ float2 smem[];
@@ -318,7 +311,6 @@ __global__ void __launch_bounds__(fr_threads(L, S), (L == 160 || L == 192) ? 3 :
 // In place: Q <- its Hermitian part (Q(f) + conj(Q(-f))) / 2 on each mask's
 // B x B band, so that IFFT(Q) is real and equals Re IFFT of the original.
 __global__ void hermitian_part(float2* __restrict__ Q, int B, int masks) {
-  pdl_begin();
   const int half = (B * B + 1) / 2;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < half * masks; e += gridDim.x * blockDim.x) {
     const int mask = e / half, i = e - mask * half;
@@ -341,7 +333,6 @@ template <int L, int S>
 __global__ void __launch_bounds__(fr_threads(L, S), (L == 160 || L == 192) ? 3 : 1)
     ilt_rows_adj_xt(const float2* __restrict__ V, const float2* __restrict__ kband, int K, int hb,
                     float2* __restrict__ Q, const float2* __restrict__ tw) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L);
   constexpr int R = fr_radix(L, NP - 1);
   constexpr int NB = fr_per(L, S, NP - 1);
@@ -436,7 +427,6 @@ __global__ void __launch_bounds__(fr_threads(L, S), (L == 160 || L == 192) ? 3 :
 // grid: (B, masks).
 __global__ void ilt_rows_adj(const float2* __restrict__ V, const float2* __restrict__ kband, int K, int hb, int lg,
                              int S, float2* __restrict__ Q, const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   const int L = 1 << lg;
   const int B = 2 * hb + 1;
@@ -474,7 +464,6 @@ __global__ void ilt_rows_adj(const float2* __restrict__ V, const float2* __restr
 __global__ void ilt_finish(const float* __restrict__ theta, const float* __restrict__ dcdm, int n, float beta,
                            float tv_w, float tv_eps, float bin_w, float* __restrict__ grad,
                            double* __restrict__ parts) {
-  pdl_begin();
   __shared__ double red[32];
   const int mask = blockIdx.y;
   const size_t npix = static_cast<size_t>(n) * n;
@@ -529,7 +518,6 @@ __global__ void __launch_bounds__(256, 4) ilt_finish_tiled(const float* __restri
                                                          const float* __restrict__ dcdm, int n, float beta,
                                                          float tv_w, float tv_eps, float bin_w,
                                                          float* __restrict__ grad, double* __restrict__ parts) {
-  pdl_begin();
   static_assert(TS % 4 == 0 && (TS * TS) % 1024 == 0, "tiles of whole 4-pixel runs, 256 threads");
   constexpr int NE = (TS + 2) * (TS + 2), NQ = (NE + 255) / 256;
   constexpr int RUNS = TS / 4;               // 4-pixel runs per row
@@ -623,7 +611,6 @@ __global__ void __launch_bounds__(256, 4) ilt_finish_tiled(const float* __restri
 __global__ void __launch_bounds__(256, 3)
     ilt_finish_4x4(const float* __restrict__ theta, const float* __restrict__ dcdm, int n, float beta, float tv_w,
                    float tv_eps, float bin_w, float* __restrict__ grad, double* __restrict__ parts) {
-  pdl_begin();
   constexpr int TS = 64, LD = 72, C0 = 4;  // column j of the tile at C0 + j: whole 16-byte runs
   __shared__ __align__(16) float sm[TS + 2][LD];
   __shared__ double red[32];
@@ -730,7 +717,6 @@ __global__ void __launch_bounds__(256, 3)
 // Per-mask reductions over n elements: out[mask] = sum a*b (dot) or max |a|.
 __global__ void batched_dot(const float* __restrict__ a, const float* __restrict__ b, size_t n,
                             double* __restrict__ parts) {
-  pdl_begin();
   __shared__ double red[32];
   const int mask = blockIdx.y;
   double s = 0.0;
@@ -742,7 +728,6 @@ __global__ void batched_dot(const float* __restrict__ a, const float* __restrict
 }
 
 __global__ void batched_maxabs(const float* __restrict__ a, size_t n, double* __restrict__ parts) {
-  pdl_begin();
   __shared__ double red[32];
   const int mask = blockIdx.y;
   float m = 0.f;
@@ -760,7 +745,6 @@ __global__ void batched_maxabs(const float* __restrict__ a, size_t n, double* __
 }
 
 __global__ void max_parts(const double* __restrict__ parts, int nparts, int masks, double* __restrict__ out) {
-  pdl_begin();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= masks) return;
   double r = 0.0;
@@ -769,7 +753,6 @@ __global__ void max_parts(const double* __restrict__ parts, int nparts, int mask
 }
 
 __global__ void scale_inplace(float* __restrict__ x, size_t n, float s) {
-  pdl_begin();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x)
     x[i] *= s;
@@ -778,7 +761,6 @@ __global__ void scale_inplace(float* __restrict__ x, size_t n, float s) {
 // parts[mask][block] = (max |a - b|, max |b|)
 __global__ void err_parts(const float* __restrict__ a, const float* __restrict__ b, size_t n,
                           double* __restrict__ parts) {
-  pdl_begin();
   __shared__ float re[32], rb[32];
   const int mask = blockIdx.y;
   float e = 0.f, m = 0.f;
@@ -811,7 +793,6 @@ __global__ void err_parts(const float* __restrict__ a, const float* __restrict__
 // cost[c] = weight * (sum r^2) / npix + reg[c]
 __global__ void ilt_combine(const double* __restrict__ data, const double* __restrict__ reg, int masks, double w,
                             double inv_npix, double* __restrict__ cost) {
-  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < masks) cost[c] = w * data[2 * c] * inv_npix + reg[c];
 }
@@ -820,7 +801,6 @@ __global__ void ilt_combine(const double* __restrict__ data, const double* __res
 __global__ void gather_axpby(const int* __restrict__ idx, const float* __restrict__ alpha,
                              const float* __restrict__ gamma, const float* __restrict__ x,
                              const float* __restrict__ y, size_t n, float* __restrict__ out) {
-  pdl_begin();
   const int j = blockIdx.y;
   const size_t m = static_cast<size_t>(idx[j]);
   const float al = alpha[j], ga = gamma[j];
@@ -835,7 +815,6 @@ __global__ void gather_axpby(const int* __restrict__ idx, const float* __restric
 // dst[idx[j]] = src[j]   (blocks of n floats)
 __global__ void scatter_blocks(const int* __restrict__ idx, const float* __restrict__ src, size_t n,
                                float* __restrict__ dst) {
-  pdl_begin();
   const int j = blockIdx.y;
   const size_t m = static_cast<size_t>(idx[j]);
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
@@ -904,8 +883,6 @@ size_t ilt_adj_xt_smem(int L, int hb) {
 }  // namespace huv_launch
 
 namespace huv {
-
-using huv_launch::pdl;
 
 namespace {
 size_t a256(size_t v) { return (v + 255) & ~size_t(255); }
@@ -1017,7 +994,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
     const int nc = std::min(chunk, masks - c0);
     const float* th = theta + npix * c0;
     const float* tg = target + npix * c0;
-    pdl(ilt_transmittance, 1184, 256, 0, st, th, npix * nc, static_cast<float>(p.beta),
+    ilt_transmittance<<<1184, 256, 0, st>>>(th, npix * nc, static_cast<float>(p.beta),
                                             static_cast<float>(p.absorber), tbuf);
     check_cuda(band_forward(tbuf, HUV_INPUT_RASTER_F32, n, lgn, hb, nc, X, Mb, nullptr, ds.W, mean, twn, st, nullptr, nullptr, true),
                "ilt band_forward");
@@ -1050,10 +1027,10 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       check_cuda(socs_rows_x(nullptr, scale, C, 1, h2, n, nc, X2, twn, st), "ilt interp rows");
       check_cuda(socs_cols_x(X2, 1, h2, n, nc, 1.f, 0.f, nullptr, img, 1, twn, st), "ilt interp cols");
     }
-    pdl(ilt_data, dim3(kRedBlocks, nc), 256, 0, st, img, tg, npix, p.cost_kind, static_cast<float>(p.threshold),
+    ilt_data<<<dim3(kRedBlocks, nc), 256, 0, st>>>(img, tg, npix, p.cost_kind, static_cast<float>(p.threshold),
                                                    static_cast<float>(p.steepness), static_cast<float>(p.dose),
                                                    img, pdata);
-    pdl(sum_parts, (nc * 2 + 3) / 4, 128, 0, st, pdata, kRedBlocks, 2, nc, sums);
+    sum_parts<<<(nc * 2 + 3) / 4, 128, 0, st>>>(pdata, kRedBlocks, 2, nc, sums);
     float* dcdm = nullptr;
     if (grad) {
       // G' = the band-2h part of G = dC/dI, sampled on the evaluation grid
@@ -1083,8 +1060,8 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
         const dim3 gr(B, nc);
         const size_t smr = 2 * static_cast<size_t>(fr_buf(M, xt_S(M))) * sizeof(float2);
 #define HUV_ILT_ADJ(LL, SS)                                                                 \
-  pdl(ilt_cols_adj_xt<LL, SS>, ga, 256, sm, st, T, Gm, ak.K, hb, keep, sums, fo, V, twm); \
-  pdl(ilt_rows_adj_xt<LL, SS>, gr, 256, smr, st, V, ak.kband, ak.K, hb, Q, twm);
+  ilt_cols_adj_xt<LL, SS><<<ga, 256, sm, st>>>(T, Gm, ak.K, hb, keep, sums, fo, V, twm); \
+  ilt_rows_adj_xt<LL, SS><<<gr, 256, smr, st>>>(V, ak.kband, ak.K, hb, Q, twm);
         switch (M) {
           case 128: HUV_ILT_ADJ(128, 32) break;
           case 160: HUV_ILT_ADJ(160, 16) break;
@@ -1102,16 +1079,16 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
         const int Wc = fit_units(8, 2 * (sizeof(float2) << lgm) + (sizeof(float) << lgm));
         const size_t sm = 2 * (static_cast<size_t>(Wc) << lgm) * sizeof(float2) +
                           (static_cast<size_t>(Wc) << lgm) * sizeof(float);
-        pdl(ilt_cols_adj, dim3(M / Wc, nc), 256, sm, st, T, Gm, K, hb, lgm, Wc, keep, sums,
+        ilt_cols_adj<<<dim3(M / Wc, nc), 256, sm, st>>>(T, Gm, K, hb, lgm, Wc, keep, sums,
                                                         flare / static_cast<float>(npix), V, twm);
         const int S = fit_units(4, 2 * (sizeof(float2) << lgm));
         const size_t sm2 = 2 * (static_cast<size_t>(S) << lgm) * sizeof(float2);
-        pdl(ilt_rows_adj, dim3(B, nc), 256, sm2, st, V, ds.kband, K, hb, lgm, S, Q, twm);
+        ilt_rows_adj<<<dim3(B, nc), 256, sm2, st>>>(V, ds.kband, K, hb, lgm, S, Q, twm);
       }
       const float scale = static_cast<float>(2.0 * (1.0 - p.absorber) * p.weight) * grid_scale;
       // Re IFFT(Q) = IFFT(Hermitian part of Q): a real synthesis, two
       // columns per transform on the register-radix path
-      pdl(hermitian_part, (nc * ((B * B + 1) / 2) + 255) / 256, 256, 0, st, Q, B, nc);
+      hermitian_part<<<(nc * ((B * B + 1) / 2) + 255) / 256, 256, 0, st>>>(Q, B, nc);
       dcdm = tbuf;  // the transmittance is no longer needed
       if (sep && interp_fused_ok(M, n)) {
         // dC/dm has band h: synthesised on the evaluation grid and
@@ -1120,7 +1097,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
         check_cuda(socs_rows_x(nullptr, scale, Q, 1, hb, M, nc, X2, twm, st), "ilt grad rows");
         check_cuda(socs_cols_x(X2, 1, hb, M, nc, 1.f, 0.f, nullptr, IM, 1, twm, st), "ilt grad cols");
         __half* planes = reinterpret_cast<__half*>(V);  // the adjoint fields are no longer needed
-        pdl(split_signed, nc, 1024, 0, st, IM, static_cast<int>(mpix), mean, planes);
+        split_signed<<<nc, 1024, 0, st>>>(IM, static_cast<int>(mpix), mean, planes);
         interp_separable(ds, M, nc, planes, mean, nullptr, dcdm, st, false);
       } else {
         check_cuda(socs_rows_x(nullptr, scale, Q, 1, hb, n, nc, T2, twn, st), "ilt grad rows");
@@ -1130,23 +1107,23 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
     // 16-byte accesses of theta and the gradient (a caller's planes may lie anywhere)
     const bool vec16 = ((reinterpret_cast<uintptr_t>(th) | reinterpret_cast<uintptr_t>(grad)) & 15u) == 0;
     if (tile == 64)
-      pdl(vec16 ? ilt_finish_4x4 : ilt_finish_tiled<64>, dim3(reg_parts, nc), 256, 0, st, 
+      (vec16 ? ilt_finish_4x4 : ilt_finish_tiled<64>)<<<dim3(reg_parts, nc), 256, 0, st>>>(
           th, dcdm, n, static_cast<float>(p.beta), static_cast<float>(p.tv_weight),
           static_cast<float>(p.tv_epsilon), static_cast<float>(p.binarization_weight),
           grad ? grad + npix * c0 : nullptr, preg);
     else if (tiled)
-      pdl(ilt_finish_tiled<32>, dim3(reg_parts, nc), 256, 0, st, 
+      ilt_finish_tiled<32><<<dim3(reg_parts, nc), 256, 0, st>>>(
           th, dcdm, n, static_cast<float>(p.beta), static_cast<float>(p.tv_weight),
           static_cast<float>(p.tv_epsilon), static_cast<float>(p.binarization_weight),
           grad ? grad + npix * c0 : nullptr, preg);
     else
-      pdl(ilt_finish, dim3(kRedBlocks, nc), 256, 0, st, th, dcdm, n, static_cast<float>(p.beta),
+      ilt_finish<<<dim3(kRedBlocks, nc), 256, 0, st>>>(th, dcdm, n, static_cast<float>(p.beta),
                                                        static_cast<float>(p.tv_weight),
                                                        static_cast<float>(p.tv_epsilon),
                                                        static_cast<float>(p.binarization_weight),
                                                        grad ? grad + npix * c0 : nullptr, preg);
-    pdl(sum_parts, (nc + 3) / 4, 128, 0, st, preg, reg_parts, 1, nc, regsum);
-    pdl(ilt_combine, (nc + 127) / 128, 128, 0, st, sums, regsum, nc, p.weight, 1.0 / static_cast<double>(npix),
+    sum_parts<<<(nc + 3) / 4, 128, 0, st>>>(preg, reg_parts, 1, nc, regsum);
+    ilt_combine<<<(nc + 127) / 128, 128, 0, st>>>(sums, regsum, nc, p.weight, 1.0 / static_cast<double>(npix),
                                                   cost_dev + c0);
     check_cuda(cudaGetLastError(), "ilt kernels");
     prof.launches += (grad ? 17 : 10) + (coarse ? (grad ? 9 : 4) : 0) - (sep ? 2 : 0);
@@ -1170,26 +1147,26 @@ void Engine::ilt_eval_surrogate(Surrogate* sur, const huv_ilt_params& p, int mas
   double* preg = pdata + static_cast<size_t>(masks) * kRedBlocks * 2;
   double* sums = preg + static_cast<size_t>(masks) * kRedBlocks;
   double* regsum = sums + 2 * masks;
-  pdl(ilt_transmittance, 1184, 256, 0, st, theta, npix * masks, static_cast<float>(p.beta),
+  ilt_transmittance<<<1184, 256, 0, st>>>(theta, npix * masks, static_cast<float>(p.beta),
                                           static_cast<float>(p.absorber), tbuf);
   sur->forward(masks, tbuf, img, st);
-  pdl(ilt_data, dim3(kRedBlocks, masks), 256, 0, st, img, target, npix, p.cost_kind, static_cast<float>(p.threshold),
+  ilt_data<<<dim3(kRedBlocks, masks), 256, 0, st>>>(img, target, npix, p.cost_kind, static_cast<float>(p.threshold),
                                                     static_cast<float>(p.steepness), static_cast<float>(p.dose), img,
                                                     pdata);
-  pdl(sum_parts, (masks * 2 + 3) / 4, 128, 0, st, pdata, kRedBlocks, 2, masks, sums);
+  sum_parts<<<(masks * 2 + 3) / 4, 128, 0, st>>>(pdata, kRedBlocks, 2, masks, sums);
   float* dcdm = nullptr;
   if (grad) {
     sur->input_grad(masks, tbuf, img, dt, st);  // img now holds G = dC/dI
     // dC/dm = weight (1 - a) dC/dt
     const float sc = static_cast<float>(p.weight * (1.0 - p.absorber));
-    pdl(scale_inplace, 1184, 256, 0, st, dt, npix * masks, sc);
+    scale_inplace<<<1184, 256, 0, st>>>(dt, npix * masks, sc);
     dcdm = dt;
   }
-  pdl(ilt_finish, dim3(kRedBlocks, masks), 256, 0, st, theta, dcdm, n, static_cast<float>(p.beta),
+  ilt_finish<<<dim3(kRedBlocks, masks), 256, 0, st>>>(theta, dcdm, n, static_cast<float>(p.beta),
                                                       static_cast<float>(p.tv_weight), static_cast<float>(p.tv_epsilon),
                                                       static_cast<float>(p.binarization_weight), grad, preg);
-  pdl(sum_parts, (masks + 3) / 4, 128, 0, st, preg, kRedBlocks, 1, masks, regsum);
-  pdl(ilt_combine, (masks + 127) / 128, 128, 0, st, sums, regsum, masks, p.weight, 1.0 / static_cast<double>(npix),
+  sum_parts<<<(masks + 3) / 4, 128, 0, st>>>(preg, kRedBlocks, 1, masks, regsum);
+  ilt_combine<<<(masks + 127) / 128, 128, 0, st>>>(sums, regsum, masks, p.weight, 1.0 / static_cast<double>(npix),
                                                    cost_dev);
   check_cuda(cudaGetLastError(), "ilt surrogate kernels");
 }
@@ -1205,7 +1182,7 @@ std::vector<double> Engine::surrogate_error(Surrogate* sur, const huv_ilt_params
              "cudaMallocAsync");
   a = t + npix * masks;
   b = a + npix * masks;
-  pdl(ilt_transmittance, 1184, 256, 0, st, theta, npix * masks, static_cast<float>(p.beta),
+  ilt_transmittance<<<1184, 256, 0, st>>>(theta, npix * masks, static_cast<float>(p.beta),
                                           static_cast<float>(p.absorber), t);
   sur->forward(masks, t, a, st);
   huv_batch bt{};
@@ -1222,7 +1199,7 @@ std::vector<double> Engine::surrogate_error(Surrogate* sur, const huv_ilt_params
   else
     run_fft_form(bt, ds, M, b, st);
   // per mask: max |a - b| and max |b|
-  pdl(err_parts, dim3(kRedBlocks, masks), 256, 0, st, a, b, npix, parts);
+  err_parts<<<dim3(kRedBlocks, masks), 256, 0, st>>>(a, b, npix, parts);
   std::vector<double> h(static_cast<size_t>(masks) * kRedBlocks * 2);
   check_cuda(cudaMemcpyAsync(h.data(), parts, h.size() * 8, cudaMemcpyDeviceToHost, st), "D2H err");
   check_cuda(cudaFreeAsync(t, st), "cudaFreeAsync");
@@ -1311,16 +1288,16 @@ void Engine::ilt_optimize(const huv_ilt_params& p, const huv_ilt_opt& o, int mas
   };
   // per-mask dot products of compact blocks a[j], b[j], j < count
   auto dot = [&](const float* a, const float* b, int count) {
-    pdl(batched_dot, dim3(kRedBlocks, count), threads, 0, st, a, b, npix, parts.as<double>());
-    pdl(sum_parts, (count + 3) / 4, 128, 0, st, parts.as<double>(), kRedBlocks, 1, count, dots.as<double>());
+    batched_dot<<<dim3(kRedBlocks, count), threads, 0, st>>>(a, b, npix, parts.as<double>());
+    sum_parts<<<(count + 3) / 4, 128, 0, st>>>(parts.as<double>(), kRedBlocks, 1, count, dots.as<double>());
     std::vector<double> h(count);
     fetch(dots, h.data(), sizeof(double) * count);
     prof.launches += 2;
     return h;
   };
   auto maxabs = [&](const float* a, int count) {
-    pdl(batched_maxabs, dim3(kRedBlocks, count), threads, 0, st, a, npix, parts.as<double>());
-    pdl(max_parts, (count + 127) / 128, 128, 0, st, parts.as<double>(), kRedBlocks, count, dots.as<double>());
+    batched_maxabs<<<dim3(kRedBlocks, count), threads, 0, st>>>(a, npix, parts.as<double>());
+    max_parts<<<(count + 127) / 128, 128, 0, st>>>(parts.as<double>(), kRedBlocks, count, dots.as<double>());
     std::vector<double> h(count);
     fetch(dots, h.data(), sizeof(double) * count);
     prof.launches += 2;
@@ -1334,7 +1311,7 @@ void Engine::ilt_optimize(const huv_ilt_params& p, const huv_ilt_opt& o, int mas
     upload(idx, ix.data(), sizeof(int) * c);
     upload(alpha, al.data(), sizeof(float) * c);
     upload(gamma, ga.data(), sizeof(float) * c);
-    pdl(gather_axpby, dim3(256, c), threads, 0, st, idx.as<int>(), alpha.as<float>(), gamma.as<float>(), x, y, npix,
+    gather_axpby<<<dim3(256, c), threads, 0, st>>>(idx.as<int>(), alpha.as<float>(), gamma.as<float>(), x, y, npix,
                                                    out);
     prof.launches += 1;
   };
@@ -1342,7 +1319,7 @@ void Engine::ilt_optimize(const huv_ilt_params& p, const huv_ilt_opt& o, int mas
     const int c = static_cast<int>(ix.size());
     if (!c) return;
     upload(idx, ix.data(), sizeof(int) * c);
-    pdl(scatter_blocks, dim3(256, c), threads, 0, st, idx.as<int>(), src, npix, dst);
+    scatter_blocks<<<dim3(256, c), threads, 0, st>>>(idx.as<int>(), src, npix, dst);
     prof.launches += 1;
   };
   bool use_sur = sur != nullptr;

@@ -32,7 +32,6 @@
 
 #include "../engine.hpp"
 #include "fft_reg.cuh"
-#include "pdl.cuh"
 #include "tc_ptx.cuh"
 
 namespace huv_dev {
@@ -75,7 +74,6 @@ struct InterpParams {
 template <int OUTBUFS>
 __global__ void __launch_bounds__(32 * (2 + kIfEpiWarps), 1)
     tc_interp_fused(const __grid_constant__ CUtensorMap tmI, const __grid_constant__ CUtensorMap tmO, InterpParams p) {
-  pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -380,9 +378,9 @@ cudaError_t interp_fused(const void* P, const void* im_split, int M, int n, int 
   p.probe_wait_ns = probe_wait_ns();
   const dim3 g(n / 256, (p.mt + p.mt_per - 1) / p.mt_per, nc);
   if (huv_dev::if_out_bufs(M) == 1)
-    pdl(huv_dev::tc_interp_fused<1>, g, 32 * (2 + huv_dev::kIfEpiWarps), huv_dev::if_smem_bytes(M), st, mi, mo, p);
+    huv_dev::tc_interp_fused<1><<<g, 32 * (2 + huv_dev::kIfEpiWarps), huv_dev::if_smem_bytes(M), st>>>(mi, mo, p);
   else
-    pdl(huv_dev::tc_interp_fused<2>, g, 32 * (2 + huv_dev::kIfEpiWarps), huv_dev::if_smem_bytes(M), st, mi, mo, p);
+    huv_dev::tc_interp_fused<2><<<g, 32 * (2 + huv_dev::kIfEpiWarps), huv_dev::if_smem_bytes(M), st>>>(mi, mo, p);
   return cudaGetLastError();
 }
 

@@ -34,7 +34,6 @@
 #include <cmath>
 #include <vector>
 
-#include "pdl.cuh"
 #include "tc_ptx.cuh"
 
 namespace huv_dev {
@@ -55,7 +54,6 @@ __host__ __device__ constexpr size_t mb_smem_bytes(int N) {
 __global__ void __launch_bounds__(192, 1)
     band_rows_i8(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmD, int kboxes,
                  int N, int hb, uint32_t tmem_cols, int L, int transposed, float2* __restrict__ X, int* err) {
-  pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -306,7 +304,7 @@ cudaError_t mask_rows_tc(const void* in, int n, int hb, int clips, float2* X, co
   const uint32_t cols = 3 * N <= 256 ? 256u : 512u;
   size_t smem = mb_smem_bytes(N);
   if (cols == 512u && smem < (120u << 10)) smem = 120u << 10;
-  pdl(band_rows_i8, clips * n / 128, 192, smem, st, ma, md, n / 128, N, hb, cols, n, transposed ? 1 : 0, X, err);
+  band_rows_i8<<<clips * n / 128, 192, smem, st>>>(ma, md, n / 128, N, hb, cols, n, transposed ? 1 : 0, X, err);
   return cudaGetLastError();
 }
 

@@ -38,7 +38,6 @@
 #include <vector>
 
 #include "../engine.hpp"
-#include "pdl.cuh"
 
 namespace huv_dev {
 
@@ -85,7 +84,6 @@ __device__ void run_terms(const double2* __restrict__ runs, int first, int count
 // X[j][m + h] and Y[j][m + h] for every row j (one warp per row).
 __global__ void rect_row_coef(const RectRowDev* __restrict__ rows, const double2* __restrict__ runs, int n_rows,
                               int h, double L, double2* __restrict__ X, double2* __restrict__ Y) {
-  pdl_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= n_rows) return;
   const int B = 2 * h + 1;
@@ -142,7 +140,6 @@ __device__ void bitonic(double* key, int16_t* val, int n) {
 __global__ void __launch_bounds__(256) rect_sort(const double* __restrict__ rects, const int32_t* __restrict__ offs,
                                                   double half, int cap, double4* __restrict__ sorted,
                                                   double* __restrict__ ys, int2* __restrict__ counts) {
-  pdl_begin();
   extern __shared__ double rsm[];
   double* key = rsm;                                          // [2 cap]
   int16_t* val = reinterpret_cast<int16_t*>(key + 2 * cap);  // [cap]
@@ -203,7 +200,6 @@ __global__ void __launch_bounds__(256) rect_edges(const int32_t* __restrict__ of
                                                    const double4* __restrict__ sorted, const double* __restrict__ ys,
                                                    int h, double L, double2* __restrict__ EX,
                                                    double2* __restrict__ EY) {
-  pdl_begin();
   const int c = blockIdx.y, o0 = offs[c] - offs[0], B = 2 * h + 1;
   const int2 n = counts[c];
   const int nx = 2 * n.x, total = (nx + n.y) * B;
@@ -229,7 +225,6 @@ __global__ void __launch_bounds__(256) rect_rows(const int32_t* __restrict__ off
                                                   const double4* __restrict__ sorted, const double* __restrict__ ys,
                                                   const double2* __restrict__ EX, const double2* __restrict__ EY, int h,
                                                   double2* __restrict__ X, double2* __restrict__ Y) {
-  pdl_begin();
   const int c = blockIdx.y, o0 = offs[c] - offs[0], B = 2 * h + 1, lane = threadIdx.x & 31;
   const int2 n = counts[c];
   const size_t e0 = 2 * static_cast<size_t>(o0);
@@ -297,7 +292,6 @@ __global__ void __launch_bounds__(256) rect_band_gemm(const int32_t* __restrict_
                                                        int c0, int h, int n, double2 dv, double2 bgn2,
                                                        const float* __restrict__ W, float2* __restrict__ Mband,
                                                        float* __restrict__ parts) {
-  pdl_begin();
   extern __shared__ double2 rs[];
   constexpr int TY = kRectTY, MAXE = (TY * 255 + 255) / 256;
   const int B = 2 * h + 1;
@@ -378,7 +372,6 @@ __global__ void __launch_bounds__(256) rect_band_gemm(const int32_t* __restrict_
 
 // mean[c] = sum_i parts[c][i] in order (deterministic).
 __global__ void rect_mean_reduce(const float* __restrict__ parts, int nparts, int clips, float* __restrict__ mean) {
-  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= clips) return;
   float s = 0.f;
@@ -389,8 +382,6 @@ __global__ void rect_mean_reduce(const float* __restrict__ parts, int nparts, in
 }  // namespace huv_dev
 
 namespace huv {
-
-using huv_launch::pdl;
 
 namespace {
 
@@ -564,18 +555,18 @@ void Engine::rect_band(int c0, int nc, int hb, const float* W, float2* Mband, fl
     if (c0 == 0) {
       int cap = 1;
       while (cap < rect.most) cap <<= 1;
-      pdl(huv_dev::rect_sort, rect.clips, 256, cap * (2 * sizeof(double) + sizeof(int16_t)), st, 
+      huv_dev::rect_sort<<<rect.clips, 256, cap * (2 * sizeof(double) + sizeof(int16_t)), st>>>(
           static_cast<const double*>(rect.rows), offs, L / 2.0, cap, sorted, ys, counts);
       const int vals = 4 * std::max(rect.most, 1) * B, rows = 2 * std::max(rect.most, 1);
-      pdl(huv_dev::rect_edges, dim3(std::min((vals + 255) / 256, 64), rect.clips), 256, 0, st, offs, counts, sorted, ys, hb,
+      huv_dev::rect_edges<<<dim3(std::min((vals + 255) / 256, 64), rect.clips), 256, 0, st>>>(offs, counts, sorted, ys, hb,
                                                                                              L, EX, EY);
-      pdl(huv_dev::rect_rows, dim3(std::min((rows + 7) / 8, 64), rect.clips), 256, 0, st, offs, counts, sorted, ys, EX, EY,
+      huv_dev::rect_rows<<<dim3(std::min((rows + 7) / 8, 64), rect.clips), 256, 0, st>>>(offs, counts, sorted, ys, EX, EY,
                                                                                         hb, X, Y);
       check_cuda(cudaGetLastError(), "rect_rows");
     }
   } else if (c0 == 0 && rect.n_rows > 0) {
     const int threads = 256, warps = threads / 32;
-    pdl(huv_dev::rect_row_coef, (rect.n_rows + warps - 1) / warps, threads, 0, st, 
+    huv_dev::rect_row_coef<<<(rect.n_rows + warps - 1) / warps, threads, 0, st>>>(
         static_cast<const huv_dev::RectRowDev*>(rect.rows), static_cast<const double2*>(rect.runs), rect.n_rows, hb,
         L, X, Y);
     check_cuda(cudaGetLastError(), "rect_row_coef");
@@ -584,12 +575,12 @@ void Engine::rect_band(int c0, int nc, int hb, const float* W, float2* Mband, fl
   float* parts = (W && mean) ? mean + nc : nullptr;
   const double n2 = static_cast<double>(n) * n;
   const size_t sm = sizeof(double2) * 16 * (huv_dev::kRectTY + B);
-  pdl(huv_dev::rect_band_gemm, dim3(tiles, nc), 256, sm, st, 
+  huv_dev::rect_band_gemm<<<dim3(tiles, nc), 256, sm, st>>>(
       offs, rect.on_device ? counts : nullptr, X, Y, c0, hb, n, rect.dv,
       make_double2(rect.bg.x * n2, rect.bg.y * n2), W, Mband, parts);
   check_cuda(cudaGetLastError(), "rect_band_gemm");
   if (parts) {
-    pdl(huv_dev::rect_mean_reduce, (nc + 127) / 128, 128, 0, st, parts, tiles, nc, mean);
+    huv_dev::rect_mean_reduce<<<(nc + 127) / 128, 128, 0, st>>>(parts, tiles, nc, mean);
     check_cuda(cudaGetLastError(), "mean_reduce(rects)");
   }
 }

@@ -24,7 +24,6 @@
 
 #include "fft_block.cuh"
 #include "fft_reg.cuh"
-#include "pdl.cuh"
 
 namespace huv_dev {
 
@@ -51,7 +50,6 @@ __device__ __forceinline__ float2 load_px<2>(const void* base, size_t idx) {
 template <int KIND>
 __global__ void band_rows_fwd(const void* __restrict__ in, int lg, int rows_per_block, int hb,
                               float2* __restrict__ X, const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   const int L = 1 << lg;
   const int B = 2 * hb + 1;
@@ -106,7 +104,6 @@ __global__ void band_cols_fwd(const float2* __restrict__ X, int lg, int hb, int 
                               const float* __restrict__ ptx, const float* __restrict__ W,
                               float2* __restrict__ Mband, float* __restrict__ parts,
                               const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   __shared__ float red[32];
   const int L = 1 << lg;
@@ -152,7 +149,6 @@ __global__ void band_cols_fwd(const float2* __restrict__ X, int lg, int hb, int 
 
 // mean[clip] = sum of the clip's parts in index order (deterministic).
 __global__ void mean_reduce(const float* __restrict__ parts, int nparts, int clips, float* __restrict__ mean) {
-  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= clips) return;
   float s = 0.f;
@@ -166,7 +162,6 @@ __global__ void mean_reduce(const float* __restrict__ parts, int nparts, int cli
 __global__ void socs_rows_inv(const float2* __restrict__ kband, float scale,
                               const float2* __restrict__ Mband, int K, int hb, int lg, int S,
                               float2* __restrict__ T, const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   const int L = 1 << lg;
   const int B = 2 * hb + 1;
@@ -203,7 +198,6 @@ template <int MODE>
 __global__ void socs_cols_inv(const float2* __restrict__ T, int K, int hb, int lg, int Wc,
                               float keep, float flare, const float* __restrict__ mean,
                               float* __restrict__ out, const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   const int L = 1 << lg;
   const int B = 2 * hb + 1;
@@ -247,7 +241,6 @@ __global__ void socs_cols_inv(const float2* __restrict__ T, int K, int hb, int l
 // order -- the same operations in the same order, with K times the blocks.
 __global__ void socs_cols_field(const float2* __restrict__ T, int K, int hb, int lg, int Wc, float2* __restrict__ E,
                                 const float2* __restrict__ tw) {
-  pdl_begin();
   extern __shared__ float2 smem[];
   const int L = 1 << lg;
   const int B = 2 * hb + 1;
@@ -270,7 +263,6 @@ __global__ void socs_cols_field(const float2* __restrict__ T, int K, int hb, int
 }
 __global__ void __launch_bounds__(256) fields_sum(const float2* __restrict__ E, int K, int npix, float keep, float flare,
                                                    const float* __restrict__ mean, float* __restrict__ out) {
-  pdl_begin();
   const int clip = blockIdx.y;
   const float add = mean ? flare * mean[clip] : 0.f;
   for (int i = blockIdx.x * 256 + threadIdx.x; i < npix; i += gridDim.x * 256) {
@@ -299,7 +291,6 @@ template <int L, int S>
 __global__ void __launch_bounds__(fr_threads(L, S), (L <= 256 ? 6 : 4))
     socs_rows_xt(const float2* __restrict__ kband, float scale, const float2* __restrict__ Mband, int K, int hb,
                  float2* __restrict__ Tt, const float2* __restrict__ tw) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L);
   constexpr int R = fr_radix(L, NP - 1);
   extern __shared__ float2 smem[];
@@ -365,7 +356,6 @@ __global__ void __launch_bounds__(fr_threads(L, S), ((L == 160 && MODE == 0) || 
     socs_cols_xt(const float2* __restrict__ Tt, int K, int hb, float keep, float flare,
                  const float* __restrict__ mean, float* __restrict__ out, const float2* __restrict__ tw,
                  __half* __restrict__ split) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L);
   constexpr int R = fr_radix(L, NP - 1);
   constexpr int XS = MODE == 1 ? 2 * S : S;
@@ -489,7 +479,6 @@ __global__ void __launch_bounds__(fr_threads(L, S), ((L == 160 && MODE == 0) || 
 template <int L, int S, typename In = float>
 __global__ void __launch_bounds__(fr_threads(L, S), (L >= 384 ? 4 : 1))
     band_rows_reg(const In* __restrict__ in, int hb, float2* __restrict__ X, const float2* __restrict__ tw) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L);
   extern __shared__ float2 smem[];
   const size_t row0 = static_cast<size_t>(blockIdx.x) * 2 * S;
@@ -536,7 +525,6 @@ __global__ void __launch_bounds__(fr_threads(L, S), (L >= 384 ? 4 : 1))
 template <int L, int S, bool CPLX>
 __global__ void __launch_bounds__(fr_threads(L, S), 3)
     band_rows_img(const void* __restrict__ in, int hb, float2* __restrict__ X, const float2* __restrict__ tw) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L), LD = L + 4;
   extern __shared__ __align__(16) float2 smem[];
   const int t = threadIdx.x;
@@ -605,7 +593,6 @@ __global__ void __launch_bounds__(fr_threads(L, S))
     band_cols_reg(const float2* __restrict__ X, bool half, bool transposed, int hb, const float* __restrict__ ptx,
                   const float* __restrict__ W, float2* __restrict__ Mband, float* __restrict__ parts,
                   const float2* __restrict__ tw) {
-  pdl_begin();
   constexpr int T = fr_threads(L, S), NP = fr_passes(L);
   constexpr int R = fr_radix(L, NP - 1);
   extern __shared__ float2 smem[];
@@ -752,15 +739,15 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     const size_t smr = static_cast<size_t>(fr_buf(n, Sr)) * sizeof(float2);
     const float* fin = static_cast<const float*>(in);
     if (n == 1024)
-      pdl(band_rows_reg<1024, 4, float>, gr, 256, smr, st, fin, hb, X, tw);
+      band_rows_reg<1024, 4><<<gr, 256, smr, st>>>(fin, hb, X, tw);
     else if (n == 2048)
-      pdl(band_rows_reg<2048, 2, float>, gr, 256, smr, st, fin, hb, X, tw);
+      band_rows_reg<2048, 2><<<gr, 256, smr, st>>>(fin, hb, X, tw);
     else if (n == 384)
-      pdl(band_rows_reg<384, 8, float>, gr, 256, smr, st, fin, hb, X, tw);
+      band_rows_reg<384, 8><<<gr, 256, smr, st>>>(fin, hb, X, tw);
     else if (n == 160)
-      pdl(band_rows_reg<160, 16, float>, gr, 256, smr, st, fin, hb, X, tw);
+      band_rows_reg<160, 16><<<gr, 256, smr, st>>>(fin, hb, X, tw);
     else
-      pdl(band_rows_reg<192, 16, float>, gr, 256, smr, st, fin, hb, X, tw);
+      band_rows_reg<192, 16><<<gr, 256, smr, st>>>(fin, hb, X, tw);
     rows_tc = cudaSuccess;
     half = true;
   }
@@ -770,7 +757,7 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     const int Sr = xt_S(n);
     const dim3 gr(static_cast<unsigned>(static_cast<size_t>(clips) * n / (2 * Sr)));
     const size_t smr = static_cast<size_t>(fr_buf(n, Sr)) * sizeof(float2);
-    pdl(band_rows_reg<2048, 2, uint8_t>, gr, 256, smr, st, static_cast<const uint8_t*>(in), hb, X, tw);
+    band_rows_reg<2048, 2, uint8_t><<<gr, 256, smr, st>>>(static_cast<const uint8_t*>(in), hb, X, tw);
     rows_tc = cudaSuccess;
     half = true;
   }
@@ -781,35 +768,35 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     const int Sr = xt_S(n);
     const unsigned blocks = static_cast<unsigned>(static_cast<size_t>(clips) * n / (kind == 2 ? Sr : 2 * Sr));
     const size_t smr = xt_buf_bytes(n) + (kind == 2 ? 0 : static_cast<size_t>(2) * Sr * (n + 4) * sizeof(float));
-    cudaError_t e = cudaErrorNotSupported;
+    rows_done = true;
 #define HUV_ROWS_IMG(LL, SS)                                                                            \
   case LL:                                                                                              \
     if (kind == 2)                                                                                      \
-      e = pdl(band_rows_img<LL, SS, true>, blocks, 256, smr, st, in, hb, X, tw);                        \
+      band_rows_img<LL, SS, true><<<blocks, 256, smr, st>>>(in, hb, X, tw);                             \
     else if (LL <= 512)                                                                                 \
-      e = pdl(band_rows_img<(LL <= 512 ? LL : 512), (LL <= 512 ? SS : 8), false>, blocks, 256, smr, st, in, hb, X, tw); \
+      band_rows_img<(LL <= 512 ? LL : 512), (LL <= 512 ? SS : 8), false><<<blocks, 256, smr, st>>>(in, hb, X, tw); \
     break;
     switch (n) {
       HUV_ROWS_IMG(128, 32) HUV_ROWS_IMG(256, 16) HUV_ROWS_IMG(512, 8) HUV_ROWS_IMG(1024, 4) HUV_ROWS_IMG(2048, 2)
+      default: rows_done = false;
     }
 #undef HUV_ROWS_IMG
-    if (e == cudaSuccess) {
+    if (rows_done) {
       rows_tc = cudaSuccess;
       half = kind == 1;
-      rows_done = true;
     }
   }
   if (!pow2 && rows_tc != cudaSuccess) return cudaErrorInvalidValue;  // no radix-4 kernel for this length
   // Only device rasters come here (rectangle clips take the analytic path).
   switch (kind) {
     case 0:
-      if (rows_tc != cudaSuccess) pdl(band_rows_fwd<0>, g1, th, sm1, st, in, lg, rows_per_block, hb, X, tw);
+      if (rows_tc != cudaSuccess) band_rows_fwd<0><<<g1, th, sm1, st>>>(in, lg, rows_per_block, hb, X, tw);
       break;
     case 1:
-      if (rows_tc != cudaSuccess) pdl(band_rows_fwd<1>, g1, th, sm1, st, in, lg, rows_per_block, hb, X, tw);
+      if (rows_tc != cudaSuccess) band_rows_fwd<1><<<g1, th, sm1, st>>>(in, lg, rows_per_block, hb, X, tw);
       break;
     case 2:
-      if (!rows_done) pdl(band_rows_fwd<2>, g1, th, sm1, st, in, lg, rows_per_block, hb, X, tw); break;
+      if (!rows_done) band_rows_fwd<2><<<g1, th, sm1, st>>>(in, lg, rows_per_block, hb, X, tw); break;
     default: return cudaErrorInvalidValue;
   }
   const int B = 2 * hb + 1;
@@ -823,14 +810,14 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     const dim3 g(nblk, clips);
     const size_t sm = xt_buf_bytes(n);
     switch (n) {
-      case 128: pdl(band_cols_reg<128, 32>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 160: pdl(band_cols_reg<160, 16>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 192: pdl(band_cols_reg<192, 16>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 256: pdl(band_cols_reg<256, 16>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 384: pdl(band_cols_reg<384, 8>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 512: pdl(band_cols_reg<512, 8>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 2048: pdl(band_cols_reg<2048, 2>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
-      case 1024: pdl(band_cols_reg<1024, 4>, g, 256, sm, st, X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 128: band_cols_reg<128, 32><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 160: band_cols_reg<160, 16><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 192: band_cols_reg<192, 16><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 256: band_cols_reg<256, 16><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 384: band_cols_reg<384, 8><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 512: band_cols_reg<512, 8><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 2048: band_cols_reg<2048, 2><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
+      case 1024: band_cols_reg<1024, 4><<<g, 256, sm, st>>>(X, half, x_transposed, hb, ptx, W, Mband, parts, tw); break;
       default: return cudaErrorInvalidValue;
     }
   } else {
@@ -838,9 +825,9 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     const int cpb = fit_units(4, 2 * (sizeof(float2) << lg));
     nblk = (B + cpb - 1) / cpb;
     const size_t sm2 = 2 * (static_cast<size_t>(cpb) << lg) * sizeof(float2);
-    pdl(band_cols_fwd, dim3(nblk, clips), 256, sm2, st, X, lg, hb, cpb, ptx, W, Mband, parts, tw);
+    band_cols_fwd<<<dim3(nblk, clips), 256, sm2, st>>>(X, lg, hb, cpb, ptx, W, Mband, parts, tw);
   }
-  if (parts) pdl(mean_reduce, (clips + 127) / 128, 128, 0, st, parts, nblk, clips, mean);
+  if (parts) mean_reduce<<<(clips + 127) / 128, 128, 0, st>>>(parts, nblk, clips, mean);
   return cudaGetLastError();
 }
 
@@ -876,14 +863,14 @@ cudaError_t socs_rows_x(const float2* kband, float scale, const float2* Mband, i
   const dim3 g((K * B + S - 1) / S, clips);
   const size_t sm = static_cast<size_t>(S) * B * sizeof(float2) + xt_buf_bytes(L);
   switch (L) {
-    case 128: pdl(socs_rows_xt<128, 32>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 160: pdl(socs_rows_xt<160, 16>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 192: pdl(socs_rows_xt<192, 16>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 256: pdl(socs_rows_xt<256, 16>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 384: pdl(socs_rows_xt<384, 8>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 512: pdl(socs_rows_xt<512, 8>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 2048: pdl(socs_rows_xt<2048, 2>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
-    case 1024: pdl(socs_rows_xt<1024, 4>, g, 256, sm, st, kband, scale, Mband, K, hb, T, tw); break;
+    case 128: socs_rows_xt<128, 32><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 160: socs_rows_xt<160, 16><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 192: socs_rows_xt<192, 16><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 256: socs_rows_xt<256, 16><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 384: socs_rows_xt<384, 8><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 512: socs_rows_xt<512, 8><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 2048: socs_rows_xt<2048, 2><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
+    case 1024: socs_rows_xt<1024, 4><<<g, 256, sm, st>>>(kband, scale, Mband, K, hb, T, tw); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -898,9 +885,9 @@ cudaError_t cols_xt(const float2* T, int K, int hb, int L, int clips, float keep
   const dim3 g(L / (mode == 0 ? S : 2 * S), clips);
 #define HUV_COLS_XT(LL, SS)                                                                                   \
   if (mode == 0)                                                                                            \
-    pdl(socs_cols_xt<LL, SS, 0>, g, 256, sm, st, T, K, hb, keep, flare, mean, out, tw, split);               \
+    socs_cols_xt<LL, SS, 0><<<g, 256, sm, st>>>(T, K, hb, keep, flare, mean, out, tw, split);               \
   else                                                                                                      \
-    pdl(socs_cols_xt<LL, SS, 1>, g, 256, sm, st, T, K, hb, keep, flare, mean, out, tw, nullptr);
+    socs_cols_xt<LL, SS, 1><<<g, 256, sm, st>>>(T, K, hb, keep, flare, mean, out, tw, nullptr);
   switch (L) {
     case 128: HUV_COLS_XT(128, 32) break;
     case 160: HUV_COLS_XT(160, 16) break;
@@ -945,7 +932,7 @@ cudaError_t socs_rows(const float2* kband, float scale, const float2* Mband, int
   const int S = fit_units(4, 2 * (sizeof(float2) << lgm));
   const size_t sm3 = 2 * (static_cast<size_t>(S) << lgm) * sizeof(float2);
   dim3 g3((K * B + S - 1) / S, clips);
-  pdl(socs_rows_inv, g3, 256, sm3, st, kband, scale, Mband, K, hb, lgm, S, T, tw);
+  socs_rows_inv<<<g3, 256, sm3, st>>>(kband, scale, Mband, K, hb, lgm, S, T, tw);
   return cudaGetLastError();
 }
 
@@ -957,9 +944,9 @@ cudaError_t socs_cols(const float2* T, int K, int hb, int lgm, int clips, float 
                      (static_cast<size_t>(Wc) << lgm) * sizeof(float);
   dim3 g4(L / Wc, clips);
   if (mode == 0)
-    pdl(socs_cols_inv<0>, g4, 256, sm4, st, T, K, hb, lgm, Wc, keep, flare, mean, out, tw);
+    socs_cols_inv<0><<<g4, 256, sm4, st>>>(T, K, hb, lgm, Wc, keep, flare, mean, out, tw);
   else
-    pdl(socs_cols_inv<1>, g4, 256, sm4, st, T, K, hb, lgm, Wc, keep, flare, mean, out, tw);
+    socs_cols_inv<1><<<g4, 256, sm4, st>>>(T, K, hb, lgm, Wc, keep, flare, mean, out, tw);
   return cudaGetLastError();
 }
 
@@ -970,9 +957,9 @@ cudaError_t socs_cols_few(const float2* T, int K, int hb, int lgm, int clips, fl
                           const float* mean, float2* E, float* out, const float2* tw, cudaStream_t st) {
   const int L = 1 << lgm;
   const int Wc = std::min(L, fit_units(8, 2 * (sizeof(float2) << lgm) + (sizeof(float) << lgm)));
-  pdl(socs_cols_field, dim3(L / Wc, clips, K), 256, 2 * (static_cast<size_t>(Wc) << lgm) * sizeof(float2), st, T, K, hb,
-      lgm, Wc, E, tw);
-  pdl(fields_sum, dim3(std::max(1, std::min(L * L / 256, 64)), clips), 256, 0, st, E, K, L * L, keep, flare, mean, out);
+  socs_cols_field<<<dim3(L / Wc, clips, K), 256, 2 * (static_cast<size_t>(Wc) << lgm) * sizeof(float2), st>>>(
+      T, K, hb, lgm, Wc, E, tw);
+  fields_sum<<<dim3(std::max(1, std::min(L * L / 256, 64)), clips), 256, 0, st>>>(E, K, L * L, keep, flare, mean, out);
   return cudaGetLastError();
 }
 
