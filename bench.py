@@ -623,15 +623,17 @@ def run_ours(args):
     # captures of this workload at 32 clips (cold cache, serialised), scaled
     # to a launch by its clips.  FFT and hybrid forms on the 160-point grid, the TC form's
     # y-contraction on 256.
+    # real rasters in focus: the kernels' transforms run in pairs (C2: 31 kernels, 16 transforms)
+    K_t = (K + 1) // 2
     traffic_per_clip = {"tc_dft_gemm<sumsq>": (166.38e6 + 6.65e6) / 32,
                         "socs_rows_tc": (19.29e6 + 110.03e6) / 32,
                         "tc_dft_gemm<interp>": (22.75e6 + 70.90e6) / 32,
                         "mask_band": (33.82e6 + 10.03e6) / 32,
-                        "socs_cols_inv": (95.29e6 + 0.13e6) / 32,
-                        "socs_rows_inv": (2.87e6 + 33.84e6) / 32,
+                        "socs_cols_inv": (49.18e6 + 0.0) / 32,
+                        "socs_rows_inv": (2.19e6 + 0.38e6) / 32,
                         "interp_band": (3.29e6 + 6.12e6) / 32,
                         "interp_rows_cols": (5.73e6 + 39.09e6 + 77.49e6) / 32,
-                        "tc_dft_gemm<interp_x>": (4.10e6 + 0.01e6) / 32}
+                        "tc_interp_fused": (4.21e6 + 76.54e6) / 32}
     # each region's own algorithmic bytes per clip (operands in and out once)
     hb_ = diag["band_half_width"]
     Bb = 2 * hb_ + 1
@@ -647,14 +649,13 @@ def run_ours(args):
     # transform of I_M and a GEMM over the Hermitian half band (K = 2 (2h + 1))
     sep = args.form in ("auto", "hybrid") and m_f <= 192
     k_int = m_f if sep else 2 * (2 * hb_ + 1)
-    if sep:  # the separable form's output GEMM (ncu --set full, 32 clips)
-        traffic_per_clip["tc_dft_gemm<interp>"] = (22.98e6 + 75.12e6) / 32
-    own_bytes = {"socs_cols_inv": 8 * K * Bb * m_f + 4 * m_f * m_f,
-                 "socs_rows_inv": 8 * K * Bb * m_f + 8 * Bb * Bb,
+    own_bytes = {"socs_cols_inv": 8 * K_t * Bb * m_f + 4 * m_f * m_f,
+                 "socs_rows_inv": 8 * K_t * Bb * m_f + 8 * Bb * Bb,
                  "tc_dft_gemm<sumsq>": 4 * K * m_f * kb + 4 * m_f * m_f,
                  "socs_rows_tc": 4 * K * m_f * kb + 8 * Bb * Bb,
-                 "tc_dft_gemm<interp>": 4 * N_GRID * N_GRID + 4 * N_GRID * (k_int if sep else kb),
-                 "tc_dft_gemm<interp_x>": 4 * m_f * m_f + 4 * N_GRID * m_f,
+                 "tc_dft_gemm<interp>": 4 * N_GRID * N_GRID + 4 * N_GRID * kb,
+                 # both products of I_N = P I_M P^T in one kernel: I_M in, the image out
+                 "tc_interp_fused": 4 * N_GRID * N_GRID + 4 * m_f * m_f,
                  # u8 raster in, the row band's orders m >= 0 out and back in, the band out
                  "mask_band": N_GRID * N_GRID + 16 * N_GRID * (hb_ + 1) + 8 * Bb * Bb,
                  # mask band in, the band kernels (8 K S, as the whole-path count has them), I_M out
@@ -691,13 +692,13 @@ def run_ours(args):
     roofline["traffic"] = (traffic_per_clip[prof["kernel"]] * images_per_launch
                            if prof["kernel"] in traffic_per_clip else None)
     # the FFT field-pass regions are bound by instruction issue, not HBM: their
-    # transform work as 5 L log2 L FLOP per L-point transform (rows: K B
-    # transforms, columns: K M transforms, on the M-point evaluation grid)
+    # transform work as 5 L log2 L FLOP per L-point transform (rows: K_t B
+    # transforms, columns: K_t M transforms, on the M-point evaluation grid)
     # against the nominal FP32 rate (148 SMs x 128 lanes x 2 x max SM clock)
     fp32_peak = 148 * 128 * 2 * 1.965e9 / 1e12
-    fft_flop = {"socs_cols_inv": K * m_f * 5 * m_f * math.log2(m_f),
-                "socs_rows_inv": K * Bb * 5 * m_f * math.log2(m_f),
-                "socs_field_fused": K * (Bb + m_f) * 5 * m_f * math.log2(m_f)}
+    fft_flop = {"socs_cols_inv": K_t * m_f * 5 * m_f * math.log2(m_f),
+                "socs_rows_inv": K_t * Bb * 5 * m_f * math.log2(m_f),
+                "socs_field_fused": K_t * (Bb + m_f) * 5 * m_f * math.log2(m_f)}
     for region, fl in fft_flop.items():
         reg = prof["regions"].get(region)
         if reg and reg[1] > 0:
@@ -705,12 +706,14 @@ def run_ours(args):
             roofline.setdefault("fft_regions", {})[region] = {
                 "transform_tflops": tf, "nominal_fp32_peak": fp32_peak, "frac_of_nominal_fp32": tf / fp32_peak,
                 "flop_per_clip": fl}
-    gi = prof["regions"].get("tc_dft_gemm<interp>")
+    interp = "tc_interp_fused" if sep else "tc_dft_gemm<interp>"
+    gi = prof["regions"].get(interp)
     if gi and gi[1] > 0:
-        # the band interpolation's N x N output GEMM: 2 N^2 k_int FLOP per
-        # image (split products counted once)
-        flop_i = 2.0 * N_GRID * N_GRID * k_int * N_CLIPS * args.steps
-        roofline["tensor_interp"] = {"kernel": "tc_dft_gemm<interp>", "achieved": flop_i / (gi[1] / 1e3) / 1e12,
+        # the band interpolation's GEMMs: 2 N^2 k_int FLOP per image for the
+        # N x N output, and 2 N M^2 for P I_M in the separable kernel (split
+        # products counted once)
+        flop_i = 2.0 * N_GRID * (N_GRID * k_int + (m_f * m_f if sep else 0)) * N_CLIPS * args.steps
+        roofline["tensor_interp"] = {"kernel": interp, "achieved": flop_i / (gi[1] / 1e3) / 1e12,
                                      "peak": tc_burst, "unit": "TFLOP/s",
                                      "frac": flop_i / (gi[1] / 1e3) / 1e12 / tc_burst if tc_burst else None,
                                      "gemm_k": k_int, "issued_products_per_algorithmic": 3}

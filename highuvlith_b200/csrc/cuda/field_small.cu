@@ -18,8 +18,8 @@
 // a strip of columns in one block (36 of 70 us of a 256^2 image at M = 64),
 // on power-of-two grids only (M = 128 where 80 or 96 suffice), and its images
 // went through the band transform to the output grid.  Whole calls, before and
-// after: one 256^2 EUV clip 70 -> 33 us, 7 complex 512^2 ArF clips 94 -> 45 us,
-// one clip at 21 planes of focus (189 launches before, 4 now) 1,391 -> 39 us.
+// after: one 256^2 EUV clip 70 -> 31 us, 7 complex 512^2 ArF clips 92 -> 38 us,
+// one clip at 21 planes of focus (189 launches before, 5 now) 1,352 -> 39 us.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
