@@ -310,72 +310,114 @@ __global__ void __launch_bounds__(256) fno_layer_bwd(const float* __restrict__ d
 }
 
 // dv[r][x][c] += Re sum_kx Z[r][kx][c] e^{+2 pi i kx x / S} (weight 1): the sum
-// over kk = (kx, re / im) ascending, then added to dv.  Rows grid-strided,
-// tiles of 128 pixels (S if smaller); thread (pg, cg) owns 8 pixels x 4
-// channels as pairs of channels, so that a step of kk costs three shared loads
-// for 16 paired multiply-adds, and fetches its dv before the sums.  Bound by
-// dv's 512 bytes per pixel and FP32 issue (8 x 512^2: 0.327 -> 0.27 ms against
-// 4 x 4 tiles of single multiply-adds).
-// Dynamic shared memory: 2m * (64 + 132) floats.
-__global__ void __launch_bounds__(256) fno_spec_to_dv(const float2* __restrict__ Z, int S, int m,
-                                                       const float2* __restrict__ twx, float* __restrict__ dv,
-                                                       int rows) {
+// over kk = (kx, re / im) ascending, then added to dv.  A block keeps one tile
+// of 128 pixels (S if smaller; blockIdx.x) with its twiddles and walks rows
+// blockIdx.y, + gridDim.y, ..., the next row's Z and dv fetched under this
+// one's sums; thread (pg, cg) owns 8 pixels x 4 channels as pairs of pixels, so
+// that a step of kk costs three shared loads for 16 paired multiply-adds.
+// Bound by dv's 512 bytes per pixel (0.16 ms at 8 x 512^2) and FP32 issue
+// (0.12), not fully overlapped with two blocks per SM: 0.327 ms with 4 x 4 tiles
+// of single multiply-adds, 0.27 with paired ones and one row's tiles per block,
+// 0.25 walking rows, 0.23 with dv's copies a row ahead (0.26 with Z held twice
+// to spare the moves that duplicate it).
+// Dynamic shared memory: 2m * (2 * 64 + 132) floats and 64 KB of dv.
+__global__ void __launch_bounds__(256, 2) fno_spec_to_dv(const float2* __restrict__ Z, int S, int m,
+                                                          const float2* __restrict__ twx, float* __restrict__ dv,
+                                                          int rows) {
   constexpr int C = 64, XT = 128, LD = 132;
   extern __shared__ __align__(16) float dsm[];
-  float* sZ = dsm;              // [2m][C]
-  float* sT = sZ + 2 * m * C;   // [2m][LD]
+  float* sT = dsm;              // [2m][LD]
+  float* sZ = sT + 2 * m * LD;  // two of [2m][C]
+  float4* sD = reinterpret_cast<float4*>(sZ + 4 * m * C) + threadIdx.x;  // this thread's dv: two of 8 x [256]
   const int t = threadIdx.x, cg = t & 15, pg = t >> 4;
-  const int xt = min(XT, S);
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    __syncthreads();
+  const int xt = min(XT, S), x0 = blockIdx.x * xt;
+  float2 zr[4];  // m <= 16
+  auto fetch = [&](int r) {
     const float2* Zr = Z + static_cast<size_t>(r) * m * C;
-    for (int e = t; e < m * C; e += 256) {
-      const int kx = e >> 6, c = e & 63;
-      const float2 zz = Zr[e];
-      sZ[(2 * kx) * C + c] = zz.x;
-      sZ[(2 * kx + 1) * C + c] = -zz.y;
-    }
-    const size_t row = static_cast<size_t>(r) * S * C;
-    for (int x0 = 0; x0 < S; x0 += xt) {
-      __syncthreads();
-      for (int e = t; e < m * xt; e += 256) {
-        const int kx = e / xt, px = e - kx * xt;
-        const float2 w = __ldg(twx + static_cast<size_t>(kx) * S + x0 + px);  // (cos, -sin)
-        sT[(2 * kx) * LD + px] = w.x;
-        sT[(2 * kx + 1) * LD + px] = -w.y;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (t + 256 * q < m * C) zr[q] = Zr[t + 256 * q];
+  };
+  auto put = [&](float* s) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = t + 256 * q, kx = e >> 6, c = e & 63;
+      if (e < m * C) {
+        s[(2 * kx) * C + c] = zr[q].x;
+        s[(2 * kx + 1) * C + c] = -zr[q].y;
       }
-      const bool live = pg * 8 < xt;
-      float4* d = reinterpret_cast<float4*>(dv + row + static_cast<size_t>(x0 + pg * 8) * C + cg * 4);
-      float4 cur[8];
+    }
+  };
+  const bool live = pg * 8 < xt;
+  auto row_of = [&](int r) {
+    return reinterpret_cast<float4*>(dv + (static_cast<size_t>(r) * S + x0 + pg * 8) * C + cg * 4);
+  };
+  auto prefetch = [&](int r, int b) {  // read back by the thread that asked for it
+    if (live && r < rows) {
+      const float4* d = row_of(r);
 #pragma unroll
-      for (int p = 0; p < 8; ++p) cur[p] = live ? d[p * (C / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
-      __syncthreads();
-      if (live) {
-        uint64_t acc[8][2];
+      for (int p = 0; p < 8; ++p) fr_cp_async16(sD + (b * 8 + p) * 256, d + p * (C / 4));
+    }
+    fr_cp_commit();
+  };
+  prefetch(blockIdx.y, 0);
+  if (blockIdx.y < rows) {
+    fetch(blockIdx.y);
+    put(sZ);
+  }
+  for (int e = t; e < m * xt; e += 256) {
+    const int kx = e / xt, px = e - kx * xt;
+    const float2 w = __ldg(twx + static_cast<size_t>(kx) * S + x0 + px);  // (cos, -sin)
+    sT[(2 * kx) * LD + px] = w.x;
+    sT[(2 * kx + 1) * LD + px] = -w.y;
+  }
+  __syncthreads();
+  int buf = 0;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y, buf ^= 1) {
+    const int next = r + static_cast<int>(gridDim.y);
+    const bool more = next < rows;
+    prefetch(next, buf ^ 1);
+    if (more) fetch(next);
+    if (live) {
+      const float* z0 = sZ + buf * 2 * m * C + cg * 4;
+      uint64_t acc[4][4];  // [pair of pixels][channel]
 #pragma unroll
-        for (int p = 0; p < 8; ++p) acc[p][0] = acc[p][1] = 0;
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[p][c] = 0;
 #pragma unroll 4
-        for (int kk = 0; kk < 2 * m; ++kk) {
-          const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(sZ + kk * C + cg * 4);
-          const float4 t0 = ld4(sT + kk * LD + pg * 8), t1 = ld4(sT + kk * LD + pg * 8 + 4);
-          const float tv[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+      for (int kk = 0; kk < 2 * m; ++kk) {
+        const float4 z = ld4(z0 + kk * C);
+        const ulonglong2 ta = *reinterpret_cast<const ulonglong2*>(sT + kk * LD + pg * 8);
+        const ulonglong2 tb = *reinterpret_cast<const ulonglong2*>(sT + kk * LD + pg * 8 + 4);
+        const uint64_t tv[4] = {ta.x, ta.y, tb.x, tb.y};
+        const float zs[4] = {z.x, z.y, z.z, z.w};
+        uint64_t zv[4];
 #pragma unroll
-          for (int p = 0; p < 8; ++p) {
-            uint64_t a;
-            asm("mov.b64 %0, {%1, %1};" : "=l"(a) : "f"(tv[p]));
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[p][0]) : "l"(a), "l"(z.x));
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[p][1]) : "l"(a), "l"(z.y));
-          }
-        }
+        for (int c = 0; c < 4; ++c) asm("mov.b64 %0, {%1, %1};" : "=l"(zv[c]) : "f"(zs[c]));
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
-          float4 s;
-          asm("mov.b64 {%0, %1}, %2;" : "=f"(s.x), "=f"(s.y) : "l"(acc[p][0]));
-          asm("mov.b64 {%0, %1}, %2;" : "=f"(s.z), "=f"(s.w) : "l"(acc[p][1]));
-          d[p * (C / 4)] = make_float4(cur[p].x + s.x, cur[p].y + s.y, cur[p].z + s.z, cur[p].w + s.w);
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[p][c]) : "l"(tv[p]), "l"(zv[c]));
+      }
+      fr_cp_wait<1>();
+      float4* d = row_of(r);
+#pragma unroll
+      for (int p = 0; p < 8; ++p) {
+        const float4 cur = sD[(buf * 8 + p) * 256];
+        float s[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float lo, hi;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[p / 2][c]));
+          s[c] = p & 1 ? hi : lo;
         }
+        d[p * (C / 4)] = make_float4(cur.x + s[0], cur.y + s[1], cur.z + s[2], cur.w + s[3]);
       }
     }
+    if (more) put(sZ + (buf ^ 1) * 2 * m * C);
+    __syncthreads();
   }
 }
 
@@ -794,7 +836,7 @@ struct Fno {
   static constexpr size_t kProjBwdSmem = (2 * 64 * 128 + 2 * 64 * 68 + 64 * 132 + 128 * 68 + 64) * 4;
   static constexpr size_t kLayerBwdSmem = (64 * 64 + 3 * 64 * 68) * 4;
   size_t layer_out_smem() const { return (2 * 64 * 68 + 2 * static_cast<size_t>(m) * (64 + 68)) * 4; }
-  size_t spec_smem() const { return (2 * static_cast<size_t>(m) * (64 + 132)) * 4; }
+  size_t spec_smem() const { return (2 * static_cast<size_t>(m) * (2 * 64 + 132)) * 4 + 2 * 8 * 256 * 16; }
   static unsigned pgrid(size_t pix) { return static_cast<unsigned>(std::min<size_t>((pix + 63) / 64, 296)); }
 
   // images[b][S][S] = FNO(masks[b]); with `keep`, everything a backward pass
@@ -838,7 +880,9 @@ struct Fno {
     using namespace huv_dev;
     const size_t pix = static_cast<size_t>(B) * S * S;
     const int rows = B * S;
-    const dim3 rgrid(std::min(rows, 4096));
+    // tiles of pixels x groups of rows, one wave of two blocks per SM
+    const int tiles = std::max(S / 128, 1);
+    const dim3 sgrid(tiles, std::min(rows, std::max(296 / tiles, 1)));
     check_cuda(cudaMemsetAsync(grad, 0, npar * 4, st), "memset grad");
     if (tc) {
       if (!huv_launch::fno_tc_proj_bwd(pix, v[L], par + oQ1, par + ob1, par + oQ2, dOut, dvA, grad + oQ1, grad + ob1,
@@ -865,7 +909,7 @@ struct Fno {
           Xl[l], Y, reinterpret_cast<const float2*>(par + oR[l]), m, modes, B,
           1.f / (static_cast<float>(S) * S), dX, reinterpret_cast<float2*>(grad + oR[l]));
       check_cuda(huv_launch::fno_idft_y(dX, B, S, m, tyt, Za, nullptr, st), "fno inverse dft y");
-      fno_spec_to_dv<<<rgrid, 256, spec_smem(), st>>>(Za, S, m, twx, dcur, rows);
+      fno_spec_to_dv<<<sgrid, 256, spec_smem(), st>>>(Za, S, m, twx, dcur, rows);
       std::swap(dnext, dcur);
     }
     check_cuda(huv_launch::fno_lift_back(masks, dnext, B, S, par + oWl, grad + oWl, grad + obl, dmask, st),
