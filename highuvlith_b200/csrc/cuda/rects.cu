@@ -458,7 +458,7 @@ void decompose(const huv_rect_clips& in, int n_clips, double L, std::vector<int3
 
 }  // namespace
 
-void Engine::upload_rects(const huv_batch& b, cudaStream_t st) {
+void Engine::check_rects(const huv_batch& b) const {
   const auto* in = static_cast<const huv_rect_clips*>(b.input);
   if (!in || !in->offsets || (in->offsets[b.n_clips] > in->offsets[0] && !in->rects))
     throw Error(HUV_ERR_INVALID_PARAMETER, "rect clips: null pointer");
@@ -474,6 +474,10 @@ void Engine::upload_rects(const huv_batch& b, cudaStream_t st) {
   if (!(std::isfinite(in->feature_re) && std::isfinite(in->feature_im) && std::isfinite(in->background_re) &&
         std::isfinite(in->background_im)))
     throw Error(HUV_ERR_INVALID_PARAMETER, "rect clips: amplitudes must be finite");
+}
+
+void Engine::upload_rects(const huv_batch& b, int hb, cudaStream_t st) {
+  const auto* in = static_cast<const huv_rect_clips*>(b.input);
   rect.dv = make_double2(in->feature_re - in->background_re, in->feature_im - in->background_im);
   rect.bg = make_double2(in->background_re, in->background_im);
   auto grow = [](void*& p, size_t& cap, size_t bytes) {
@@ -485,12 +489,12 @@ void Engine::upload_rects(const huv_batch& b, cudaStream_t st) {
     cap = bytes;
   };
   // Clips that fit rect_sort's shared memory are resolved on the device, as
-  // long as the batch's edge tables stay moderate (96 bytes per rectangle and
-  // order at most); the copies are ordered on the stream.
+  // long as the batch's tables (X, Y and both edge tables: 128 bytes per
+  // rectangle and order) stay moderate; the copies are ordered on the stream.
   const int total = in->offsets[b.n_clips] - in->offsets[0];
   int most = 0;
   for (int c = 0; c < b.n_clips; ++c) most = std::max(most, in->offsets[c + 1] - in->offsets[c]);
-  const int B = 2 * device_set(b.defocus_nm).hb + 1;
+  const int B = 2 * hb + 1;
   rect.on_device = most <= huv_dev::kRectSortMax && b.n_clips <= 65535 && B <= 255 &&
                    static_cast<size_t>(total) * B * 128 <= size_t(512) << 20;
   if (rect.on_device) {

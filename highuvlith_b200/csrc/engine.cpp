@@ -312,10 +312,14 @@ void Engine::prebuild_planes(const double* z, int planes) {
 bool Engine::sweep_small(const huv_batch& b, const double* z, int planes, float* out, cudaStream_t st) {
   if (planes < 2 || (b.form != HUV_FORM_AUTO && b.form != HUV_FORM_HYBRID)) return false;
   std::lock_guard<std::mutex> lock(mu);
-  check_batch(b, out);
+  huv_batch first = b;  // the batch's own defocus_nm is no part of a sweep
+  first.defocus_nm = z[0];
+  check_batch(first, out);
+  if (b.input_kind == HUV_INPUT_RECTS) check_rects(b);
   for (int p = 0; p < planes; ++p)
     if (!held_set(z[p])) return false;
   ensure_device();
+  // (pointers into the plane cache: nothing below may look a plane up)
   std::vector<DeviceSet*> sets(planes);
   int M = 0;
   for (int p = 0; p < planes; ++p) {
@@ -325,7 +329,7 @@ bool Engine::sweep_small(const huv_batch& b, const double* z, int planes, float*
     if (!m || (p > 0 && (m != M || sets[p]->hb != sets[0]->hb))) return false;
     M = m;
   }
-  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, st);
+  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, sets[0]->hb, st);
   run_small_form(b, sets.data(), nullptr, nullptr, planes, M, out, st);
   return true;
 }
@@ -678,8 +682,9 @@ void Engine::image_batch(const huv_batch& b, float* out, cudaStream_t st) {
   check_batch(b, out);
   if (b.n_clips == 0) return;
   ensure_device();
-  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, st);
+  if (b.input_kind == HUV_INPUT_RECTS) check_rects(b);
   DeviceSet& ds = device_set(b.defocus_nm == 0.0 ? 0.0 : b.defocus_nm);
+  if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, ds.hb, st);
   int form = b.form;
   // FFT and hybrid forms evaluate on the smallest supported grid above 4h
   // (160 or 192 where that beats the next power of two); the tcgen05
@@ -713,8 +718,8 @@ void Engine::image_batch_host(const huv_batch& b, float* out_host, cudaStream_t 
   if (b.n_clips <= 0) return;
   if (!b.input || !out_host) throw Error(HUV_ERR_INVALID_PARAMETER, "input/out: null pointer");
   if (b.input_kind < 0 || b.input_kind > 3) throw Error(HUV_ERR_INVALID_PARAMETER, "input_kind: unknown");
-  // Rectangle clips are read on the host (their tables are built there):
-  // nothing to copy in, each chunk views its slice of the offsets.
+  // Rectangle clips are read on the host (upload_rects copies a chunk's):
+  // nothing to copy in here, each chunk views its slice of the offsets.
   const bool rects = b.input_kind == HUV_INPUT_RECTS;
   const size_t in_elem = b.input_kind == HUV_INPUT_RASTER_U8
                              ? 1

@@ -219,9 +219,12 @@ struct Engine {
   KernelSet build_set(double z);
   void image_batch(const huv_batch& b, float* out, cudaStream_t st);
   void image_batch_host(const huv_batch& b, float* out_host, cudaStream_t st);
-  // Rectangle clips (HUV_INPUT_RECTS): the batch's row/run table on the
-  // device, then the exact band spectrum of clips [c0, c0 + nc).
-  void upload_rects(const huv_batch& b, cudaStream_t st);
+  // Rectangle clips (HUV_INPUT_RECTS): refusal of what is no such batch, the
+  // batch's rectangles (or its host-resolved row/run table) on the device for
+  // a band of half-width hb, then the exact band spectrum of clips
+  // [c0, c0 + nc).
+  void check_rects(const huv_batch& b) const;
+  void upload_rects(const huv_batch& b, int hb, cudaStream_t st);
   void rect_band(int c0, int nc, int hb, const float* W, float2* Mband, float* mean, cudaStream_t st);
   // Kernel sets of the focus planes not cached yet, built concurrently (one
   // plane per host thread) and cached.
