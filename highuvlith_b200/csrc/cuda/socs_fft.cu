@@ -762,9 +762,12 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     half = true;
   }
   // f32 rows of 128 to 512 points and complex rows, unless the caller wants
-  // the radix-4 kernel's bits
+  // the radix-4 kernel's bits.  The f32 rows are staged by 16-byte copies: a
+  // raster that lies elsewhere (a clip of a plan may) takes the radix-4
+  // kernel, which loads single floats.
+  const bool aligned16 = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
   if (rows_tc != cudaSuccess && cols_reg && !radix4_rows && n <= 2048 &&
-      (kind == 2 ? n >= 128 : (kind == 1 && n <= 512))) {
+      (kind == 2 ? n >= 128 : (kind == 1 && n <= 512 && aligned16))) {
     const int Sr = xt_S(n);
     const unsigned blocks = static_cast<unsigned>(static_cast<size_t>(clips) * n / (kind == 2 ? Sr : 2 * Sr));
     const size_t smr = xt_buf_bytes(n) + (kind == 2 ? 0 : static_cast<size_t>(2) * Sr * (n + 4) * sizeof(float));
