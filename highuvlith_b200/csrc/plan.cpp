@@ -238,6 +238,12 @@ huv_status huv_plan_create(const huv_clip* clips, int32_t n_clips, int32_t pixel
       }
       g.in_base = clips[g.clips[0]].input;
       g.out_base = clips[g.clips[0]].out;
+      // Images are written by TMA and vector stores (16 bytes), complex maps
+      // read by elements: buffers that lie otherwise are staged.  Real inputs
+      // may lie anywhere (their row kernels check).
+      if ((reinterpret_cast<uintptr_t>(g.out_base) & 15u) != 0 ||
+          (g.kind == HUV_INPUT_TRANSMITTANCE_C64 && (reinterpret_cast<uintptr_t>(g.in_base) & 7u) != 0))
+        g.contiguous = false;
       if (!g.contiguous) {
         huv::check_cuda(cudaMalloc(&g.stage_in, in_bytes * g.clips.size()), "cudaMalloc(plan stage in)");
         huv::check_cuda(cudaMalloc(reinterpret_cast<void**>(&g.stage_out), out_bytes * g.clips.size()),

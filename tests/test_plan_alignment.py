@@ -60,3 +60,38 @@ def test_inputs(n, dtype, skip, clips, autotune):
     got, groups = _images(eng, _view(x, skip), out, autotune)
     assert len(groups) == 1 and groups[0]["contiguous"] == 1
     assert float((got - ref).abs().max() / ref.max()) < 1e-4
+
+
+@pytest.mark.parametrize("autotune", [False, True])
+@pytest.mark.parametrize("clips", [1, 3])
+@pytest.mark.parametrize("n,dtype,skip", [(128, "uint8", 2), (256, "uint8", 1), (256, "uint8", 2), (512, "uint8", 2),
+                                          (512, "float32", 3), (256, "complex64", 2)])
+def test_outputs(n, dtype, skip, clips, autotune):
+    import torch
+    eng, x = _engine(n), _maps(n, clips, dtype)
+    ref = eng.compute_batch(x, pixel_transfer=dtype == "uint8", form="fft")
+    buf = torch.full((clips * n * n + 2 * skip,), -7.0, device="cuda")
+    out = buf[skip:skip + clips * n * n].view(clips, n, n)
+    got, _ = _images(eng, x, out, autotune)
+    assert float((got - ref).abs().max() / ref.max()) < 1e-4
+    assert bool((buf[:skip] == -7.0).all()) and bool((buf[-skip:] == -7.0).all())
+
+
+def test_complex_maps_between_elements():
+    import torch
+    eng, x = _engine(256), _maps(256, 2, "complex64")
+    buf = torch.zeros(2 * x.numel() + 1, device="cuda")
+    buf[1:].copy_(torch.view_as_real(x).reshape(-1))
+    out = torch.empty((2, 256, 256), device="cuda")
+    bytes_per = 8 * 256 * 256
+    from highuvlith_b200 import _lib as L
+    import ctypes as C
+    arr = (L.Clip * 2)(*[L.Clip(eng.handle, 10, L.INPUT_C64, buf.data_ptr() + 4 + bytes_per * i, out[i].data_ptr())
+                         for i in range(2)])
+    h = C.c_void_p()
+    L.check(L.lib().huv_plan_create(arr, 2, 0, 0, C.byref(h)))
+    L.check(L.lib().huv_plan_launch(h, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    L.lib().huv_plan_destroy(h)
+    ref = eng.compute_batch(x, pixel_transfer=False, form="fft")
+    assert float((out - ref).abs().max() / ref.max()) < 1e-4
