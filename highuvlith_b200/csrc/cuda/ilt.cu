@@ -933,7 +933,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   const size_t s_t = a256(sizeof(float) * npix);           // transmittance, then dC/dm
   const size_t s_x = a256(sizeof(float2) * n * B2);        // row transforms of N x N inputs (band <= 2h)
   const size_t s_m = a256(sizeof(float2) * B * B);
-  const size_t s_mean = a256(sizeof(float) * (1 + (B2 + 3) / 4));
+  const size_t s_mean = a256(sizeof(float) * (1 + band_mean_parts(n, hb)));
   const size_t s_T = a256(sizeof(float2) * static_cast<size_t>(K) * B * M);
   const size_t s_im = coarse ? a256(sizeof(float) * mpix) : 0;  // I on M, then G' on M
   const size_t s_c = coarse ? a256(sizeof(float2) * B2 * B2) : 0;

@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "../engine.hpp"
+#include "band_plan.cuh"
 
 namespace huv_dev {
 
@@ -283,7 +284,6 @@ __global__ void __launch_bounds__(256) rect_rows(const int32_t* __restrict__ off
 // M(ky, kx) for clip c0 + blockIdx.y, band rows ky in [blockIdx.x * TY, +TY).
 // Thread t owns (ky, kx) pairs t, t + 256, ... of the tile; rows staged 16 at
 // a time.  Dynamic shared memory: 16 * (TY + B) double2.
-constexpr int kRectTY = 16;
 // The rows of clip c are clip_rows[c] .. clip_rows[c + 1] (resolved on the
 // host), or, with `counts`, the counts[c].y - 1 rows from 2 (clip_rows[c] -
 // clip_rows[0]) on (clip_rows = the clips' rectangle offsets).

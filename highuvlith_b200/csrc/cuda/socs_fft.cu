@@ -22,6 +22,7 @@
 
 #include <algorithm>
 
+#include "band_plan.cuh"
 #include "fft_block.cuh"
 #include "fft_reg.cuh"
 
@@ -700,8 +701,8 @@ cudaError_t socs_cols(const float2* T, int K, int hb, int lgm, int clips, float 
                       const float* mean, float* out, int mode, const float2* tw, cudaStream_t st);
 
 // Mask (or image) band: rows then columns.  When W is given, `mean` must hold
-// clips + clips * ceil(B / 4) floats: the first `clips` receive the flare
-// means, the rest holds the per-block parts.  `row_digits` (may be NULL) is
+// clips (1 + band_mean_parts(n, hb)) floats: the first `clips` receive the
+// flare means, the rest holds the per-block parts.  `row_digits` (may be NULL) is
 // the device digit table of the tensor-core row band for u8 rasters; `err`
 // receives that kernel's timeout code.
 cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int clips, float2* X,
@@ -806,9 +807,7 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
   float* parts = (W && mean) ? mean + clips : nullptr;
   int nblk;
   if (cols_reg) {
-    // register-radix columns: S <= 4 ... 32 columns per block, at most
-    // ceil(B / 4) parts per clip as the callers size them
-    const int S = xt_S(n);
+    const int S = band_cols_per_block(n, hb);
     nblk = ((half ? hb + 1 : B) + S - 1) / S;
     const dim3 g(nblk, clips);
     const size_t sm = xt_buf_bytes(n);
@@ -825,7 +824,7 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
     }
   } else {
     if (!pow2) return cudaErrorInvalidValue;
-    const int cpb = fit_units(4, 2 * (sizeof(float2) << lg));
+    const int cpb = band_cols_per_block(n, hb);
     nblk = (B + cpb - 1) / cpb;
     const size_t sm2 = 2 * (static_cast<size_t>(cpb) << lg) * sizeof(float2);
     band_cols_fwd<<<dim3(nblk, clips), 256, sm2, st>>>(X, lg, hb, cpb, ptx, W, Mband, parts, tw);
@@ -834,17 +833,8 @@ cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int cl
   return cudaGetLastError();
 }
 
-// Whether the register-radix kernels (x-major band layout) apply to length
-// L (128, 160, 192, 256, 512, 1024, 2048) and band half-width hb: every one of
-// them within the shared-memory budget.
-bool xt_ok(int L, int hb) {
-  const int S = xt_S(L);
-  if (S == 0 || 2 * hb >= L) return false;
-  // the largest user: the column pass with two band buffers and two FFT buffers
-  const size_t cols = 2 * static_cast<size_t>(S) * (2 * hb + 1) * sizeof(float2) +
-                      2 * static_cast<size_t>(fr_buf(L, S)) * sizeof(float2);
-  return cols <= static_cast<size_t>(kXtSmemMax);
-}
+bool xt_ok(int L, int hb) { return xt_fits(L, hb); }
+int band_mean_parts(int n, int hb) { return huv_dev::band_mean_parts(n, hb); }
 
 static int ilog2_exact(int v) {
   int l = 0;

@@ -1159,7 +1159,7 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
   const size_t per_c = sep ? 0 : align256(sizeof(float2) * B2 * B2);
   // Z^T of the two-kernel separable interpolation, or the Hermitian half band
   const size_t per_bi = sep && interp_fused_ok(M, n) ? 0 : align256(static_cast<size_t>(2) * n * std::max(kbI, M) * 2);
-  const size_t per_mean = align256(sizeof(float) * (1 + (B + 3) / 4));
+  const size_t per_mean = align256(sizeof(float) * (1 + band_mean_parts(n, hb)));
   const size_t per_clip = per_x + per_m + per_be + per_p + per_i + per_x2 + per_c + per_bi + per_mean;
   // a C2 step (256 clips) runs as one chunk of the engine's own workspace, so
   // the column pass (2 blocks per SM, 10 blocks per clip) fills whole waves

@@ -590,7 +590,7 @@ void Engine::run_fft_form(const huv_batch& b, DeviceSet& ds, int M, float* out, 
   const size_t per_x2 = coarse ? align256(sizeof(float2) * M * B2) : 0;
   const size_t per_c = coarse ? align256(sizeof(float2) * B2 * B2) : 0;
   const size_t per_t2 = coarse ? align256(sizeof(float2) * static_cast<size_t>(B2) * n) : 0;
-  const size_t per_mean = align256(sizeof(float) * (1 + (B + 3) / 4));
+  const size_t per_mean = align256(sizeof(float) * (1 + huv_launch::band_mean_parts(n, hb)));
   const size_t per_clip = per_x + per_m + per_t + per_i + per_x2 + per_c + per_t2 + per_mean;
   // a C2 step (256 clips) runs as one chunk of the engine's own workspace, so
   // the column pass (2 blocks per SM, 10 blocks per clip) fills whole waves

@@ -20,6 +20,8 @@ namespace huv_launch {
 cudaError_t band_forward(const void* in, int kind, int n, int lg, int hb, int clips, float2* X, float2* Mband,
                          const float* ptx, const float* W, float* mean, const float2* tw, cudaStream_t st,
                          const uint8_t* row_digits, int* err, bool radix4_rows = false);
+// Partial sums of one clip's flare mean, at most (csrc/cuda/band_plan.cuh).
+int band_mean_parts(int n, int hb);
 }  // namespace huv_launch
 
 namespace huv {
