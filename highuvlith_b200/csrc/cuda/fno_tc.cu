@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2)
     // dW rows o = lanes 0..63 of the second accumulator, once every MMA is complete
     if (quad < 2) {
       const bool fin = __all_sync(0xffffffffu, mbar_wait(done, 0, kFnoWaitNs));
-      if (fin && !*abort_flag) {
+      if (__all_sync(0xffffffffu, fin && !*abort_flag)) {  // one finding per warp: tcgen05.ld is .sync.aligned
         tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + 128;
         // through the staging tiles, so that a warp's atomics cover 128
@@ -727,6 +727,7 @@ struct FnoProjBwdParams {
   float* dQ2;         // [128]
   float* db2;         // [1]
   int* err;
+  unsigned long long probe_wait_ns;  // one warp's wait at the end runs out after this time (0: none)
 };
 
 __global__ void __launch_bounds__(kPbThreads, 2)
@@ -944,9 +945,21 @@ __global__ void __launch_bounds__(kPbThreads, 2)
     // every TMA store must have finished before the CTA's shared memory goes
     if (lane == 0 && nst > 0) bulk_wait<0>();
     __syncwarp();
-    // weight-gradient sums: rows j = lanes of the quadrant
-    const bool fin = __all_sync(0xffffffffu, mbar_wait(done, 0, kFnoWaitNs));
-    if (fin && !*abort_flag) {
+    // weight-gradient sums: rows j = lanes of the quadrant.  Whether they are
+    // added is each warp's own finding (its wait, or the flag of another's):
+    // the barrier of the db2 sum lies outside, where every warp comes by.
+    const bool fin = __all_sync(0xffffffffu, mbar_wait(done, 0, kFnoWaitNs) &&
+                                                 (!p.probe_wait_ns || half != 0 || quad != 1 ||
+                                                  mbar_wait(done, 1, p.probe_wait_ns)));  // no second phase comes
+    const bool add = __all_sync(0xffffffffu, fin && !*abort_flag);
+    if (half == 0) {
+#pragma unroll
+      for (int sh = 16; sh > 0; sh >>= 1) gd2 += __shfl_xor_sync(0xffffffffu, gd2, sh);
+      if (lane == 0) sd2[quad] = gd2;
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      if (add && quad == 0 && lane == 0) atomicAdd(p.db2, (sd2[0] + sd2[1]) + (sd2[2] + sd2[3]));
+    }
+    if (add) {
       tc_fence_after();
       const int j = quad * 32 + lane;
       float a[32];
@@ -969,11 +982,6 @@ __global__ void __launch_bounds__(kPbThreads, 2)
         tmem_ld16(tmem_base + lrow + cG, g);
         atomicAdd(p.db1 + j, b[0]);
         atomicAdd(p.dQ2 + j, g[0]);
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) gd2 += __shfl_xor_sync(0xffffffffu, gd2, sh);
-        if (lane == 0) sd2[quad] = gd2;
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-        if (quad == 0 && lane == 0) atomicAdd(p.db2, (sd2[0] + sd2[1]) + (sd2[2] + sd2[3]));
       }
     } else if (!fin && lane == 0) {
       fail(47);
@@ -1015,6 +1023,7 @@ __global__ void fno_tw_table(const float2* __restrict__ twx, int S, int m, __nv_
 }  // namespace huv_dev
 
 namespace huv_launch {
+unsigned long long probe_wait_ns();
 bool tc_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, int kp, int box_rows);
 
 bool tc_map_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols);
@@ -1122,6 +1131,7 @@ bool fno_tc_proj_bwd(size_t pix, const __nv_bfloat16* v, const float* Q1, const 
   p.dQ2 = dQ2;
   p.db2 = db2;
   p.err = err;
+  p.probe_wait_ns = probe_wait_ns();
   int sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;

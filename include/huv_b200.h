@@ -390,7 +390,8 @@ huv_status huv_device_status(void* engine, void* stream);
 /* Test hook for the give-up path of the bounded waits (no counterpart in
  * the reference).  ns > 0: every tensor-core GEMM launched afterwards (the
  * TC and hybrid forms) first waits ns nanoseconds on a barrier nothing
- * arrives at; the wait runs out, the kernel records the failure, unwinds
+ * arrives at, and one warp of the FNO's projection backward does so at the
+ * end; the wait runs out, the kernel records the failure, unwinds
  * (in-flight copies drained, tensor memory freed) and the next
  * huv_device_status reports HUV_ERR_DEVICE_TIMEOUT.  ns <= 0 turns it off
  * (the default).  Process-wide; not for production use. */
