@@ -945,7 +945,11 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   const bool sep = coarse && xt_fwd && separable_ok(ds, M);
   const size_t s_bi = sep && !interp_fused_ok(M, n) ? a256(sizeof(uint16_t) * 2 * static_cast<size_t>(n) * M) : 0;
   const size_t s_img = a256(sizeof(float) * npix);         // image on N, then G
-  const size_t s_V = grad ? a256(sizeof(float2) * static_cast<size_t>(K) * B * M) : 0;
+  // the adjoint's column transforms, then the FP16 planes of the gradient's interpolation
+  const bool grad_fused = sep && interp_fused_ok(M, n);
+  const size_t s_V = grad ? a256(std::max(sizeof(float2) * static_cast<size_t>(K) * B * M,
+                                          grad_fused ? 2 * sizeof(__half) * mpix : size_t(0)))
+                          : 0;
   const size_t s_q = grad ? a256(sizeof(float2) * B * B) : 0;
   const size_t s_t2 = grad ? a256(sizeof(float2) * static_cast<size_t>(B) * n) : 0;
   // few masks of a narrow band: the fields kept one by one (socs_cols_few)
@@ -1090,7 +1094,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       // columns per transform on the register-radix path
       hermitian_part<<<(nc * ((B * B + 1) / 2) + 255) / 256, 256, 0, st>>>(Q, B, nc);
       dcdm = tbuf;  // the transmittance is no longer needed
-      if (sep && interp_fused_ok(M, n)) {
+      if (grad_fused) {
         // dC/dm has band h: synthesised on the evaluation grid and
         // interpolated as the image is, 64 masks of 1024^2 in 0.09 ms instead
         // of 0.146 for 1024-point row and column transforms
