@@ -133,20 +133,30 @@ __device__ void bitonic(double* key, int16_t* val, int n) {
   __syncthreads();
 }
 
+// First rectangle of clip c and the clip's count.  Held within the `total`
+// rectangles that the tables are sized for: a caller's graph that captured a
+// call may be launched after other calls have brought other offsets.
+__device__ __forceinline__ int2 rect_span(const int32_t* __restrict__ offs, int c, int total) {
+  const int o0 = min(max(offs[c] - offs[0], 0), total);
+  return make_int2(o0, min(max(offs[c + 1] - offs[c], 0), total - o0));
+}
+
 // One block per clip: its rectangles, clipped to the field and with empty
 // ones left out, sorted by left edge into sorted[o0 ..], its distinct y edges
 // ascending into ys[2 o0 ..], and the counts (rectangles, edges).  Absent
 // entries sort as +infinity.  Shared memory: keys [2 cap], values [cap], cap =
 // the power of two that holds the largest clip.
 __global__ void __launch_bounds__(256) rect_sort(const double* __restrict__ rects, const int32_t* __restrict__ offs,
-                                                  double half, int cap, double4* __restrict__ sorted,
+                                                  int total, double half, int cap, double4* __restrict__ sorted,
                                                   double* __restrict__ ys, int2* __restrict__ counts) {
   extern __shared__ double rsm[];
   double* key = rsm;                                          // [2 cap]
   int16_t* val = reinterpret_cast<int16_t*>(key + 2 * cap);  // [cap]
   __shared__ int s_n;
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
-  const int c = blockIdx.x, o0 = offs[c] - offs[0], n = offs[c + 1] - offs[c];
+  const int c = blockIdx.x;
+  const int2 span = rect_span(offs, c, total);
+  const int o0 = span.x, n = min(span.y, cap);
   const double* q = rects + 4 * static_cast<size_t>(o0);
   auto rect = [&](int i) {
     return make_double4(fmax(q[4 * i] - q[4 * i + 2] / 2.0, -half), fmin(q[4 * i] + q[4 * i + 2] / 2.0, half),
@@ -197,11 +207,11 @@ __global__ void __launch_bounds__(256) rect_sort(const double* __restrict__ rect
 
 // g_m(x) = e^{-2 pi i m x / L} / (-2 pi i m), g_0 = x / L, for every order of
 // the band: EX[rect][left, right][B], EY[y edge][B].  One thread per value.
-__global__ void __launch_bounds__(256) rect_edges(const int32_t* __restrict__ offs, const int2* __restrict__ counts,
+__global__ void __launch_bounds__(256) rect_edges(const int32_t* __restrict__ offs, int rects, const int2* __restrict__ counts,
                                                    const double4* __restrict__ sorted, const double* __restrict__ ys,
                                                    int h, double L, double2* __restrict__ EX,
                                                    double2* __restrict__ EY) {
-  const int c = blockIdx.y, o0 = offs[c] - offs[0], B = 2 * h + 1;
+  const int c = blockIdx.y, o0 = rect_span(offs, c, rects).x, B = 2 * h + 1;
   const int2 n = counts[c];
   const int nx = 2 * n.x, total = (nx + n.y) * B;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -222,11 +232,11 @@ __global__ void __launch_bounds__(256) rect_edges(const int32_t* __restrict__ of
 // One warp per row j of a clip (between its y edges j and j + 1): X[j][m] =
 // sum over the row's runs of g(right) - g(left), Y[j][m] = g(y_j+1) - g(y_j).
 // A run grows while the next covering rectangle starts at or before its end.
-__global__ void __launch_bounds__(256) rect_rows(const int32_t* __restrict__ offs, const int2* __restrict__ counts,
+__global__ void __launch_bounds__(256) rect_rows(const int32_t* __restrict__ offs, int rects, const int2* __restrict__ counts,
                                                   const double4* __restrict__ sorted, const double* __restrict__ ys,
                                                   const double2* __restrict__ EX, const double2* __restrict__ EY, int h,
                                                   double2* __restrict__ X, double2* __restrict__ Y) {
-  const int c = blockIdx.y, o0 = offs[c] - offs[0], B = 2 * h + 1, lane = threadIdx.x & 31;
+  const int c = blockIdx.y, o0 = rect_span(offs, c, rects).x, B = 2 * h + 1, lane = threadIdx.x & 31;
   const int2 n = counts[c];
   const size_t e0 = 2 * static_cast<size_t>(o0);
   for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j + 1 < n.y; j += (gridDim.x * blockDim.x) >> 5) {
@@ -285,9 +295,9 @@ __global__ void __launch_bounds__(256) rect_rows(const int32_t* __restrict__ off
 // Thread t owns (ky, kx) pairs t, t + 256, ... of the tile; rows staged 16 at
 // a time.  Dynamic shared memory: 16 * (TY + B) double2.
 // The rows of clip c are clip_rows[c] .. clip_rows[c + 1] (resolved on the
-// host), or, with `counts`, the counts[c].y - 1 rows from 2 (clip_rows[c] -
-// clip_rows[0]) on (clip_rows = the clips' rectangle offsets).
-__global__ void __launch_bounds__(256) rect_band_gemm(const int32_t* __restrict__ clip_rows,
+// host), or, with `counts`, the counts[c].y - 1 rows from twice the clip's first
+// rectangle on (clip_rows = the offsets of the clips among `rects` rectangles).
+__global__ void __launch_bounds__(256) rect_band_gemm(const int32_t* __restrict__ clip_rows, int rects,
                                                        const int2* __restrict__ counts, const double2* __restrict__ X, const double2* __restrict__ Y,
                                                        int c0, int h, int n, double2 dv, double2 bgn2,
                                                        const float* __restrict__ W, float2* __restrict__ Mband,
@@ -300,7 +310,7 @@ __global__ void __launch_bounds__(256) rect_band_gemm(const int32_t* __restrict_
   const int ty = min(TY, B - ky0);
   double2* sy = rs;               // [16][TY]
   double2* sx = rs + 16 * TY;     // [16][B]
-  const int j0 = counts ? 2 * (clip_rows[cg] - clip_rows[0]) : clip_rows[cg];
+  const int j0 = counts ? 2 * rect_span(clip_rows, cg, rects).x : clip_rows[cg];
   const int j1 = counts ? j0 + max(counts[cg].y - 1, 0) : clip_rows[cg + 1];
   const int nout = ty * B;
   double2 acc[MAXE];
@@ -508,8 +518,17 @@ void Engine::upload_rects(const huv_batch& b, int hb, cudaStream_t st) {
     rect.stage.resize(rb + ob);
     if (total > 0) std::memcpy(rect.stage.data(), in->rects + in->offsets[0], rb);
     std::memcpy(rect.stage.data() + rb, in->offsets, ob);
-    grow(rect.rows, rect.rows_cap, rb + ob);
-    check_cuda(cudaMemcpyAsync(rect.rows, rect.stage.data(), rb + ob, cudaMemcpyHostToDevice, st), "upload rects");
+    grow(rect.dev, rect.dev_cap, rb + ob);
+    // Inside a stream capture an asynchronous copy would become a node that
+    // reads `stage` at every launch of the graph, when the vector may long have
+    // moved.  The synchronous copy is made there and then, as the copies of the
+    // host-resolved tables are.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    check_cuda(cudaStreamIsCapturing(st, &capture), "cudaStreamIsCapturing");
+    check_cuda(capture == cudaStreamCaptureStatusNone
+                   ? cudaMemcpyAsync(rect.dev, rect.stage.data(), rb + ob, cudaMemcpyHostToDevice, st)
+                   : cudaMemcpy(rect.dev, rect.stage.data(), rb + ob, cudaMemcpyHostToDevice),
+               "upload rects");
     return;
   }
   std::vector<int32_t> clip_rows;
@@ -553,18 +572,18 @@ void Engine::rect_band(int c0, int nc, int hb, const float* W, float2* Mband, fl
   double4* sorted = reinterpret_cast<double4*>((reinterpret_cast<uintptr_t>(EX + n_edges * B) + 31) & ~uintptr_t(31));
   double* ys = reinterpret_cast<double*>(sorted + (n_rows + 1) / 2);
   int2* counts = reinterpret_cast<int2*>(ys + n_rows);
-  const int32_t* offs = rect.on_device ? reinterpret_cast<const int32_t*>(static_cast<const huv_rect*>(rect.rows) + rect.total)
+  const int32_t* offs = rect.on_device ? reinterpret_cast<const int32_t*>(static_cast<const huv_rect*>(rect.dev) + rect.total)
                                        : static_cast<const int32_t*>(rect.clip_rows);
   if (rect.on_device) {
     if (c0 == 0) {
       int cap = 1;
       while (cap < rect.most) cap <<= 1;
       huv_dev::rect_sort<<<rect.clips, 256, cap * (2 * sizeof(double) + sizeof(int16_t)), st>>>(
-          static_cast<const double*>(rect.rows), offs, L / 2.0, cap, sorted, ys, counts);
+          static_cast<const double*>(rect.dev), offs, rect.total, L / 2.0, cap, sorted, ys, counts);
       const int vals = 4 * std::max(rect.most, 1) * B, rows = 2 * std::max(rect.most, 1);
-      huv_dev::rect_edges<<<dim3(std::min((vals + 255) / 256, 64), rect.clips), 256, 0, st>>>(offs, counts, sorted, ys, hb,
+      huv_dev::rect_edges<<<dim3(std::min((vals + 255) / 256, 64), rect.clips), 256, 0, st>>>(offs, rect.total, counts, sorted, ys, hb,
                                                                                              L, EX, EY);
-      huv_dev::rect_rows<<<dim3(std::min((rows + 7) / 8, 64), rect.clips), 256, 0, st>>>(offs, counts, sorted, ys, EX, EY,
+      huv_dev::rect_rows<<<dim3(std::min((rows + 7) / 8, 64), rect.clips), 256, 0, st>>>(offs, rect.total, counts, sorted, ys, EX, EY,
                                                                                         hb, X, Y);
       check_cuda(cudaGetLastError(), "rect_rows");
     }
@@ -580,7 +599,7 @@ void Engine::rect_band(int c0, int nc, int hb, const float* W, float2* Mband, fl
   const double n2 = static_cast<double>(n) * n;
   const size_t sm = sizeof(double2) * 16 * (huv_dev::kRectTY + B);
   huv_dev::rect_band_gemm<<<dim3(tiles, nc), 256, sm, st>>>(
-      offs, rect.on_device ? counts : nullptr, X, Y, c0, hb, n, rect.dv,
+      offs, rect.total, rect.on_device ? counts : nullptr, X, Y, c0, hb, n, rect.dv,
       make_double2(rect.bg.x * n2, rect.bg.y * n2), W, Mband, parts);
   check_cuda(cudaGetLastError(), "rect_band_gemm");
   if (parts) {

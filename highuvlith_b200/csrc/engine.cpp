@@ -205,6 +205,7 @@ Engine::~Engine() {
     cudaFree(rect.clip_rows);
     cudaFree(rect.rows);
     cudaFree(rect.runs);
+    cudaFree(rect.dev);
     cudaFree(rect.coef);
     if (io_h2d) {
       cudaStreamDestroy(io_h2d);

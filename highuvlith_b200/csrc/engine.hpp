@@ -363,9 +363,11 @@ struct Engine {
     void *clip_rows = nullptr, *rows = nullptr, *runs = nullptr, *coef = nullptr;
     size_t clip_rows_cap = 0, rows_cap = 0, runs_cap = 0, coef_cap = 0;
     int n_rows = 0;
-    // resolved on the device: rows holds the rectangles and, after them, the
+    // resolved on the device: dev holds the rectangles and, after them, the
     // clips' offsets; most = rectangles of the largest clip
     bool on_device = false;
+    void* dev = nullptr;
+    size_t dev_cap = 0;
     std::vector<uint8_t> stage;
     int most = 0, total = 0, clips = 0;
     double2 dv{0, 0}, bg{0, 0};
