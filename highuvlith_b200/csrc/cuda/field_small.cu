@@ -641,7 +641,7 @@ void Engine::run_small_form(const huv_batch& b, DeviceSet* const* sets, const in
   std::vector<SmallPlane> pl(planes);
   for (int p = 0; p < planes; ++p) {
     const int K = K_use && K_use[p] ? K_use[p] : sets[p]->K;
-    const BandKernels bk = kernels_for(b, *sets[p], K);
+    const BandKernels bk = kernels_for(b, *sets[p], K, st);
     pl[p] = SmallPlane{bk.kband, W_use && W_use[p] ? W_use[p] : sets[p]->W, bk.K, std::min(huv_dev::fs_split(M, K), bk.K),
                        sets[p]->keep, sets[p]->flare};
   }

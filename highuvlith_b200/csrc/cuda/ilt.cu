@@ -1054,7 +1054,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       // transforms, Engine::kernels_for) gives the same gradient; its row
       // transforms replace the forward's, which the image has consumed.
       const bool adj_small = !xt && ilt_adj_small_ok(M, hb);
-      const BandKernels ak = xt || adj_small ? kernels_for(real_kind, ds, K) : BandKernels{ds.kband, K};
+      const BandKernels ak = xt || adj_small ? kernels_for(real_kind, ds, K, st) : BandKernels{ds.kband, K};
       if (xt && ak.K < K)
         check_cuda(socs_rows_x(ak.kband, 0.f, Mb, ak.K, hb, M, nc, T, twm, st), "ilt adjoint rows");
       if (xt) {

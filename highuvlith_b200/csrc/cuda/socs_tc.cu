@@ -1082,7 +1082,7 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
   static std::atomic<uint64_t> smem_set{0};
   once_per_device(smem_set, [] { check_cuda(tc_set_smem(), "cudaFuncSetAttribute(tc)"); });
   const int lgn = ilog2i(n), lgm = ilog2i(M);  // lgm: log2 of M rounded up (M need not be a power of two)
-  const BandKernels bk = kernels_for(b, ds, K_use > 0 ? K_use : ds.K);
+  const BandKernels bk = kernels_for(b, ds, K_use > 0 ? K_use : ds.K, st);
   const int B = ds.B, K = bk.K, hb = ds.hb;
   const float* Wf = W_use ? W_use : ds.W;
   const int h2 = 2 * hb, B2 = 2 * h2 + 1;

@@ -464,12 +464,15 @@ void DeviceSet::release() {
   *this = DeviceSet();
 }
 
-Engine::BandKernels Engine::kernels_for(const huv_batch& b, DeviceSet& ds, int K) {
+Engine::BandKernels Engine::kernels_for(const huv_batch& b, DeviceSet& ds, int K, cudaStream_t st) {
   const bool real = b.input_kind == HUV_INPUT_RASTER_U8 || b.input_kind == HUV_INPUT_RASTER_F32 ||
                     (b.input_kind == HUV_INPUT_RECTS && rect.dv.y == 0.0 && rect.bg.y == 0.0);
   if (!real) return {ds.kband, K};
   auto it = ds.folded.find(K);
   if (it == ds.folded.end()) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    check_cuda(cudaStreamIsCapturing(st, &capture), "cudaStreamIsCapturing");
+    if (capture != cudaStreamCaptureStatusNone) return {ds.kband, K};
     DeviceSet::Folded f;
     FoldedKernels p;
     double div = ds.source->divisor(settings.normalization);
@@ -573,7 +576,7 @@ bool Engine::field_fused(const DeviceSet& ds, int M) const {
 void Engine::run_fft_form(const huv_batch& b, DeviceSet& ds, int M, float* out, cudaStream_t st, int K_use,
                           const float* W_use) {
   const int lgn = ilog2(n), lgm = ilog2(M);  // lgm: rounded up where M is 160, 192 or 384
-  const BandKernels bk = kernels_for(b, ds, K_use > 0 ? K_use : ds.K);
+  const BandKernels bk = kernels_for(b, ds, K_use > 0 ? K_use : ds.K, st);
   const int B = ds.B, K = bk.K, hb = ds.hb;
   const float* Wf = W_use ? W_use : ds.W;
   const bool coarse = M < n;

@@ -300,12 +300,13 @@ struct Engine {
                         cudaStream_t st, bool profile);
   // The band kernels to image the batch's input kind with: the first K of the
   // set, or, for real masks, their folded form (half as many) where the set
-  // has one.  Built on first use, kept with the set.
+  // has one.  Built on first use, kept with the set; inside a caller's capture
+  // of `st`, where nothing can be built, a set not folded yet is used as it is.
   struct BandKernels {
     const float2* kband;
     int K;
   };
-  BandKernels kernels_for(const huv_batch& b, DeviceSet& ds, int K);
+  BandKernels kernels_for(const huv_batch& b, DeviceSet& ds, int K, cudaStream_t st);
   // Flare weights W = sum_{k < K} lambda_k |u_k|^2 / N^4 of the first K kernels (device, cached).
   const float* flare_weights(DeviceSet& ds, int K);
   // Kernel count for a budget of `max_kernels` under the reference's truncation rule.
