@@ -717,7 +717,7 @@ struct Fno {
     check_cuda(cudaMalloc(&grad, npar * 4), "cudaMalloc(fno grad)");
     check_cuda(cudaMalloc(&m1, npar * 4), "cudaMalloc(fno m1)");
     check_cuda(cudaMalloc(&m2, npar * 4), "cudaMalloc(fno m2)");
-    check_cuda(cudaMemcpy(par, h.data(), npar * 4, cudaMemcpyHostToDevice), "upload fno params");
+    upload(par, h.data(), npar * 4, "upload fno params");
     check_cuda(cudaMemset(m1, 0, npar * 4), "memset");
     check_cuda(cudaMemset(m2, 0, npar * 4), "memset");
     std::vector<float2> tx(static_cast<size_t>(m) * S), txt(static_cast<size_t>(S) * 16, make_float2(0.f, 0.f)),
@@ -732,7 +732,7 @@ struct Fno {
       for (int y = 0; y < S; ++y) tyt_h[static_cast<size_t>(y) * 32 + j] = w(j < m ? j : j - J, y);
     auto table = [&](float2** d, const std::vector<float2>& h2) {
       check_cuda(cudaMalloc(d, h2.size() * 8), "cudaMalloc(fno twiddles)");
-      check_cuda(cudaMemcpy(*d, h2.data(), h2.size() * 8, cudaMemcpyHostToDevice), "upload fno twiddles");
+      upload(*d, h2.data(), h2.size() * 8, "upload fno twiddles");
     };
     table(&twx, tx);
     table(&twt, txt);
@@ -1024,7 +1024,7 @@ huv_status huv_fno_set_params(void* fno, const float* host, int64_t count) {
     Fno* f = as_fno(fno);
     if (!host || count != static_cast<int64_t>(f->npar)) throw Error(HUV_ERR_DIMENSION_MISMATCH, "fno params: count");
     huv::check_cuda(cudaSetDevice(f->device), "cudaSetDevice");
-    huv::check_cuda(cudaMemcpy(f->par, host, f->npar * 4, cudaMemcpyHostToDevice), "H2D params");
+    huv::upload(f->par, host, f->npar * 4, "H2D params");
   });
 }
 

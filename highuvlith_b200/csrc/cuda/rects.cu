@@ -498,6 +498,8 @@ void Engine::upload_rects(const huv_batch& b, int hb, cudaStream_t st) {
     check_cuda(cudaMalloc(&p, bytes), "cudaMalloc(rect table)");
     cap = bytes;
   };
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  check_cuda(cudaStreamIsCapturing(st, &capture), "cudaStreamIsCapturing");
   // Clips that fit rect_sort's shared memory are resolved on the device, as
   // long as the batch's tables (X, Y and both edge tables: 128 bytes per
   // rectangle and order) stay moderate; the copies are ordered on the stream.
@@ -523,8 +525,6 @@ void Engine::upload_rects(const huv_batch& b, int hb, cudaStream_t st) {
     // reads `stage` at every launch of the graph, when the vector may long have
     // moved.  The synchronous copy is made there and then, as the copies of the
     // host-resolved tables are.
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    check_cuda(cudaStreamIsCapturing(st, &capture), "cudaStreamIsCapturing");
     check_cuda(capture == cudaStreamCaptureStatusNone
                    ? cudaMemcpyAsync(rect.dev, rect.stage.data(), rb + ob, cudaMemcpyHostToDevice, st)
                    : cudaMemcpy(rect.dev, rect.stage.data(), rb + ob, cudaMemcpyHostToDevice),
@@ -539,13 +539,16 @@ void Engine::upload_rects(const huv_batch& b, int hb, cudaStream_t st) {
   grow(rect.clip_rows, rect.clip_rows_cap, sizeof(int32_t) * clip_rows.size());
   grow(rect.rows, rect.rows_cap, sizeof(huv_dev::RectRowDev) * std::max<size_t>(rows.size(), 1));
   grow(rect.runs, rect.runs_cap, sizeof(double2) * std::max<size_t>(runs.size(), 1));
-  check_cuda(cudaMemcpy(rect.clip_rows, clip_rows.data(), sizeof(int32_t) * clip_rows.size(), cudaMemcpyHostToDevice),
-             "upload rect rows");
+  auto copy = [&](void* dst, const void* src, size_t bytes) {
+    if (capture == cudaStreamCaptureStatusNone)
+      upload(dst, src, bytes, "upload rect table");
+    else  // no synchronisation inside a capture
+      check_cuda(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), "upload rect table");
+  };
+  copy(rect.clip_rows, clip_rows.data(), sizeof(int32_t) * clip_rows.size());
   if (!rows.empty()) {
-    check_cuda(cudaMemcpy(rect.rows, rows.data(), sizeof(huv_dev::RectRowDev) * rows.size(), cudaMemcpyHostToDevice),
-               "upload rect rows");
-    check_cuda(cudaMemcpy(rect.runs, runs.data(), sizeof(double2) * runs.size(), cudaMemcpyHostToDevice),
-               "upload rect runs");
+    copy(rect.rows, rows.data(), sizeof(huv_dev::RectRowDev) * rows.size());
+    copy(rect.runs, runs.data(), sizeof(double2) * runs.size());
   }
 }
 

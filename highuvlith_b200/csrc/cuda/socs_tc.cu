@@ -1121,7 +1121,7 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
       }
     const auto pe = split_planes(ae, 2 * M, kcE, kpE);
     check_cuda(cudaMalloc(&tc.gy, pe.size() * 2), "cudaMalloc(A_E)");
-    check_cuda(cudaMemcpy(tc.gy, pe.data(), pe.size() * 2, cudaMemcpyHostToDevice), "upload A_E");
+    upload(tc.gy, pe.data(), pe.size() * 2, "upload A_E");
     if (!make_map(&tc.map_ae, tc.gy, 2ull * 2 * M, kpE, 128))
       throw Error(HUV_ERR_CUDA, "cuTensorMapEncodeTiled failed for the DFT operands");
   }
@@ -1137,7 +1137,7 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
       }
     const auto pi = split_planes(ai, n, kcI, kpI);
     check_cuda(cudaMalloc(&tc.gx, pi.size() * 2), "cudaMalloc(A_I)");
-    check_cuda(cudaMemcpy(tc.gx, pi.data(), pi.size() * 2, cudaMemcpyHostToDevice), "upload A_I");
+    upload(tc.gx, pi.data(), pi.size() * 2, "upload A_I");
     if (!make_map(&tc.map_ai, tc.gx, 2ull * n, kpI, 128) ||
         !make_map_sw64(&tc.map_ai32, tc.gx, 2ull * n, kpI, 128, kpI, false))
       throw Error(HUV_ERR_CUDA, "cuTensorMapEncodeTiled failed for the DFT operands");
@@ -1383,7 +1383,7 @@ void Engine::interp_matrix(DeviceSet& ds, int M) {
           t[interp_tiled_offset(y, m, 1, M) / 2] = lo[index(y, m)];
         }
       check_cuda(cudaMalloc(&tc.gpt, t.size() * 2), "cudaMalloc(P tiles)");
-      check_cuda(cudaMemcpy(tc.gpt, t.data(), t.size() * 2, cudaMemcpyHostToDevice), "upload P tiles");
+      upload(tc.gpt, t.data(), t.size() * 2, "upload P tiles");
       return;
     }
     std::vector<double> pm(static_cast<size_t>(n) * M);
@@ -1391,7 +1391,7 @@ void Engine::interp_matrix(DeviceSet& ds, int M) {
       for (int m = 0; m < M; ++m) pm[static_cast<size_t>(y) * M + m] = val[index(y, m)];
     const auto pp = split_planes_f16(pm, n, M, kpP);
     check_cuda(cudaMalloc(&tc.gp, pp.size() * 2), "cudaMalloc(P)");
-    check_cuda(cudaMemcpy(tc.gp, pp.data(), pp.size() * 2, cudaMemcpyHostToDevice), "upload P");
+    upload(tc.gp, pp.data(), pp.size() * 2, "upload P");
     if (!make_map(&tc.map_pi, tc.gp, 2ull * n, kpP, 128, 0, true) ||
         !make_map_sw64(&tc.map_pi32, tc.gp, 2ull * n, kpP, 128, kpP, true))
       throw Error(HUV_ERR_CUDA, "cuTensorMapEncodeTiled failed for the interpolation operand");

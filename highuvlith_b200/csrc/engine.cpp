@@ -69,6 +69,11 @@ void check_cuda(cudaError_t e, const char* what) {
   }
 }
 
+void upload(void* dst, const void* src, size_t bytes, const char* what) {
+  check_cuda(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what);
+  check_cuda(cudaStreamSynchronize(cudaStreamLegacy), what);
+}
+
 // ------------------------------------------------------------ construction
 Engine::Engine(const huv_source& s, const huv_optics& o, const huv_grid& g, const huv_settings& st,
                int dev)
@@ -373,7 +378,7 @@ const float2* Engine::twiddle_n(int L) {
   }
   float2* d = nullptr;
   check_cuda(cudaMalloc(&d, sizeof(float2) * L), "cudaMalloc(twiddle)");
-  check_cuda(cudaMemcpy(d, h.data(), sizeof(float2) * L, cudaMemcpyHostToDevice), "cudaMemcpy(twiddle)");
+  upload(d, h.data(), sizeof(float2) * L, "cudaMemcpy(twiddle)");
   twiddles[L] = d;
   return d;
 }
@@ -386,7 +391,7 @@ const uint8_t* Engine::row_digit_table(int hb) {
   if (!(env && std::string(env) == "fft") && huv_launch::mask_rows_tc_supported(n, hb)) {
     const std::vector<uint8_t> h = huv_launch::mask_rows_tc_digits(n, hb);
     check_cuda(cudaMalloc(&d, h.size()), "cudaMalloc(row digits)");
-    check_cuda(cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice), "cudaMemcpy(row digits)");
+    upload(d, h.data(), h.size(), "cudaMemcpy(row digits)");
   }
   row_digits[hb] = d;
   return d;
@@ -447,9 +452,9 @@ DeviceSet& Engine::device_set(double z) {
   check_cuda(cudaMalloc(&d.kband, sizeof(float2) * d.host_kband.size()), "cudaMalloc(kband)");
   check_cuda(cudaMalloc(&d.W, sizeof(float) * wf.size()), "cudaMalloc(W)");
   check_cuda(cudaMalloc(&d.ptx, sizeof(float) * ptx.size()), "cudaMalloc(ptx)");
-  check_cuda(cudaMemcpy(d.kband, d.host_kband.data(), sizeof(float2) * d.host_kband.size(), cudaMemcpyHostToDevice), "upload kband");
-  check_cuda(cudaMemcpy(d.W, wf.data(), sizeof(float) * wf.size(), cudaMemcpyHostToDevice), "upload W");
-  check_cuda(cudaMemcpy(d.ptx, ptx.data(), sizeof(float) * ptx.size(), cudaMemcpyHostToDevice), "upload ptx");
+  upload(d.kband, d.host_kband.data(), sizeof(float2) * d.host_kband.size(), "upload kband");
+  upload(d.W, wf.data(), sizeof(float) * wf.size(), "upload W");
+  upload(d.ptx, ptx.data(), sizeof(float) * ptx.size(), "upload ptx");
   *slot = std::move(d);
   return *slot;
 }
@@ -482,8 +487,7 @@ Engine::BandKernels Engine::kernels_for(const huv_batch& b, DeviceSet& ds, int K
       for (size_t i = 0; i < 2 * p.size; ++i) h[i] = static_cast<float>(p.v[i]);
       check_cuda(cudaMalloc(&f.kband, sizeof(float2) * p.size), "cudaMalloc(folded kernels)");
       f.K = (K + 1) / 2;
-      check_cuda(cudaMemcpy(f.kband, h.get(), sizeof(float2) * p.size, cudaMemcpyHostToDevice),
-                 "upload folded kernels");
+      upload(f.kband, h.get(), sizeof(float2) * p.size, "upload folded kernels");
     }
     it = ds.folded.emplace(K, f).first;
   }
@@ -506,7 +510,7 @@ const float* Engine::flare_weights(DeviceSet& ds, int K) {
   for (size_t i = 0; i < wd.size(); ++i) w[i] = static_cast<float>(wd[i]);
   float* d = nullptr;
   check_cuda(cudaMalloc(&d, sizeof(float) * w.size()), "cudaMalloc(W prefix)");
-  check_cuda(cudaMemcpy(d, w.data(), sizeof(float) * w.size(), cudaMemcpyHostToDevice), "upload W prefix");
+  upload(d, w.data(), sizeof(float) * w.size(), "upload W prefix");
   ds.W_by_k[K] = d;
   return d;
 }

@@ -39,6 +39,10 @@ inline int balanced_chunk(int max_chunk, int n) {
 void set_last_error(const std::string& m);
 const char* last_error();
 void check_cuda(cudaError_t e, const char* what);
+// Copy of host memory to the device that has landed when the call returns.
+// cudaMemcpy may return with the end of a copy from pageable memory still on
+// its way on the legacy stream, and a non-blocking stream does not wait for it.
+void upload(void* dst, const void* src, size_t bytes, const char* what);
 
 // Runs fn once per CUDA device for settings that CUDA keeps per device
 // (function attributes): bit d of `done` is set after device d ran it.  Two

@@ -264,8 +264,7 @@ huv_status huv_plan_create(const huv_clip* clips, int32_t n_clips, int32_t pixel
           void** d = nullptr;
           huv::check_cuda(cudaMalloc(reinterpret_cast<void**>(&d), sizeof(void*) * 4 * nc),
                           "cudaMalloc(plan copy pointers)");
-          huv::check_cuda(cudaMemcpy(d, ptrs.data(), sizeof(void*) * 4 * nc, cudaMemcpyHostToDevice),
-                          "upload plan copy pointers");
+          huv::upload(d, ptrs.data(), sizeof(void*) * 4 * nc, "upload plan copy pointers");
           g.gather_src = const_cast<const void**>(d);
           g.gather_dst = d + nc;
           g.scatter_src = const_cast<const void**>(d + 2 * nc);
