@@ -1125,7 +1125,7 @@ void Engine::run_tc_form(const huv_batch& b, DeviceSet& ds, int M, float* out, c
     if (!make_map(&tc.map_ae, tc.gy, 2ull * 2 * M, kpE, 128))
       throw Error(HUV_ERR_CUDA, "cuTensorMapEncodeTiled failed for the DFT operands");
   }
-  if (!tc.gx) {
+  if (!sep && !tc.gx) {
     // A_I: rows y over the N grid, K = (qy >= 0, re/im), Hermitian weights.
     std::vector<double> ai(static_cast<size_t>(n) * kcI);
     for (int y = 0; y < n; ++y)
@@ -1378,9 +1378,13 @@ void Engine::interp_matrix(DeviceSet& ds, int M) {
         lo[j] = static_cast<__half_raw>(__float2half_rn(f - __half2float(h))).x;
       }
       for (int y = 0; y < n; ++y)
-        for (int m = 0; m < M; ++m) {
-          t[interp_tiled_offset(y, m, 0, M) / 2] = hi[index(y, m)];
-          t[interp_tiled_offset(y, m, 1, M) / 2] = lo[index(y, m)];
+        for (int m0 = 0; m0 < M; m0 += 8) {  // eight columns lie together
+          uint16_t* th = &t[interp_tiled_offset(y, m0, 0, M) / 2];
+          uint16_t* tl = &t[interp_tiled_offset(y, m0, 1, M) / 2];
+          for (int e = 0; e < 8; ++e) {
+            th[e] = hi[index(y, m0 + e)];
+            tl[e] = lo[index(y, m0 + e)];
+          }
         }
       check_cuda(cudaMalloc(&tc.gpt, t.size() * 2), "cudaMalloc(P tiles)");
       upload(tc.gpt, t.data(), t.size() * 2, "upload P tiles");

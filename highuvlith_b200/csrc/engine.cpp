@@ -360,7 +360,8 @@ void Engine::image_focus_sweep(const huv_batch& b, const double* z, int planes, 
 void Engine::ensure_device() {
   check_cuda(cudaSetDevice(device), "cudaSetDevice");
   if (device_ready) return;
-  check_cuda(huv_launch::set_smem_limits(), "cudaFuncSetAttribute");
+  static std::atomic<uint64_t> smem_set{0};
+  once_per_device(smem_set, [] { check_cuda(huv_launch::set_smem_limits(), "cudaFuncSetAttribute"); });
   check_cuda(cudaMalloc(&dev_err, sizeof(int)), "cudaMalloc(error flag)");
   check_cuda(cudaMemset(dev_err, 0, sizeof(int)), "cudaMemset(error flag)");
   device_ready = true;
@@ -419,17 +420,16 @@ DeviceSet& Engine::device_set(double z) {
   const double n2 = static_cast<double>(n) * n;
   std::vector<float2> kb(static_cast<size_t>(K) * B * B, make_float2(0.f, 0.f));
   std::vector<double> wd(static_cast<size_t>(B) * B, 0.0);
+  const std::vector<uint32_t> pos = ks->band_positions();
   for (int k = 0; k < K; ++k) {
     const double lam = ks->eigenvalues[k] / div;
     const double sc = std::sqrt(lam) / n2;
+    const cd* values = &ks->values[static_cast<size_t>(k) * S];
+    float2* band = &kb[static_cast<size_t>(k) * B * B];
     for (int t = 0; t < S; ++t) {
-      const int64_t idx = ks->support[t];
-      const int i = static_cast<int>(idx / n), j = static_cast<int>(idx % n);
-      const int my = i < n / 2 ? i : i - n, mx = j < n / 2 ? j : j - n;
-      const cd u = ks->values[static_cast<size_t>(k) * S + t];
-      const size_t o = (static_cast<size_t>(my + h)) * B + (mx + h);
-      kb[static_cast<size_t>(k) * B * B + o] = make_float2(static_cast<float>(u.real() * sc), static_cast<float>(u.imag() * sc));
-      wd[o] += lam * std::norm(u) / (n2 * n2);
+      const cd u = values[t];
+      band[pos[t]] = make_float2(static_cast<float>(u.real() * sc), static_cast<float>(u.imag() * sc));
+      wd[pos[t]] += lam * std::norm(u) / (n2 * n2);
     }
   }
   std::vector<float> wf(wd.begin(), wd.end());
@@ -449,12 +449,16 @@ DeviceSet& Engine::device_set(double z) {
   d.eig_scaled.resize(K);
   for (int k = 0; k < K; ++k) d.eig_scaled[k] = ks->eigenvalues[k] / div;
   d.host_kband = std::move(kb);
-  check_cuda(cudaMalloc(&d.kband, sizeof(float2) * d.host_kband.size()), "cudaMalloc(kband)");
-  check_cuda(cudaMalloc(&d.W, sizeof(float) * wf.size()), "cudaMalloc(W)");
-  check_cuda(cudaMalloc(&d.ptx, sizeof(float) * ptx.size()), "cudaMalloc(ptx)");
-  upload(d.kband, d.host_kband.data(), sizeof(float2) * d.host_kband.size(), "upload kband");
-  upload(d.W, wf.data(), sizeof(float) * wf.size(), "upload W");
-  upload(d.ptx, ptx.data(), sizeof(float) * ptx.size(), "upload ptx");
+  // one allocation: [kernels][W][ptx], each on a 256-byte boundary
+  const size_t kb_bytes = sizeof(float2) * d.host_kband.size();
+  const size_t w0 = (kb_bytes + 255) & ~size_t(255), nw = (wf.size() + 63) & ~size_t(63);
+  check_cuda(cudaMalloc(&d.kband, w0 + sizeof(float) * (nw + ptx.size())), "cudaMalloc(kernel set)");
+  d.W = reinterpret_cast<float*>(reinterpret_cast<char*>(d.kband) + w0);
+  d.ptx = d.W + nw;
+  wf.resize(nw, 0.f);
+  wf.insert(wf.end(), ptx.begin(), ptx.end());
+  check_cuda(cudaMemcpy(d.kband, d.host_kband.data(), kb_bytes, cudaMemcpyHostToDevice), "upload kband");
+  upload(d.W, wf.data(), sizeof(float) * wf.size(), "upload W and ptx");
   *slot = std::move(d);
   return *slot;
 }
@@ -462,9 +466,7 @@ DeviceSet& Engine::device_set(double z) {
 void DeviceSet::release() {
   for (auto& kv : W_by_k) cudaFree(kv.second);
   for (auto& kv : folded) cudaFree(kv.second.kband);
-  cudaFree(kband);
-  cudaFree(W);
-  cudaFree(ptx);
+  cudaFree(kband);  // and W and ptx behind it
   huv_launch::tc_release_all(tc);
   *this = DeviceSet();
 }
@@ -479,15 +481,14 @@ Engine::BandKernels Engine::kernels_for(const huv_batch& b, DeviceSet& ds, int K
     check_cuda(cudaStreamIsCapturing(st, &capture), "cudaStreamIsCapturing");
     if (capture != cudaStreamCaptureStatusNone) return {ds.kband, K};
     DeviceSet::Folded f;
-    FoldedKernels p;
+    std::unique_ptr<float[]> h;
+    size_t size = 0;
     double div = ds.source->divisor(settings.normalization);
     if (div == 0.0) div = 1.0;
-    if (fold_real_kernels(*ds.source, K, div, p)) {
-      std::unique_ptr<float[]> h(new float[2 * p.size]);
-      for (size_t i = 0; i < 2 * p.size; ++i) h[i] = static_cast<float>(p.v[i]);
-      check_cuda(cudaMalloc(&f.kband, sizeof(float2) * p.size), "cudaMalloc(folded kernels)");
+    if (fold_real_kernels(*ds.source, K, div, h, size)) {
+      check_cuda(cudaMalloc(&f.kband, sizeof(float2) * size), "cudaMalloc(folded kernels)");
       f.K = (K + 1) / 2;
-      upload(f.kband, h.get(), sizeof(float2) * p.size, "upload folded kernels");
+      upload(f.kband, h.get(), sizeof(float2) * size, "upload folded kernels");
     }
     it = ds.folded.emplace(K, f).first;
   }

@@ -70,6 +70,8 @@ struct KernelSet {
   double defocus_nm = 0, wavelength_nm = 0;
   int num_kernels() const { return static_cast<int>(eigenvalues.size()); }
   int band_half_width() const;     // max |order| over the support
+  // index of every support point in a band [2 h + 1][2 h + 1], h = band_half_width()
+  std::vector<uint32_t> band_positions() const;
   double divisor(int normalization) const;  // 0 if images stay absolute
 };
 
@@ -82,6 +84,8 @@ struct FoldedKernels {
   cd operator[](size_t i) const { return cd(v[2 * i], v[2 * i + 1]); }
 };
 bool fold_real_kernels(const KernelSet& ks, int K, double div, FoldedKernels& folded);
+// The same rounded to FP32, `size` complex values as (re, im) pairs.
+bool fold_real_kernels(const KernelSet& ks, int K, double div, std::unique_ptr<float[]>& v, size_t& size);
 
 int select_kernel_count(const std::vector<double>& values, double trace, int max_kernels,
                         double fraction);

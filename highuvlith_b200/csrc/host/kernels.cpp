@@ -486,6 +486,16 @@ int KernelSet::band_half_width() const {
   return h;
 }
 
+std::vector<uint32_t> KernelSet::band_positions() const {
+  const int h = band_half_width(), B = 2 * h + 1;
+  std::vector<uint32_t> pos(support.size());
+  for (size_t t = 0; t < support.size(); ++t) {
+    const int i = static_cast<int>(support[t] / n), j = static_cast<int>(support[t] % n);
+    pos[t] = static_cast<uint32_t>(((i < n / 2 ? i : i - n) + h) * B + ((j < n / 2 ? j : j - n) + h));
+  }
+  return pos;
+}
+
 double KernelSet::divisor(int normalization) const {
   const bool bright = clear_field > 0.0 && clear_field >= 1e-2 * pupil_peak;
   return (normalization == 0 && bright) ? clear_field : 0.0;
