@@ -8,7 +8,9 @@
 // candidates on the group's own clips, pre-allocates every buffer, runs the
 // whole batch once, and captures it into a CUDA graph.  huv_plan_launch is
 // then one cudaGraphLaunch for the whole uneven batch.  Tuning results are
-// cached per (grid, band, kernel count, input kind) for the process.
+// cached for the process per (grid, band, kernel count, transforms per clip,
+// input kind); the transforms tell sets that fold for real masks from sets
+// that do not, whose times differ by up to two.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,7 +40,7 @@ struct Choice {
 };
 
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, Choice> g_tuned;  // (N, h, K, kind) -> choice
+std::map<std::tuple<int, int, int, int, int>, Choice> g_tuned;  // (N, h, K, transforms, kind) -> choice
 
 size_t elem_size(int kind) { return kind == HUV_INPUT_RASTER_U8 ? 1 : (kind == HUV_INPUT_RASTER_F32 ? 4 : 8); }
 
@@ -272,7 +274,9 @@ huv_status huv_plan_create(const huv_clip* clips, int32_t n_clips, int32_t pixel
           g.copy_kernel = true;
         }
       }
-      const auto key = std::make_tuple(g.n, g.h, g.K, g.kind);
+      huv_batch kind{};
+      kind.input_kind = g.kind;
+      const auto key = std::make_tuple(g.n, g.h, g.K, g.e->kernels_for(kind, ds, g.K, st).K, g.kind);
       bool cached = false;
       {
         std::lock_guard<std::mutex> tl(huv::g_tune_mu);
