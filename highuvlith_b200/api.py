@@ -461,10 +461,17 @@ class SimulationEngine:
     def _rect_clips(clips, feature, background):
         """ctypes view of rectangle clips (centre x, y and size w, h in nm,
         field-centred coordinates); keeps the arrays alive on the view."""
+        rects = None
         try:
-            rects = np.concatenate([np.asarray(c, dtype=np.float64).reshape(len(c), 4) for c in clips] or [np.zeros((0, 4))])
-        except (TypeError, ValueError):  # rectangles of other number types
+            tables = [np.asarray(c, dtype=np.float64) for c in clips]
+            if all(t.shape == (len(c), 4) for t, c in zip(tables, clips) if len(c)):
+                rects = np.concatenate([t.reshape(-1, 4) for t in tables] or [np.zeros((0, 4))])
+        except (TypeError, ValueError):
+            pass
+        if rects is None or np.isnan(rects).any():  # one by one: other number types, and the errors of what is none
             flat = [tuple(map(float, r)) for c in clips for r in c]
+            if any(len(r) != 4 for r in flat):
+                raise ValueError("rectangles must be (x, y, w, h)")
             rects = np.ascontiguousarray(np.asarray(flat, dtype=np.float64).reshape(-1, 4))
         offs = np.zeros(len(clips) + 1, dtype=np.int32)
         offs[1:] = np.cumsum([len(c) for c in clips])
