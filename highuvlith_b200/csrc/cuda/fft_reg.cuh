@@ -546,7 +546,7 @@ __host__ __device__ __forceinline__ void fr_last_pass_pre(int u, const float2* s
 // so their scale does not depend on the normalisation, and a non-negative
 // band-limited image on M^2 points (max <= M^2 mean) stays below M^2 / 16
 // (2304 at M = 192), far inside FP16's range.  The limits keep s and 1 / s
-// finite; between them faint images and gradients keep FP32's range.
+// finite; between them faint images keep FP32's range.
 __device__ __forceinline__ float interp_scale(float mean) { return 16.f * fminf(fmaxf(mean, 1e-36f), 2e37f); }
 
 }  // namespace huv_dev

@@ -10,7 +10,6 @@
 //     Q = sum_k conj(kappa_k) . band(FFT(G0 . E_k)),   dC/dm = 2 (1 - a) Re IFFT(Q)
 // with E_k = IFFT(kappa_k . M) on the full grid and kappa_k the pre-scaled band
 // kernels (sqrt(lambda_k) / N^2 folded in), G0 = (1 - phi) dC/dI + phi mean(dC/dI).
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -125,33 +124,6 @@ __global__ void __launch_bounds__(128) sum_parts(const double* __restrict__ part
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) out[t] = s;
-}
-
-// FP16 hi/lo planes of v / interp_scale(mean) for a signed image v on L x L
-// points, with mean[mask] chosen so that the largest |v| becomes 1024: the
-// separable interpolation's operand (csrc/cuda/interp_tc.cu).  grid: masks.
-__global__ void __launch_bounds__(1024) split_signed(const float* __restrict__ v, int n, float* __restrict__ mean,
-                                                      __half* __restrict__ planes) {
-  __shared__ float red[32];
-  const float* x = v + static_cast<size_t>(blockIdx.x) * n;
-  float m = 0.f;
-  for (int i = threadIdx.x; i < n; i += 1024) m = fmaxf(m, fabsf(x[i]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  m = red[threadIdx.x & 31];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  const float mn = m * (1.f / 16384.f), inv = 1.f / interp_scale(mn);
-  if (threadIdx.x == 0) mean[blockIdx.x] = mn;
-  __half* hi = planes + static_cast<size_t>(blockIdx.x) * 2 * n;
-  for (int i = threadIdx.x; i < n; i += 1024) {
-    const float s = x[i] * inv;
-    const __half h = __float2half_rn(s);
-    hi[i] = h;
-    hi[n + i] = __float2half_rn(s - __half2float(h));
-  }
 }
 
 // Adjoint column pass.  CTA per (mask, strip of Wc columns): for every kernel
@@ -945,11 +917,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
   const bool sep = coarse && xt_fwd && separable_ok(ds, M);
   const size_t s_bi = sep && !interp_fused_ok(M, n) ? a256(sizeof(uint16_t) * 2 * static_cast<size_t>(n) * M) : 0;
   const size_t s_img = a256(sizeof(float) * npix);         // image on N, then G
-  // the adjoint's column transforms, then the FP16 planes of the gradient's interpolation
-  const bool grad_fused = sep && interp_fused_ok(M, n);
-  const size_t s_V = grad ? a256(std::max(sizeof(float2) * static_cast<size_t>(K) * B * M,
-                                          grad_fused ? 2 * sizeof(__half) * mpix : size_t(0)))
-                          : 0;
+  const size_t s_V = grad ? a256(sizeof(float2) * static_cast<size_t>(K) * B * M) : 0;
   const size_t s_q = grad ? a256(sizeof(float2) * B * B) : 0;
   const size_t s_t2 = grad ? a256(sizeof(float2) * static_cast<size_t>(B) * n) : 0;
   // few masks of a narrow band: the fields kept one by one (socs_cols_few)
@@ -1094,19 +1062,12 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       // columns per transform on the register-radix path
       hermitian_part<<<(nc * ((B * B + 1) / 2) + 255) / 256, 256, 0, st>>>(Q, B, nc);
       dcdm = tbuf;  // the transmittance is no longer needed
-      if (grad_fused) {
-        // dC/dm has band h: synthesised on the evaluation grid and
-        // interpolated as the image is, 64 masks of 1024^2 in 0.09 ms instead
-        // of 0.146 for 1024-point row and column transforms
-        check_cuda(socs_rows_x(nullptr, scale, Q, 1, hb, M, nc, X2, twm, st), "ilt grad rows");
-        check_cuda(socs_cols_x(X2, 1, hb, M, nc, 1.f, 0.f, nullptr, IM, 1, twm, st), "ilt grad cols");
-        __half* planes = reinterpret_cast<__half*>(V);  // the adjoint fields are no longer needed
-        split_signed<<<nc, 1024, 0, st>>>(IM, static_cast<int>(mpix), mean, planes);
-        interp_separable(ds, M, nc, planes, mean, nullptr, dcdm, st, false);
-      } else {
-        check_cuda(socs_rows_x(nullptr, scale, Q, 1, hb, n, nc, T2, twn, st), "ilt grad rows");
-        check_cuda(socs_cols_x(T2, 1, hb, n, nc, 1.f, 0.f, nullptr, dcdm, 1, twn, st), "ilt grad cols");
-      }
+      // (N-point transforms in FP32: through the FP16 hi/lo operands of the
+      // image's interpolation it took 0.09 ms instead of 0.146 for 64 masks of
+      // 1024^2, but the gradient came out further from FP64, 3.3e-6 against
+      // 3.0e-6 on average over masks of 512^2 and 1024^2)
+      check_cuda(socs_rows_x(nullptr, scale, Q, 1, hb, n, nc, T2, twn, st), "ilt grad rows");
+      check_cuda(socs_cols_x(T2, 1, hb, n, nc, 1.f, 0.f, nullptr, dcdm, 1, twn, st), "ilt grad cols");
     }
     // 16-byte accesses of theta and the gradient (a caller's planes may lie anywhere)
     const bool vec16 = ((reinterpret_cast<uintptr_t>(th) | reinterpret_cast<uintptr_t>(grad)) & 15u) == 0;

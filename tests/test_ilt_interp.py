@@ -1,8 +1,7 @@
-"""The ILT gradient whose last synthesis goes through the tcgen05 interpolation
-(evaluation grids 128 and 160 of output grids that are multiples of 256),
-against the FP64 objective (oracle/ilt.py), at both ends of the bands that
-these grids serve, with one kernel (whose adjoint fields are smaller than the
-interpolation's operand) and with several.
+"""The ILT gradient on the evaluation grids whose images go through the tcgen05
+interpolation (128 and 160, output grids that are multiples of 256), against
+the FP64 objective (oracle/ilt.py), at both ends of the bands that these grids
+serve, with one kernel and with several.
 
 Tolerance as in tests/test_ilt_small.py: FP32 transforms through a resist
 sigmoid of steepness 25, 1e-4 of the largest gradient."""

@@ -1,7 +1,7 @@
-"""The separable interpolation carries images and ILT gradients as FP16 hi/lo
-planes of their own scale, so they keep FP32's range: inputs scaled by a power
-of two give the same bits, scaled (every operation before and after is FP32 and
-far from its limits)."""
+"""The separable interpolation carries images as FP16 hi/lo planes of their own
+scale, so they keep FP32's range, and ILT gradients are FP32 throughout: inputs
+scaled by a power of two give the same bits, scaled (every other operation is
+FP32 and far from its limits)."""
 import numpy as np
 import pytest
 
