@@ -393,9 +393,12 @@ class SimulationEngine:
         ``form``: "fft" (FP32 register-radix FFTs throughout), "tc" (split-BF16x3
         tcgen05 y-contraction and band interpolation), "tc_rows" (row
         transforms on tcgen05 too), "hybrid" (FP32 FFT field pass on the
-        coarse grid, then the exact band interpolation I_N = P I_M P^T as two
-        split-FP16x3 tcgen05 GEMMs) or "auto" (hybrid where its kernels
-        apply, else fft).
+        coarse grid, then the exact band interpolation I_N = P I_M P^T by
+        split-FP16x3 products on tcgen05, in one kernel where N is a multiple
+        of 256 and the grid at most 160) or "auto" (hybrid where its kernels
+        apply, else fft).  ``eval_grid``: 0 picks the smallest supported grid
+        above 4h (16 to 96 in steps of 16 for narrow bands, 128, 160, 192 or
+        384, or a power of two); a power of two, 160, 192 or 384 asks for one.
         Returns a float32 (B, N, N) tensor; ``out``, if given, must be a
         contiguous float32 (B, N, N) tensor on the rasters' device."""
         import torch

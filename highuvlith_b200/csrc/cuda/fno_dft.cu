@@ -55,7 +55,7 @@ __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
 // (group g takes the g-th quarter of every chunk, in order, one fused
 // multiply-add per term); the groups are added as ((0 + 1) + 2) + 3.
 //
-// 512 threads take four rows; a thread owns 8 kx x 4 c, so that a step of x
+// 256 threads take two rows; a thread owns 8 kx x 4 c, so that a step of x
 // costs five shared loads for 32 paired multiply-adds (bound by FP32 issue:
 // the 4 x 4 tile it replaces spent five loads on 32 single ones and staged
 // its input with blocking 2-byte loads).  Input and twiddles arrive by

@@ -1004,6 +1004,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
                                                    img, pdata);
     sum_parts<<<(nc * 2 + 3) / 4, 128, 0, st>>>(pdata, kRedBlocks, 2, nc, sums);
     float* dcdm = nullptr;
+    int adj_launches = 0;
     if (grad) {
       // G' = the band-2h part of G = dC/dI, sampled on the evaluation grid
       const float* Gm = img;
@@ -1023,6 +1024,7 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
       // transforms replace the forward's, which the image has consumed.
       const bool adj_small = !xt && ilt_adj_small_ok(M, hb);
       const BandKernels ak = xt || adj_small ? kernels_for(real_kind, ds, K, st) : BandKernels{ds.kband, K};
+      adj_launches = adj_small ? 1 : (xt && ak.K < K ? 3 : 2);
       if (xt && ak.K < K)
         check_cuda(socs_rows_x(ak.kband, 0.f, Mb, ak.K, hb, M, nc, T, twm, st), "ilt adjoint rows");
       if (xt) {
@@ -1091,7 +1093,11 @@ void Engine::ilt_eval(const huv_ilt_params& p, int masks, const float* theta, co
     ilt_combine<<<(nc + 127) / 128, 128, 0, st>>>(sums, regsum, nc, p.weight, 1.0 / static_cast<double>(npix),
                                                   cost_dev + c0);
     check_cuda(cudaGetLastError(), "ilt kernels");
-    prof.launches += (grad ? 17 : 10) + (coarse ? (grad ? 9 : 4) : 0) - (sep ? 2 : 0);
+    // transmittance, mask band (rows, columns, mean), fields (2, or 3 kept one
+    // by one), interpolation, data term, regulariser, sums
+    prof.launches += 1 + 3 + (few ? 3 : 2) + (sep ? (interp_fused_ok(M, n) ? 1 : 2) : (coarse ? 4 : 0)) + 2 + 3;
+    if (grad)  // G's band and synthesis, the adjoint, the gradient's synthesis
+      prof.launches += (coarse ? 4 : 0) + adj_launches + 3;
   }
   prof.end(st);
 }
