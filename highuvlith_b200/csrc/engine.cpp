@@ -336,7 +336,12 @@ bool Engine::sweep_small(const huv_batch& b, const double* z, int planes, float*
     M = m;
   }
   if (b.input_kind == HUV_INPUT_RECTS) upload_rects(b, sets[0]->hb, st);
-  run_small_form(b, sets.data(), nullptr, nullptr, planes, M, out, st);
+  // Slices of planes: one launch holds at most 65,535 images, and the coarse
+  // images of a slice are kept together (at most 37 MB per clip).
+  constexpr int kSlice = 1024;
+  const size_t plane = static_cast<size_t>(b.n_clips) * n * n;
+  for (int p = 0; p < planes; p += kSlice)
+    run_small_form(b, sets.data() + p, nullptr, nullptr, std::min(kSlice, planes - p), M, out + plane * p, st);
   return true;
 }
 
