@@ -415,15 +415,22 @@ __global__ void ilt_rows_adj(const float2* __restrict__ V, const float2* __restr
     }
     __syncthreads();
     const float2* r = block_fft<-1>(a, b, lg, S, tw);
-    if (threadIdx.x < B) {
-      const int mx = threadIdx.x;
+    auto add = [&](int mx, float2& sum) {
       for (int s = 0; s < ns; ++s) {
         const float2 v = r[(s << lg) + ((mx - hb) & (L - 1))];
         const float2 u = kband[(static_cast<size_t>(k0 + s) * B + my) * B + mx];
         // conj(u) * v
-        acc.x += u.x * v.x + u.y * v.y;
-        acc.y += u.x * v.y - u.y * v.x;
+        sum.x += u.x * v.x + u.y * v.y;
+        sum.y += u.x * v.y - u.y * v.x;
       }
+    };
+    if (threadIdx.x < B) add(threadIdx.x, acc);
+    // bands wider than the block: the further columns are summed in Q itself
+    for (int mx = threadIdx.x + blockDim.x; mx < B; mx += blockDim.x) {
+      float2& q = Q[(static_cast<size_t>(mask) * B + my) * B + mx];
+      float2 sum = k0 > 0 ? q : make_float2(0.f, 0.f);
+      add(mx, sum);
+      q = sum;
     }
     __syncthreads();
   }
