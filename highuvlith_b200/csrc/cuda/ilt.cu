@@ -154,9 +154,14 @@ __global__ void ilt_cols_adj(const float2* __restrict__ T, const float* __restri
     __syncthreads();
     for (int t = threadIdx.x; t < B * Wc; t += blockDim.x) {
       const int my = t / Wc, w = t - my * Wc;
-      a[(w << lg) + ((my - hb) & (L - 1))] = Tm[((static_cast<size_t>(k) * B + my) << lg) + x0 + w];
+      if (my - hb != L / 2) a[(w << lg) + ((my - hb) & (L - 1))] = Tm[((static_cast<size_t>(k) * B + my) << lg) + x0 + w];
     }
     __syncthreads();
+    if (2 * hb == L) {  // the band reaches Nyquist: its last row shares the first one's bin
+      for (int w = threadIdx.x; w < Wc; w += blockDim.x)
+        a[(w << lg) + hb] = cadd(a[(w << lg) + hb], Tm[((static_cast<size_t>(k) * B + 2 * hb) << lg) + x0 + w]);
+      __syncthreads();
+    }
     float2* r = block_fft<+1>(a, b, lg, Wc, tw);
     float2* o = (r == a) ? b : a;
     for (int t = threadIdx.x; t < (Wc << lg); t += blockDim.x) {

@@ -180,9 +180,17 @@ __global__ void socs_rows_inv(const float2* __restrict__ kband, float scale,
     const int k = seq / B, my = seq - k * B;
     const float2 m = Mc[static_cast<size_t>(my) * B + mx];
     const float2 u = kband ? kband[(static_cast<size_t>(k) * B + my) * B + mx] : make_float2(scale, 0.f);
-    a[(s << lg) + ((mx - hb) & (L - 1))] = cmul(u, m);
+    if (mx - hb != L / 2) a[(s << lg) + ((mx - hb) & (L - 1))] = cmul(u, m);
   }
   __syncthreads();
+  if (2 * hb == L) {  // the band reaches Nyquist: its last order shares the first one's bin
+    for (int s = threadIdx.x; s < nseq; s += blockDim.x) {
+      const int seq = seq0 + s, k = seq / B, my = seq - k * B;
+      const float2 u = kband ? kband[(static_cast<size_t>(k) * B + my) * B + 2 * hb] : make_float2(scale, 0.f);
+      a[(s << lg) + hb] = cadd(a[(s << lg) + hb], cmul(u, Mc[static_cast<size_t>(my) * B + 2 * hb]));
+    }
+    __syncthreads();
+  }
   const float2* r = block_fft<+1>(a, b, lg, S, tw);
   float2* Tc = T + static_cast<size_t>(clip) * K * B * L;
   for (int t = threadIdx.x; t < (nseq << lg); t += blockDim.x) {
@@ -215,9 +223,14 @@ __global__ void socs_cols_inv(const float2* __restrict__ T, int K, int hb, int l
     for (int t = threadIdx.x; t < B * Wc; t += blockDim.x) {
       const int my = t / Wc, w = t - my * Wc;
       const float2 v = Tc[((static_cast<size_t>(k) * B + my) << lg) + x0 + w];
-      a[(w << lg) + ((my - hb) & (L - 1))] = v;
+      if (my - hb != L / 2) a[(w << lg) + ((my - hb) & (L - 1))] = v;
     }
     __syncthreads();
+    if (2 * hb == L) {  // as in socs_rows_inv
+      for (int w = threadIdx.x; w < Wc; w += blockDim.x)
+        a[(w << lg) + hb] = cadd(a[(w << lg) + hb], Tc[((static_cast<size_t>(k) * B + 2 * hb) << lg) + x0 + w]);
+      __syncthreads();
+    }
     const float2* r = block_fft<+1>(a, b, lg, Wc, tw);
     for (int t = threadIdx.x; t < (Wc << lg); t += blockDim.x) {
       const float2 e = r[t];
@@ -253,9 +266,14 @@ __global__ void socs_cols_field(const float2* __restrict__ T, int K, int hb, int
   __syncthreads();
   for (int t = threadIdx.x; t < B * Wc; t += blockDim.x) {
     const int my = t / Wc, w = t - my * Wc;
-    a[(w << lg) + ((my - hb) & (L - 1))] = T[((ck * B + my) << lg) + x0 + w];
+    if (my - hb != L / 2) a[(w << lg) + ((my - hb) & (L - 1))] = T[((ck * B + my) << lg) + x0 + w];
   }
   __syncthreads();
+  if (2 * hb == L) {  // as in socs_rows_inv
+    for (int w = threadIdx.x; w < Wc; w += blockDim.x)
+      a[(w << lg) + hb] = cadd(a[(w << lg) + hb], T[((ck * B + 2 * hb) << lg) + x0 + w]);
+    __syncthreads();
+  }
   const float2* r = block_fft<+1>(a, b, lg, Wc, tw);
   for (int t = threadIdx.x; t < (Wc << lg); t += blockDim.x) {
     const int y = t / Wc, w = t - y * Wc;
